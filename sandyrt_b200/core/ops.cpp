@@ -178,9 +178,19 @@ void gemm_simt(const Launch& l, const Tensor& a, const Tensor& w, const Tensor* 
     if (residual && (residual->dtype != DType::F32 || residual->rows != M || residual->cols != N))
         throw KernelError("gemm: residual must be float32 [M, N]");
     if (bias && (bias->dtype != w.dtype || bias->numel() != N)) throw KernelError("gemm: bias must have the weight's dtype and N elements");
-    static auto fn = SANDY_KERNEL(gemm_simt, sandy_gemm_simt);
     OpTimer timer(l, "product, FFMA (float32)", tensor_bytes(&a) + tensor_bytes(&w) + tensor_bytes(&out) + 2 * tensor_bytes(residual),
                   2.0 * M * N * K);
+    // weights whose rows run along k from 16-byte boundaries: the kernels that load four k at a time
+    if (w_out_in && a.dtype == DType::F32 && w.dtype == DType::F32 && out.dtype == DType::F32 && K % 4 == 0 && a.ld % 4 == 0 &&
+        w.ld % 4 == 0 && !((uintptr_t)a.data & 15) && !((uintptr_t)w.data & 15)) {
+        static auto fast = SANDY_KERNEL(gemm_f32, sandy_gemm_f32);
+        check(fast((const float*)a.data, (const float*)w.data, bias ? (const float*)bias->data : nullptr,
+                   residual ? (const float*)residual->data : nullptr, (float*)out.data, (int)M, (int)N, (int)K, (int)a.ld, (int)w.ld,
+                   residual ? (int)residual->ld : 0, (int)out.ld, (int)act, 0, 1, l.stream),
+              "gemm_f32(M=" + std::to_string(M) + ",N=" + std::to_string(N) + ",K=" + std::to_string(K) + ")");
+        return;
+    }
+    static auto fn = SANDY_KERNEL(gemm_simt, sandy_gemm_simt);
     check(fn(a.data, w.data, bias ? bias->data : nullptr, residual ? (const float*)residual->data : nullptr, out.data, (int)M,
              (int)N, (int)K, (int)a.ld, (int)w.ld, residual ? (int)residual->ld : 0, (int)out.ld, w_out_in ? 1 : 0, (int)act,
              code_of(a.dtype), code_of(w.dtype), code_of(out.dtype), l.stream),

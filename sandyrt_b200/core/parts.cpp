@@ -85,8 +85,9 @@ void Linear::bind(const TensorMap& tensors, DType dtype, const Tensor* shared_we
         weight_.view = *shared_weight;
         w_out_in_ = true;
     } else {
-        // the tensor-core kernels read K-major operand rows: one-time repack to [out, in]
-        const bool turn = use_tc_ && layout_ == "in_out";
+        // the tensor-core kernels and the float32 kernels that load four k at a time read K-major operand rows:
+        // one-time repack to [out, in]
+        const bool turn = (use_tc_ || (dtype == DType::F32 && in_ % 4 == 0)) && layout_ == "in_out";
         weight_ = to_device(tensors.at(name_ + ".weight"), dtype, false, turn);
         w_out_in_ = layout_ == "out_in" || turn;
     }

@@ -36,6 +36,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "embed": [],
     "norm": [],
     "gemm_simt": [],
+    "gemm_f32": [],
     "gemm_tc": [],
     "gemm_tc2": [],
     "gemm_skinny": [],

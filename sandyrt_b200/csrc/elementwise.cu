@@ -117,6 +117,21 @@ inline unsigned blocks_for(long long n) {
     return (unsigned)(want < 1 ? 1 : (want > cap ? cap : want));
 }
 
+// dst [cols, rows] = src [rows, cols] transposed, tiles of 32 x 32 through shared memory (bound by memory; weights, once).
+template <typename T>
+__global__ void transpose_kernel(const T* __restrict__ src, T* __restrict__ dst, long long rows, long long cols) {
+    __shared__ T tile[32][33];
+    const long long c0 = (long long)blockIdx.x * 32;
+    for (long long r0 = (long long)blockIdx.y * 32; r0 < rows; r0 += (long long)gridDim.y * 32) {
+        for (int i = threadIdx.y; i < 32; i += 8)
+            if (r0 + i < rows && c0 + threadIdx.x < cols) tile[i][threadIdx.x] = src[(r0 + i) * cols + c0 + threadIdx.x];
+        __syncthreads();
+        for (int i = threadIdx.y; i < 32; i += 8)
+            if (c0 + i < cols && r0 + threadIdx.x < rows) dst[(c0 + i) * rows + r0 + threadIdx.x] = tile[threadIdx.x][i];
+        __syncthreads();
+    }
+}
+
 }  // namespace
 
 // a, b: [rows, cols] of dtype with the same pitch ld_in; out: [rows, cols] of dtype.  act: 0 silu, 1 gelu (tanh).
@@ -194,4 +209,16 @@ SANDY_API int sandy_softcap_f32(float* x, long long n, float cap, cudaStream_t s
     if (!x) return SANDY_ERR_ARGUMENT;
     if (!(cap > 0.0f)) return SANDY_ERR_UNSUPPORTED;
     return sandy_launch(softcap_f32_kernel, dim3(blocks_for(n)), dim3(256), 0, stream, x, n, cap);
+}
+
+// dst [cols, rows] = src [rows, cols] transposed, elements of 2 or 4 bytes.
+SANDY_API int sandy_transpose(const void* src, void* dst, long long rows, long long cols, int elem_size, cudaStream_t stream) {
+    if (rows == 0 || cols == 0) return SANDY_OK;
+    if (!src || !dst || rows < 0 || cols < 0) return SANDY_ERR_ARGUMENT;
+    const long long down = (rows + 31) / 32;
+    const dim3 grid((unsigned)((cols + 31) / 32), (unsigned)(down < 32768 ? down : 32768)), block(32, 8);
+    if (elem_size == 4) transpose_kernel<unsigned><<<grid, block, 0, stream>>>((const unsigned*)src, (unsigned*)dst, rows, cols);
+    else if (elem_size == 2) transpose_kernel<unsigned short><<<grid, block, 0, stream>>>((const unsigned short*)src, (unsigned short*)dst, rows, cols);
+    else return SANDY_ERR_UNSUPPORTED;
+    return sandy_launch_status();
 }

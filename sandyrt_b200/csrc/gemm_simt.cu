@@ -3,9 +3,10 @@
 //
 //   out[m, n] = act( sum_k a[m, k] * w(k, n) + bias[n] ) + residual[m, n]
 //
-// This is the kernel of the true 32-bit path: operands are read as they are stored
+// This is the general kernel of the true 32-bit path: operands are read as they are stored
 // (float, or bfloat16 widened exactly), every product and sum is an IEEE float operation,
-// no tensor-core or reduced-precision matrix mode is involved.  It also serves bfloat16
+// no tensor-core or reduced-precision matrix mode is involved.  float32 weights [N, K] whose rows
+// start on 16-byte boundaries go to gemm_f32.cu instead; this kernel serves the others, and bfloat16
 // operands whose sizes the tensor-core kernel refuses.  The reference computes the same
 // thing with a scalar triple loop (src/core/TensorCalc.cpp:759-770) or one cuBLAS call
 // with CUBLAS_COMPUTE_32F (src/device/cuda/CudaMatMulKernels.cu:196-215).

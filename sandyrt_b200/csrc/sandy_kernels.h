@@ -34,6 +34,10 @@ int sandy_gemm_simt(const void* a, const void* w, const void* bias, const float*
                     int lda, int ldw, int ldr, int ldc, int w_out_in, int act, int a_dtype, int w_dtype, int out_dtype,
                     cudaStream_t stream);
 
+/* gemm_f32.cu */
+int sandy_gemm_f32(const float* a, const float* w, const float* bias, const float* residual, float* out, int M, int N, int K,
+                   int lda, int ldw, int ldr, int ldc, int act, int form, int splits, cudaStream_t stream);
+
 /* gemm_tc.cu, gemm_tc2.cu */
 int sandy_gemm_tc(const void* a, const void* w, const void* bias, const float* residual, void* out, int M, int N, int K,
                   int lda, int ldw, int ldr, int ldc, int act, int out_dtype, int tile_n, void* k_cache, void* v_cache,
@@ -300,6 +304,7 @@ int sandy_head_norm_gate(const float* o, int ldo, const float* gain, int gain_st
 /* elementwise.cu */
 int sandy_glu(const void* a, const void* b, int ld_in, void* out, int ld_out, int rows, int cols, int act, int dtype,
               cudaStream_t stream);
+int sandy_transpose(const void* src, void* dst, long long rows, long long cols, int elem_size, cudaStream_t stream);
 int sandy_cast_cols(const float* x, int ldx, void* out, int ld_out, int rows, int cols, int out_dtype, cudaStream_t stream);
 int sandy_scale_add(const float* y, int ldy, const float* gain, const float* y2, int ldy2, const float* gain2, float* x, int ldx,
                     int rows, int cols, cudaStream_t stream);
