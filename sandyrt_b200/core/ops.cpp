@@ -553,6 +553,18 @@ void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const K
               "prefill_attention" + shape);
         return;
     }
+    // float32 prompts.  The general kernel keeps heads above 128, and small heads on tables of few keys: it starts at once and
+    // then takes 0.2 to 0.4 us a key, where the prompt kernel brings a tile of 64 keys whatever it needs of it.  Alone, us, general /
+    // prompt kernel: 4 heads of 16, prompts of 8 tokens 4.6 / 10.8, of 16 6.7 / 13.0, of 33 11.1 / 14.0, of 64 16.8 / 14.8, of 100
+    // 26.3 / 19.7; 12 heads of 64: 7.0 / 11.5, 9.5 / 13.7, 18.0 / 14.7, 25.5 / 15.6, 44.7 / 21.3.
+    if (s.max_q_len > 1 && q.dtype == DType::F32 && d <= 128 && (d > 32 || s.max_blocks * c.page_size > 128)) {
+        static auto fn = SANDY_KERNEL(attention_prefill_f32, sandy_prefill_attention_f32_rules);
+        OpTimer timer(l, "attention, prompt (float32)", attn_bytes, attn_flops);
+        const int code = fn((const float*)q.data, (int)q.ld, (const float*)c.k, (const float*)c.v, c.page_stride, s.block_table,
+                            s.max_blocks, s.q_start, s.kv_before, (float*)out.data, (int)out.ld, s.n_seqs, s.max_q_len, n_heads, hkv, d,
+                            c.page_size, scale, &rules, c.num_pages, l.kernel_status, l.stream);
+        if (code != -1) { check(code, "prefill_attention_f32" + shape); return; }
+    }
     // Many query heads on one key/value head (attention over a latent, few key/value heads): the heads as the rows
     // of the tensor-core instruction, keys fetched once per sixteen heads (attention_decode_shared.cu).  Blocks of
     // (token, group, sixteen heads) are few, so the keys are cut into enough splits for two blocks an SM, but no

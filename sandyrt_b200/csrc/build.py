@@ -48,6 +48,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "attention_decode_shared": [],
     "attention_prefill": [],
     "attention_prefill_tc": [],
+    "attention_prefill_f32": [],
     "sampling": [],
     "rmsnorm": [],
     "elementwise": [],

@@ -417,6 +417,31 @@ def prefill_attention(q, k_cache, v_cache, block_table, q_start, kv_before, out,
     _check(code, f"prefill_attention(H={n_heads},Hkv={hkv},D={d})")
 
 
+def prefill_attention_f32(q, k_cache, v_cache, block_table, q_start, kv_before, out, *, sink=None, out_gate=None, n_heads: int,
+                          max_q_len: int, scale: float, window: int = 0, softcap: float = 0.0, chunk: int = 0, dist_bias=None,
+                          keep_first: int = 0, elem_gate=None) -> None:
+    """Attention of prompt portions in float32, head sizes 16..128 in steps of 16; q_start and kv_before as in prefill_attention,
+    the rules as in paged_attention."""
+    _cuda(q, k_cache, v_cache, block_table, q_start, kv_before, out, sink, out_gate)
+    hkv, ps, d, page_stride, num_pages = _cache_args(k_cache, v_cache)
+    if q.dtype != torch.float32 or d % 16 != 0 or d > 128:
+        raise UnsupportedShape(f"prefill_attention_f32: float32 and head sizes 16..128 only, got {q.dtype}, {d}")
+    if q.shape[1] != n_heads * d or out.shape != q.shape or q.stride(1) != 1 or out.stride(1) != 1 \
+            or q.dtype != k_cache.dtype or out.dtype != q.dtype:
+        raise KernelError("attention: q and out must be [T, H*D] of the cache's dtype")
+    _i32(block_table, "block_table"); _i32(q_start, "q_start"); _i32(kv_before, "kv_before")
+    S = kv_before.numel()
+    if q_start.numel() != S + 1 or block_table.shape[0] != S:
+        raise KernelError("prefill_attention_f32: q_start, kv_before and block_table disagree on the requests")
+    code = load_library("attention_prefill_f32").sandy_prefill_attention_f32_rules(
+        _p(q), ctypes.c_int(q.stride(0)), _p(k_cache), _p(v_cache), ctypes.c_longlong(page_stride), _p(block_table),
+        ctypes.c_int(block_table.shape[1]), _p(q_start), _p(kv_before), _p(out), ctypes.c_int(out.stride(0)), ctypes.c_int(S),
+        ctypes.c_int(max_q_len), ctypes.c_int(n_heads), ctypes.c_int(hkv), ctypes.c_int(d), ctypes.c_int(ps), ctypes.c_float(scale),
+        _rules(q, n_heads, window, keep_first, softcap, chunk, sink, out_gate, dist_bias, elem_gate), ctypes.c_int(num_pages),
+        _p(kernel_status(q.device)), _stream())
+    _check(code, f"prefill_attention_f32(H={n_heads},Hkv={hkv},D={d})")
+
+
 def _f32(t, name: str) -> None:
     if t is not None and (t.dtype != torch.float32 or not t.is_contiguous()):
         raise KernelError(f"{name} must be a contiguous float32 tensor")

@@ -1,9 +1,11 @@
 """The float32 kernels alone, at the edges of their tiles and splits, against torch in 64 bits."""
+import numpy as np
 import pytest
 import torch
 
+from test_kernels_gpu import DEV, _paged_case
+
 pytestmark = pytest.mark.gpu
-DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("form,splits", [(0, 1), (1, 1), (2, 1), (2, 8), (3, 1), (3, 2), (4, 1), (4, 4), (4, 8)])
@@ -40,3 +42,67 @@ def test_gemm_f32_refuses_what_it_cannot_load():
         ops.gemm_f32(a, w, None, out)                                       # K is no multiple of 4
     with pytest.raises(ops.UnsupportedShape):
         ops.gemm_f32(torch.zeros(25, device=DEV)[1:].view(3, 8)[:, :4], w[:, :4].contiguous(), None, out)   # not on 16 bytes
+
+
+# ---- attention of prompt portions ---------------------------------------------------------------------------------
+def _both(case, H, kw):
+    """The prompt kernel's output and the general kernel's, which reads one (token, head) pair at a time."""
+    from sandyrt_b200.csrc import ops
+
+    lens = [n for _, n in case["seqs"]]
+    q_start = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32, device=DEV)
+    kv_before = torch.tensor([b for b, _ in case["seqs"]], dtype=torch.int32, device=DEV)
+    got = torch.full(case["q"].shape, float("nan"), device=DEV)
+    want = torch.full(case["q"].shape, float("nan"), device=DEV)
+    ops.prefill_attention_f32(case["q"], case["kc"], case["vc"], case["table"], q_start, kv_before, got, n_heads=H,
+                              max_q_len=max(lens), **kw)
+    ops.paged_attention(case["q"], case["kc"], case["vc"], case["table"], case["tok_seq"], case["tok_pos"], want, n_heads=H, **kw)
+    ops.check_kernel_status(DEV)
+    return got, want
+
+
+RULES = [{}, {"window": 70}, {"window": 1}, {"window": 90, "keep_first": 70}, {"window": 30, "keep_first": 3, "gates": True},
+         {"softcap": 3.0, "chunk": 50}, {"softcap": 20.0, "bias": 40, "sink": True}, {"sink": True, "out_gate": True, "gates": True}]
+
+
+@pytest.mark.parametrize("rules", RULES)
+@pytest.mark.parametrize("H,Hkv,D,page_size", [(3, 3, 64, 16), (4, 2, 16, 8), (2, 1, 128, 32), (3, 1, 80, 4), (2, 2, 48, 1)])
+def test_prompt_attention_f32(H, Hkv, D, page_size, rules):
+    """Portions at tile edges (63, 64, 65 tokens), from position 0 and from the middle, single tokens beside them; every
+    rule.  A sum of at most 330 weighted values of size 3, weights that add up to at most 1, against the same in another
+    order: 330 * 2^-24 of the weights twice (exponentials and sums) and of the values, 3 * 3 * 2e-5 = 1.8e-4 at the worst,
+    a tenth of it allowed."""
+    g = torch.Generator().manual_seed(D + page_size)
+    seqs = [(0, 130), (40, 1), (17, 64), (0, 1), (63, 65), (0, 63), (199, 130)]
+    case = _paged_case(torch.float32, H, Hkv, D, page_size, seqs, seed=D + H)
+    T = case["q"].shape[0]
+    kw = {k: v for k, v in rules.items() if k in ("window", "keep_first", "softcap", "chunk")}
+    kw["scale"] = 0.8 / D ** 0.5
+    if rules.get("sink"):
+        kw["sink"] = torch.randn(H, generator=g).to(DEV)
+    if rules.get("out_gate"):
+        kw["out_gate"] = torch.rand(T, H, generator=g).to(DEV)
+    if rules.get("bias"):
+        kw["dist_bias"] = torch.randn(H, rules["bias"], generator=g).to(DEV)
+    if rules.get("gates"):
+        kw["elem_gate"] = torch.randn(T, H * (D - 5) + 9, generator=g).to(DEV)[:, 2:2 + H * (D - 5)]
+    got, want = _both(case, H, kw)
+    assert not torch.isnan(got).any()
+    assert (got - want).abs().max().item() < 2e-5
+    # queries whose rows do not start on 16-byte boundaries
+    wide = torch.zeros(T, case["q"].shape[1] + 3, device=DEV)
+    wide[:, 1:-2] = case["q"]
+    odd, _ = _both({**case, "q": wide[:, 1:-2]}, H, kw)
+    assert torch.equal(odd, got)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_value_that_is_not_finite_reaches_only_the_queries_that_see_it(D, bad):
+    """Token 70's value: the queries before it share its tile of keys."""
+    case = _paged_case(torch.float32, 2, 2, D, 16, [(0, 100), (0, 70)], seed=3)
+    page = int(case["table"][0, 70 // 16])
+    case["vc"][page, :, 70 % 16] = bad
+    got, want = _both(case, 2, {"scale": 0.1})
+    assert torch.isfinite(got[:70]).all() and torch.isfinite(got[100:]).all() and not torch.isfinite(got[70:100]).any()
+    assert (got[:70] - want[:70]).abs().max().item() < 2e-5 and (got[100:] - want[100:]).abs().max().item() < 2e-5
