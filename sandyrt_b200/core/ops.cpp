@@ -1112,8 +1112,23 @@ void embed_bigram(const Launch& l, const StepSeqs& s, const int* ids, const int*
 }
 
 
+namespace {
+// Scratch of the recurrences that form all chunks side by side (matrix_state_chunks.cu), or null where a step stays with the
+// kernels that walk its chunks one by one: heads above 64, portions below 96 tokens (alone, us, walk / side by side: 64 tokens 21 /
+// 23 and 16 / 21, 96 tokens 29 / 25 and 22 / 21), and steps whose scratch would pass half a gigabyte.
+float* chunk_scratch(int kind, const StepSeqs& s, int n_heads, int qk_dim, int v_dim, int max_q_len, Workspace& ws) {
+    constexpr int kWideFrom = 96;
+    constexpr long long kMostFloats = 128ll << 20;
+    if (qk_dim > 64 || v_dim > 1024 || max_q_len < kWideFrom) return nullptr;
+    static auto need = SANDY_KERNEL(matrix_state_chunks, sandy_matrix_chunks_scratch);
+    const long long floats = need(kind, s.n_tokens, s.n_seqs, n_heads, v_dim);
+    if (floats > kMostFloats) return nullptr;
+    return (float*)ws.raw("matrix_chunks", (size_t)floats * sizeof(float));
+}
+}  // namespace
+
 void delta_scan(const Launch& l, const StepSeqs& s, const DeltaShape& d, const Tensor& qkv, const Tensor& bg, const StateView& state,
-                Tensor& out, int max_q_len) {
+                Tensor& out, int max_q_len, Workspace& ws) {
     if (out.dtype != DType::F32 || out.cols != (int64_t)d.n_heads * d.v_dim || qkv.dtype != DType::F32)
         throw KernelError("delta_scan: float32 qkv and out [T, H * e] expected");
     static auto fn = SANDY_KERNEL(matrix_state, sandy_delta_scan);
@@ -1125,15 +1140,23 @@ void delta_scan(const Launch& l, const StepSeqs& s, const DeltaShape& d, const T
     check(fn((const float*)qkv.data, (int)qkv.ld, (const float*)bg.data, (float*)state.data, state.row_elems, s.q_start, s.seq_slots,
              (float*)out.data, (int)out.ld, s.n_seqs, d.n_heads, d.n_qk_heads, d.qk_dim, d.v_dim, long_from, l.stream),
           "delta_scan" + shape);
-    if (long_from)
-        check(chunked((const float*)qkv.data, (int)qkv.ld, (const float*)bg.data, (float*)state.data, state.row_elems, s.q_start,
-                      s.seq_slots, (float*)out.data, (int)out.ld, s.n_seqs, d.n_heads, d.n_qk_heads, d.qk_dim, d.v_dim, long_from,
-                      l.stream),
-              "delta_chunk_scan" + shape);
+    if (!long_from) return;
+    if (float* scratch = chunk_scratch(0, s, d.n_heads, d.qk_dim, d.v_dim, max_q_len, ws)) {
+        static auto wide = SANDY_KERNEL(matrix_state_chunks, sandy_delta_chunks);
+        g_launches += 2;                                   // three launches
+        check(wide((const float*)qkv.data, (int)qkv.ld, (const float*)bg.data, (float*)state.data, state.row_elems, s.q_start, s.seq_slots,
+                   scratch, (float*)out.data, (int)out.ld, s.n_tokens, s.n_seqs, max_q_len, d.n_heads, d.n_qk_heads, d.qk_dim, d.v_dim,
+                   long_from, l.stream),
+              "delta_chunks" + shape);
+        return;
+    }
+    check(chunked((const float*)qkv.data, (int)qkv.ld, (const float*)bg.data, (float*)state.data, state.row_elems, s.q_start,
+                  s.seq_slots, (float*)out.data, (int)out.ld, s.n_seqs, d.n_heads, d.n_qk_heads, d.qk_dim, d.v_dim, long_from, l.stream),
+          "delta_chunk_scan" + shape);
 }
 
 void mlstm_scan(const Launch& l, const StepSeqs& s, const MlstmShape& m, const Tensor& proj, const Tensor& gates,
-                const float* gate_bias, const StateView& state, Tensor& out, int max_q_len) {
+                const float* gate_bias, const StateView& state, Tensor& out, int max_q_len, Workspace& ws) {
     if (out.dtype != DType::F32 || out.cols != (int64_t)m.n_heads * m.v_dim || gates.dtype != DType::F32 || gates.cols < 2 * m.n_heads ||
         state.dtype != DType::F32 || state.row_elems < mlstm_state_floats(m.n_heads, m.qk_dim, m.v_dim))
         throw KernelError("mlstm_scan: shapes disagree");
@@ -1147,11 +1170,20 @@ void mlstm_scan(const Launch& l, const StepSeqs& s, const MlstmShape& m, const T
              m.cap, m.q_scale, (float*)state.data, state.row_elems, s.q_start, s.seq_slots, (float*)out.data, (int)out.ld, s.n_seqs,
              m.n_heads, m.qk_dim, m.v_dim, long_from, l.stream),
           "mlstm_scan" + shape);
-    if (long_from)
-        check(chunked(proj.data, (int)proj.ld, code_of(proj.dtype), m.q_off, m.k_off, m.v_off, (const float*)gates.data, (int)gates.ld,
-                      gate_bias, m.cap, m.q_scale, (float*)state.data, state.row_elems, s.q_start, s.seq_slots, (float*)out.data,
-                      (int)out.ld, s.n_seqs, m.n_heads, m.qk_dim, m.v_dim, long_from, l.stream),
-              "mlstm_chunk_scan" + shape);
+    if (!long_from) return;
+    if (float* scratch = chunk_scratch(1, s, m.n_heads, m.qk_dim, m.v_dim, max_q_len, ws)) {
+        static auto wide = SANDY_KERNEL(matrix_state_chunks, sandy_mlstm_chunks);
+        g_launches += 2;                                   // three launches
+        check(wide(proj.data, (int)proj.ld, code_of(proj.dtype), m.q_off, m.k_off, m.v_off, (const float*)gates.data, (int)gates.ld, gate_bias,
+                   m.cap, m.q_scale, (float*)state.data, state.row_elems, s.q_start, s.seq_slots, scratch, (float*)out.data, (int)out.ld,
+                   s.n_tokens, s.n_seqs, max_q_len, m.n_heads, m.qk_dim, m.v_dim, long_from, l.stream),
+              "mlstm_chunks" + shape);
+        return;
+    }
+    check(chunked(proj.data, (int)proj.ld, code_of(proj.dtype), m.q_off, m.k_off, m.v_off, (const float*)gates.data, (int)gates.ld,
+                  gate_bias, m.cap, m.q_scale, (float*)state.data, state.row_elems, s.q_start, s.seq_slots, (float*)out.data,
+                  (int)out.ld, s.n_seqs, m.n_heads, m.qk_dim, m.v_dim, long_from, l.stream),
+          "mlstm_chunk_scan" + shape);
 }
 
 int64_t fade_state_floats(const FadeShape& m) { return (int64_t)m.n_heads * m.v_dim * m.qk_dim; }

@@ -321,11 +321,11 @@ constexpr int kChunkedFrom = 8;
 // `max_q_len`: the step's longest portion.  Below kChunkedFrom only the token-by-token kernel is launched; from there
 // on both are, each taking the requests of its own kind (which requests those are is read on the device).
 void delta_scan(const Launch& l, const StepSeqs& s, const DeltaShape& d, const Tensor& qkv, const Tensor& bg,
-                const StateView& state, Tensor& out, int max_q_len);
+                const StateView& state, Tensor& out, int max_q_len, Workspace& ws);
 struct MlstmShape { int n_heads = 0, qk_dim = 0, v_dim = 0, q_off = 0, k_off = 0, v_off = 0; float cap = 1.0f, q_scale = 1.0f; };
 // gates float32 [T, >= 2H]: input-gate pre-activations, then forget-gate ones; gate_bias float32 [2H].
 void mlstm_scan(const Launch& l, const StepSeqs& s, const MlstmShape& m, const Tensor& proj, const Tensor& gates,
-                const float* gate_bias, const StateView& state, Tensor& out, int max_q_len);
+                const float* gate_bias, const StateView& state, Tensor& out, int max_q_len, Workspace& ws);
 
 // ---- recurrences with a decay per key channel and token (gated_linear.cu) ----------------------------------------
 enum class FadeKind : int { Add = SANDY_FADE_ADD, Bonus = SANDY_FADE_BONUS, Delta = SANDY_FADE_DELTA };

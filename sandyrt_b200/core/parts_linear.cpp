@@ -388,7 +388,7 @@ public:
         ms.cap = cap_;
         ms.q_scale = 1.0f / std::sqrt((float)d_);
         Tensor read = ws.get("mix_read", T, (int64_t)H_ * e_, DType::F32);
-        ops::mlstm_scan(l, seqs_of(ctx), ms, wide, gates, (const float*)gate_bias_.view.data, ctx.caches->state(call.cache), read, ctx.max_q_len);
+        ops::mlstm_scan(l, seqs_of(ctx), ms, wide, gates, (const float*)gate_bias_.view.data, ctx.caches->state(call.cache), read, ctx.max_q_len, *ctx.workspace);
         Tensor heads = ws.get("mix_heads", T, (int64_t)H_ * e_, ctx.compute_dtype);
         Tensor gate = wide.col_range(n_wide_ - (int64_t)H_ * e_, n_wide_);
         ops::head_norm_gate(l, read, &gain_.view, &gate, ops::GateAct::Sigmoid, 1.0f, eps_, H_, heads);

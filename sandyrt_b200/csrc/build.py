@@ -54,6 +54,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "elementwise": [],
     "attention_prepare": [],
     "matrix_state": [],
+    "matrix_state_chunks": [],
     "gated_linear": [],
     "latent_prepare": [],
     "grouped_gemm": [],

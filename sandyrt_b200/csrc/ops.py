@@ -1126,3 +1126,53 @@ def small_gemm_kernel(M: int, N: int, K: int) -> str:
 def gemm_small_splits(N: int, K: int) -> int:
     """How many blocks share an output tile of gemm_small for this shape on this device."""
     return int(load_library("gemm_small").sandy_gemm_small_splits(ctypes.c_int(N), ctypes.c_int(K)))
+
+
+def _recurrence_args(state, q_start, seq_slots, out):
+    _cuda(state, q_start, seq_slots, out)
+    _i32(q_start, "q_start"); _i32(seq_slots, "seq_slots")
+    if state.dtype != torch.float32 or out.dtype != torch.float32 or state.stride(1) != 1 or out.stride(1) != 1:
+        raise KernelError("a recurrence keeps float32 states [slots, floats] and leaves float32 rows")
+    return seq_slots.numel()
+
+
+def _chunk_scratch(kind: int, n_tokens: int, n_seqs: int, n_heads: int, v_dim: int, device):
+    need = load_library("matrix_state_chunks").sandy_matrix_chunks_scratch
+    need.restype = ctypes.c_longlong
+    return torch.empty(int(need(kind, n_tokens, n_seqs, n_heads, v_dim)), dtype=torch.float32, device=device)
+
+
+def delta_scan(qkv, bg, state, q_start, seq_slots, out, *, n_heads: int, n_qk_heads: int, qk_dim: int, v_dim: int,
+               long_from: int = 0, max_q_len: int = 0, form: str = "tokens") -> None:
+    """The gated delta rule over a step's requests: "tokens" one by one, "walk" chunk by chunk in one block a head's columns,
+    "chunks" all chunks side by side (query/key sizes up to 64).  "tokens" takes the requests of fewer than long_from tokens
+    (0: all), the others those of at least long_from."""
+    S = _recurrence_args(state, q_start, seq_slots, out)
+    head = (_p(qkv), ctypes.c_int(qkv.stride(0)), _p(bg), _p(state), ctypes.c_longlong(state.stride(0)), _p(q_start), _p(seq_slots))
+    tail = (ctypes.c_int(n_heads), ctypes.c_int(n_qk_heads), ctypes.c_int(qk_dim), ctypes.c_int(v_dim), ctypes.c_int(long_from), _stream())
+    if form == "chunks":
+        scratch = _chunk_scratch(0, qkv.shape[0], S, n_heads, v_dim, qkv.device)
+        code = load_library("matrix_state_chunks").sandy_delta_chunks(*head, _p(scratch), _p(out), ctypes.c_int(out.stride(0)),
+                                                                      ctypes.c_int(qkv.shape[0]), ctypes.c_int(S), ctypes.c_int(max_q_len), *tail)
+    else:
+        fn = getattr(load_library("matrix_state"), "sandy_delta_scan" if form == "tokens" else "sandy_delta_chunk_scan")
+        code = fn(*head, _p(out), ctypes.c_int(out.stride(0)), ctypes.c_int(S), *tail)
+    _check(code, f"delta_scan({form},d={qk_dim},e={v_dim})")
+
+
+def mlstm_scan(proj, q_off: int, k_off: int, v_off: int, gates, gate_bias, state, q_start, seq_slots, out, *, cap: float,
+               q_scale: float, n_heads: int, qk_dim: int, v_dim: int, long_from: int = 0, max_q_len: int = 0, form: str = "tokens") -> None:
+    """The matrix memory over a step's requests, in the forms of delta_scan."""
+    S = _recurrence_args(state, q_start, seq_slots, out)
+    head = (_p(proj), ctypes.c_int(proj.stride(0)), ctypes.c_int(_dt(proj)), ctypes.c_int(q_off), ctypes.c_int(k_off), ctypes.c_int(v_off),
+            _p(gates), ctypes.c_int(gates.stride(0)), _p(gate_bias), ctypes.c_float(cap), ctypes.c_float(q_scale), _p(state),
+            ctypes.c_longlong(state.stride(0)), _p(q_start), _p(seq_slots))
+    tail = (ctypes.c_int(n_heads), ctypes.c_int(qk_dim), ctypes.c_int(v_dim), ctypes.c_int(long_from), _stream())
+    if form == "chunks":
+        scratch = _chunk_scratch(1, proj.shape[0], S, n_heads, v_dim, proj.device)
+        code = load_library("matrix_state_chunks").sandy_mlstm_chunks(*head, _p(scratch), _p(out), ctypes.c_int(out.stride(0)),
+                                                                      ctypes.c_int(proj.shape[0]), ctypes.c_int(S), ctypes.c_int(max_q_len), *tail)
+    else:
+        fn = getattr(load_library("matrix_state"), "sandy_mlstm_scan" if form == "tokens" else "sandy_mlstm_chunk_scan")
+        code = fn(*head, _p(out), ctypes.c_int(out.stride(0)), ctypes.c_int(S), *tail)
+    _check(code, f"mlstm_scan({form},d={qk_dim},e={v_dim})")

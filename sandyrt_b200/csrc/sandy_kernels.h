@@ -410,6 +410,17 @@ int sandy_conv_tail(const void* proj, int ld, int dtype, int channels, int n_tap
 int sandy_delta_scan(const float* qkv, int ld, const float* bg, float* state, long long state_stride, const int* q_start,
                      const int* seq_slots, float* out, int ld_out, int n_seqs, int n_heads, int n_qk_heads, int qk_dim,
                      int v_dim, int long_from, cudaStream_t stream);
+/* matrix_state_chunks.cu */
+long long sandy_matrix_chunks_scratch(int kind, int n_tokens, int n_seqs, int n_heads, int v_dim);
+int sandy_delta_chunks(const float* qkv, int ld, const float* bg, float* state, long long state_stride, const int* q_start,
+                       const int* seq_slots, float* scratch, float* out, int ld_out, int n_tokens, int n_seqs, int max_q_len,
+                       int n_heads, int n_qk_heads, int qk_dim, int v_dim, int long_from, cudaStream_t stream);
+int sandy_mlstm_chunks(const void* proj, int ld, int dtype, int q_off, int k_off, int v_off, const float* gates, int ld_gates,
+                       const float* gate_bias, float cap, float q_scale, float* state, long long state_stride, const int* q_start,
+                       const int* seq_slots, float* scratch, float* out, int ld_out, int n_tokens, int n_seqs, int max_q_len,
+                       int n_heads, int qk_dim, int v_dim, int long_from, cudaStream_t stream);
+
+/* matrix_state.cu, continued */
 int sandy_delta_chunk_scan(const float* qkv, int ld, const float* bg, float* state, long long state_stride,
                            const int* q_start, const int* seq_slots, float* out, int ld_out, int n_seqs, int n_heads,
                            int n_qk_heads, int qk_dim, int v_dim, int long_from, cudaStream_t stream);
