@@ -15,8 +15,10 @@
 // Two kernels.  bfloat16 operands whose rows start on 16-byte boundaries go through tensor cores (mma.sync
 // m16n8k16; tiles of 64 x 64, or 128 x 64 where the groups are long; operands staged by cp.async in a ring of
 // stages and read with ldmatrix; rows a tile does not have are zero-filled, so a decode step's one or two rows per
-// expert cost a tile's weight traffic and nothing else).  float32 operands and odd sizes take FFMA tiles.  Which kernel runs is a matter of the model's
-// sizes alone, never of a step's rows.
+// expert cost a tile's weight traffic and nothing else).  float32 operands in rows of whole 16 bytes: tiles of 64 x 64 with packed fma behind a
+// cp.async ring, as in gemm_f32.cu, or, where a group has few rows, its weights streamed past them, a warp four rows of w.
+// What is left (odd sizes) takes plain FFMA tiles.  Which kernel runs is a matter of the sizes and of the most rows a step
+// may bring, never of how they fall on the groups.
 #include "common.cuh"
 
 namespace {
@@ -264,6 +266,194 @@ __global__ void __launch_bounds__(MTHREADS) grouped_mma_kernel(GroupedArgs p) {
         }
 }
 
+// ---- float32 ---------------------------------------------------------------------------------------------------
+// Which group and which of its row tiles of `rows` rows a block is; false behind the step's last tile.
+__device__ __forceinline__ bool find_tile(const GroupedArgs& p, int rows, int& g, int& row0, int& row_end) {
+    if (!p.group_start) {
+        g = blockIdx.z;
+        row0 = blockIdx.y * rows;
+        row_end = p.rows;
+        return true;
+    }
+    int tile = blockIdx.y, start = p.group_start[0];
+    for (g = 0; g < p.G; g++) {
+        const int end = p.group_start[g + 1], tiles = (end - start + rows - 1) / rows;
+        if (tile < tiles) {
+            row0 = start + tile * rows;
+            row_end = end;
+            return true;
+        }
+        tile -= tiles;
+        start = end;
+    }
+    return false;
+}
+__device__ __forceinline__ int row_of(const GroupedArgs& p, int s) { return p.a_row ? p.a_row[s] / p.a_row_div : s; }
+__device__ __forceinline__ float finish_f32(const GroupedArgs& p, float v) {
+    if (p.act == 1) {
+        v = fmaxf(v, 0.0f);
+        v = v * v;
+    }
+    return v;
+}
+
+// Tiles of 64 rows x 64 columns, 128 threads of 8 x 4 outputs, stages of 32 k at a pitch of 144 bytes.  Bound by the fma rate and its
+// loads from shared memory.  4,096 slots on 16 experts, 768 x 1,024 and back, a launch: 519 us on the plain tiles -> 167 us (38 TFLOP/s).
+constexpr int FM = 64, FN = 64, FK = 32, FSTAGES = 3, FTHREADS = 128, FPITCH = FK * 4 + 16, FSTAGE = (FM + FN) * FPITCH;
+
+__global__ void __launch_bounds__(FTHREADS) grouped_f32_kernel(const GroupedArgs p) {
+    extern __shared__ __align__(128) unsigned char ring[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_wait();
+    pdl_launch_dependents();
+    int g, row0, row_end;
+    if (!find_tile(p, FM, g, row0, row_end)) return;
+    const int n0 = blockIdx.x * FN;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(ring);
+    // a thread copies one piece of every sixteenth row of both operands
+    const int copy_row = tid / 8, copy_k = tid % 8 * 4;
+    const float* a_src[FM / 16];
+#pragma unroll
+    for (int i = 0; i < FM / 16; i++) {
+        const int s = row0 + copy_row + 16 * i;
+        a_src[i] = s < row_end ? (const float*)p.a + (size_t)row_of(p, s) * p.lda + (size_t)g * p.a_gcols + copy_k : nullptr;
+    }
+    const float* w_src = (const float*)p.w + (size_t)g * p.w_gstride + (size_t)(n0 + copy_row) * p.ldw + copy_k;
+    const uint32_t dst = base + copy_row * FPITCH + copy_k * 4;
+    auto copy = [](uint32_t to, const void* from, bool valid) {
+        const int bytes = valid ? 16 : 0;       // 0: zeros, nothing is read
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(bytes) : "memory");
+    };
+    const int steps = (p.K + FK - 1) / FK;
+    auto load = [&](int step) {
+        if (step < steps) {
+            const int k0 = step * FK;
+            const uint32_t stage = dst + step % FSTAGES * FSTAGE;
+            const bool k_ok = k0 + copy_k < p.K;
+#pragma unroll
+            for (int i = 0; i < FM / 16; i++) copy(stage + 16 * i * FPITCH, a_src[i] ? a_src[i] + k0 : (const float*)p.a, k_ok && a_src[i]);
+#pragma unroll
+            for (int i = 0; i < FN / 16; i++) {
+                const bool ok = k_ok && n0 + copy_row + 16 * i < p.N;
+                copy(stage + (FM + 16 * i) * FPITCH, ok ? w_src + (size_t)16 * i * p.ldw + k0 : (const float*)p.w, ok);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int s = 0; s < FSTAGES - 1; s++) load(s);
+    const int a_row = warp % 2 * 32 + lane / 8, w_row = warp / 2 * 32 + lane % 8;
+    float2 acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = make_float2(0.0f, 0.0f);
+    for (int step = 0; step < steps; step++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(FSTAGES - 2) : "memory");
+        __syncthreads();
+        load(step + FSTAGES - 1);
+        const unsigned char* stage = ring + step % FSTAGES * FSTAGE;
+        const unsigned char *ap = stage + a_row * FPITCH, *wp = stage + (FM + w_row) * FPITCH;
+#pragma unroll
+        for (int c = 0; c < FK / 4; c++) {
+            float4 av[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) av[i] = *reinterpret_cast<const float4*>(ap + 4 * i * FPITCH + 16 * c);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float4 w = *reinterpret_cast<const float4*>(wp + 8 * j * FPITCH + 16 * c);
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[i][j] = __ffma2_rn(make_float2(av[i].x, av[i].y), make_float2(w.x, w.y), acc[i][j]);
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[i][j] = __ffma2_rn(make_float2(av[i].z, av[i].w), make_float2(w.z, w.w), acc[i][j]);
+            }
+        }
+    }
+    float* O = (float*)p.out + (size_t)g * p.o_gcols;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const int s = row0 + a_row + 4 * i;
+        if (s >= row_end) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int n = n0 + w_row + 8 * j;
+            if (n < p.N) O[(size_t)s * p.ldo + n] = finish_f32(p, acc[i][j].x + acc[i][j].y);
+        }
+    }
+}
+
+// Up to four rows of a group: a warp takes four rows of w, its lanes run along k in float4 steps, and the sums cross the
+// lanes at the end.  Bound by the weights' way from memory: 16 slots on the same experts 78 us on the plain tiles -> 20 us (2.5 TB/s).
+constexpr int SM_ROWS = 4, SW_ROWS = 4, SWARPS = 8, SAHEAD = 3;
+
+__global__ void __launch_bounds__(SWARPS * 32, 2) grouped_f32_few_kernel(const GroupedArgs p) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_wait();
+    pdl_launch_dependents();
+    int g, row0, row_end;
+    if (!find_tile(p, SM_ROWS, g, row0, row_end)) return;
+    const int n0 = (blockIdx.x * SWARPS + warp) * SW_ROWS;
+    if (n0 >= p.N) return;
+    const float* w[SW_ROWS];
+    const float* a[SM_ROWS];
+#pragma unroll
+    for (int r = 0; r < SW_ROWS; r++) w[r] = (const float*)p.w + (size_t)g * p.w_gstride + (size_t)min(n0 + r, p.N - 1) * p.ldw;
+#pragma unroll
+    for (int m = 0; m < SM_ROWS; m++) a[m] = (const float*)p.a + (size_t)row_of(p, min(row0 + m, row_end - 1)) * p.lda + (size_t)g * p.a_gcols;
+    const int steps = (p.K + 127) / 128, k_last = p.K - 4;
+    float4 wv[SAHEAD][SW_ROWS];
+    auto load = [&](int slot, int step) {
+        const int k = step * 128 + lane * 4;
+#pragma unroll
+        for (int r = 0; r < SW_ROWS; r++) {
+            const float4 x = __ldg(reinterpret_cast<const float4*>(w[r] + min(k, k_last)));
+            wv[slot][r] = k <= k_last ? x : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < SAHEAD; i++)
+        if (i < steps) load(i, i);
+    float2 acc[SM_ROWS][SW_ROWS];
+#pragma unroll
+    for (int m = 0; m < SM_ROWS; m++)
+#pragma unroll
+        for (int r = 0; r < SW_ROWS; r++) acc[m][r] = make_float2(0.0f, 0.0f);
+    for (int first = 0; first < steps; first += SAHEAD) {
+#pragma unroll
+        for (int i = 0; i < SAHEAD; i++) {
+            const int step = first + i;
+            if (step < steps) {
+                const int k = min(step * 128 + lane * 4, k_last);
+#pragma unroll
+                for (int m = 0; m < SM_ROWS; m++) {
+                    const float4 av = *reinterpret_cast<const float4*>(a[m] + k);
+#pragma unroll
+                    for (int r = 0; r < SW_ROWS; r++)
+                        acc[m][r] = __ffma2_rn(make_float2(av.z, av.w), make_float2(wv[i][r].z, wv[i][r].w),
+                                               __ffma2_rn(make_float2(av.x, av.y), make_float2(wv[i][r].x, wv[i][r].y), acc[m][r]));
+                }
+                if (step + SAHEAD < steps) load(i, step + SAHEAD);
+            }
+        }
+    }
+    float* O = (float*)p.out + (size_t)g * p.o_gcols;
+#pragma unroll
+    for (int m = 0; m < SM_ROWS; m++)
+#pragma unroll
+        for (int r = 0; r < SW_ROWS; r++) {
+            float v = acc[m][r].x + acc[m][r].y;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == m * SW_ROWS + r && row0 + m < row_end && n0 + r < p.N) O[(size_t)(row0 + m) * p.ldo + n0 + r] = finish_f32(p, v);
+        }
+}
+
+// Whether the float32 kernels can load a problem four k at a time.
+bool f32_takes(const GroupedArgs& p) {
+    return p.K % 4 == 0 && p.K > 0 && p.lda % 4 == 0 && p.ldw % 4 == 0 && p.a_gcols % 4 == 0 && p.w_gstride % 4 == 0 && !((uintptr_t)p.a & 15) &&
+           !((uintptr_t)p.w & 15);
+}
+
 // Whether the tensor-core kernel can take a problem: every row piece a cp.async fetches starts on a 16-byte boundary.
 bool mma_takes(const GroupedArgs& p) {
     return p.K % 8 == 0 && p.lda % 8 == 0 && p.ldw % 8 == 0 && p.a_gcols % 8 == 0 && p.w_gstride % 8 == 0 &&
@@ -291,6 +481,17 @@ int dispatch(const GroupedArgs& p, F row_tiles, int groups_z, int in_dtype, int 
             return tall ? sandy_launch(grouped_mma_kernel<float, 4>, grid, dim3(MTHREADS), 0, stream, p)
                         : sandy_launch(grouped_mma_kernel<float, 2>, grid, dim3(MTHREADS), 0, stream, p);
         return SANDY_ERR_UNSUPPORTED;
+    }
+    if (in_dtype == SANDY_F32 && out_dtype == SANDY_F32 && f32_takes(p)) {
+        // few rows a group on the average (row_tiles(1) counts a group's one partly filled tile too)
+        const bool few = row_tiles(1) / (p.group_start ? p.G : 1) <= SM_ROWS;
+        const dim3 wide(few ? (p.N + SWARPS * SW_ROWS - 1) / (SWARPS * SW_ROWS) : (p.N + FN - 1) / FN, row_tiles(few ? SM_ROWS : FM), groups_z);
+        if (wide.y <= 65535) {
+            if (few) return sandy_launch(grouped_f32_few_kernel, wide, dim3(SWARPS * 32), 0, stream, p);
+            const cudaError_t set = cudaFuncSetAttribute(grouped_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FSTAGES * FSTAGE);
+            if (set != cudaSuccess) return (int)set;
+            return sandy_launch(grouped_f32_kernel, wide, dim3(FTHREADS), FSTAGES * FSTAGE, stream, p);
+        }
     }
     const dim3 grid((p.N + TN - 1) / TN, row_tiles(TM), groups_z);
     if (grid.y > 65535) return SANDY_ERR_UNSUPPORTED;

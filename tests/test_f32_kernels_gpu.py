@@ -1,4 +1,6 @@
 """The float32 kernels alone, at the edges of their tiles and splits, against torch in 64 bits."""
+import types
+
 import numpy as np
 import pytest
 import torch
@@ -106,3 +108,41 @@ def test_a_value_that_is_not_finite_reaches_only_the_queries_that_see_it(D, bad)
     got, want = _both(case, 2, {"scale": 0.1})
     assert torch.isfinite(got[:70]).all() and torch.isfinite(got[100:]).all() and not torch.isfinite(got[70:100]).any()
     assert (got[:70] - want[:70]).abs().max().item() < 2e-5 and (got[100:] - want[100:]).abs().max().item() < 2e-5
+
+
+# ---- one small matrix per group of rows or columns ---------------------------------------------------------------------
+@pytest.mark.parametrize("sizes,N,K", [([1, 0, 2, 1], 33, 132), ([3, 3, 3], 4, 4), ([64, 65, 0, 127, 1], 130, 100), ([200], 64, 64), ([5, 9], 1000, 768)])
+def test_expert_product_f32(sizes, N, K):
+    """Few rows a group and many, tile edges, empty groups, gathered rows; K that is no multiple of a step."""
+    from sandyrt_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(N + K)
+    n, G = sum(sizes), len(sizes)
+    a, w = torch.randn(n, K, generator=g), torch.randn(G, N, K, generator=g)
+    rows = torch.randperm(n, generator=g).to(torch.int32)
+    start = torch.tensor([0] + list(np.cumsum(sizes)), dtype=torch.int32)
+    out = torch.full((n, N), float("nan"), device=DEV)
+    r = types.SimpleNamespace(n_experts=G, n_tokens=n, top=1, group_start=start.to(DEV), entry_of_slot=rows.to(DEV))
+    ops.expert_product(r, a.to(DEV), w.view(G * N, K).to(DEV), out, gather=True, act="relu_squared")
+    src = a[rows.long()].double()
+    which = torch.repeat_interleave(torch.arange(G), torch.tensor(sizes))
+    z = torch.einsum("sk,snk->sn", src, w[which].double())
+    size = torch.einsum("sk,snk->sn", src.abs(), w[which].double().abs())
+    off = (K + 2) * 2.0 ** -24 * size                       # of a sum of K products in any order; its square moves by 2 |z| off
+    want = torch.relu(z) ** 2
+    assert bool(((out.double().cpu() - want).abs() <= 2 * torch.relu(z) * off + off ** 2 + 2.0 ** -23 * want).all())
+
+
+@pytest.mark.parametrize("T", [1, 4, 5, 64, 65, 150])
+def test_head_product_f32(T):
+    from sandyrt_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(T)
+    a, w = torch.randn(T, 3 * 100 + 4, generator=g), torch.randn(3, 40, 96, generator=g)
+    out = torch.full((T, 3 * 48), 7.0, device=DEV)
+    ops.head_product(a.to(DEV), w.view(120, 96).to(DEV), out, n_groups=3, a_gcols=100, o_gcols=48)
+    for h in range(3):
+        want = a[:, h * 100:h * 100 + 96].double() @ w[h].double().t()
+        bound = 97 * 2.0 ** -24 * (a[:, h * 100:h * 100 + 96].double().abs() @ w[h].double().abs().t())
+        assert bool(((out[:, h * 48:h * 48 + 40].double().cpu() - want).abs() <= bound).all())
+        assert bool((out[:, h * 48 + 40:(h + 1) * 48] == 7.0).all())
