@@ -157,6 +157,15 @@ gemm_f32_stream_kernel(const Product p) {
 #pragma unroll
             for (int r = 0; r < ROWS; r++) v[m * ROWS + r] = acc[m][r].x + acc[m][r].y;
         lane_exchange<V>(v, lane);
+        if (parts == 1) {           // nothing to add up across warps: the lanes write their sums, no warp waits for another
+#pragma unroll
+            for (int i = 0; i < (V + 31) / 32; i++) {
+                const int at = V >= 32 ? lane * (V / 32) + i : lane * V / 32;
+                const int m = m0 + at / ROWS, n = quad * ROWS + at % ROWS;
+                if ((V >= 32 || lane * V % 32 == 0) && m < p.M && n < p.N) write_back(p, m, n, v[i]);
+            }
+            continue;
+        }
         const int warp = group * parts + part;
         __syncthreads();            // the sums of the rows before have been read
         if constexpr (V >= 32) {
