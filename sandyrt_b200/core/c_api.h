@@ -123,6 +123,7 @@ int sandy_engine_burst_tokens(void* engine, int burst, int* out);      /* out: [
 int sandy_engine_synchronize(void* engine);
 void* sandy_engine_stream(void* engine);
 /* device time in milliseconds between two marks on the engine's stream */
+int sandy_engine_release(void* engine, long long rid);
 int sandy_engine_mark(void* engine, int which);
 /* Keeps the engine's stream busy for so many microseconds (a kernel that only waits), so that what the
    host queues meanwhile runs back to back behind it: for timing the device's share of a step. */

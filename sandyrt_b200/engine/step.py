@@ -19,6 +19,7 @@ queued and read with `burst_tokens`.
 """
 from __future__ import annotations
 
+import array
 import ctypes
 import dataclasses
 from typing import Hashable, List, Optional, Sequence
@@ -97,14 +98,27 @@ def _ints(values) -> "ctypes.Array":
     return (ctypes.c_int * max(len(values), 1))(*values)
 
 
-def _int_array(parts) -> np.ndarray:
-    """The concatenation of integer sequences (lists or arrays) as one contiguous int32 array: for the
-    token ids of a step, which may be thousands (a ctypes array built from a list costs ten times this)."""
+def _int_array(parts):
+    """The concatenation of integer sequences as one buffer of C ints: (what holds it, its address).  For the token ids of a
+    step: many lists of one id each, or lists of thousands.  numpy takes long lists fastest (30 ns an id) but 0.8 us to begin each:
+    64 lists of one take it 50 us and an array.array 7; what that does not take goes through numpy."""
+    if all(type(p) is list or type(p) is tuple for p in parts) and sum(map(len, parts)) <= 16 * len(parts):
+        try:
+            out = array.array("i")
+            for p in parts:
+                out.extend(p)
+            if not out:
+                out.append(0)
+            return out, out.buffer_info()[0]
+        except (TypeError, OverflowError):
+            pass
     arrays = [np.asarray(p, dtype=np.int32).reshape(-1) for p in parts]
     if not arrays:
-        return np.zeros(1, dtype=np.int32)
-    out = arrays[0] if len(arrays) == 1 else np.concatenate(arrays)
-    return np.ascontiguousarray(out) if out.size else np.zeros(1, dtype=np.int32)
+        arrays = [np.zeros(1, dtype=np.int32)]
+    out = np.ascontiguousarray(arrays[0] if len(arrays) == 1 else np.concatenate(arrays))
+    if not out.size:
+        out = np.zeros(1, dtype=np.int32)
+    return out, out.ctypes.data
 
 
 class Engine:
@@ -148,7 +162,8 @@ class Engine:
         return self._h.call("admit", rid=self.ids.of(rid))
 
     def release(self, rid: Hashable) -> None:
-        self._h.call("release", rid=self.ids.of(rid))
+        if self._lib.sandy_engine_release(ctypes.c_void_p(self._h.handle), ctypes.c_longlong(self.ids.of(rid))) != 0:
+            core.raise_last_error()
 
     def length(self, rid: Hashable) -> int:
         return self._h.call("length", rid=self.ids.of(rid))
@@ -164,7 +179,7 @@ class Engine:
         wanted place) the drawn tokens are read with `read_sampled(n)` afterwards."""
         n = len(entries)
         rids = (ctypes.c_longlong * max(n, 1))(*[self.ids.of(e.rid) for e in entries])
-        tokens = _int_array([e.tokens for e in entries])
+        tokens, tokens_at = _int_array([e.tokens for e in entries])
         want = [int(w) for e in entries for w in e.want]
         samp = None
         if sampling is not None:
@@ -172,7 +187,7 @@ class Engine:
             samp = (ctypes.c_float * max(len(flat), 1))(*flat)
         logits, rows, cols = ctypes.c_void_p(), ctypes.c_int(), ctypes.c_int()
         code = self._lib.sandy_engine_step(ctypes.c_void_p(self._h.handle), n, rids, _ints([len(e.tokens) for e in entries]),
-                                           tokens.ctypes.data_as(ctypes.POINTER(ctypes.c_int)),
+                                           ctypes.c_void_p(tokens_at),
                                            _ints([len(e.want) for e in entries]), _ints(want), samp,
                                            ctypes.byref(logits), ctypes.byref(rows), ctypes.byref(cols))
         if code != 0:
