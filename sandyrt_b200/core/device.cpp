@@ -47,6 +47,8 @@ PinnedBuffer& PinnedBuffer::operator=(PinnedBuffer&& o) noexcept {
     return *this;
 }
 
+thread_local TransposeStage* TransposeStage::current_ = nullptr;
+
 DeviceWeight to_device(const HostTensor& t, DType compute, bool keep_32bit, bool transpose, bool as_rows) {
     int64_t rows = 1, cols = t.numel();
     if (t.shape.size() >= 2 && as_rows) {
@@ -78,9 +80,10 @@ DeviceWeight to_device(const HostTensor& t, DType compute, bool keep_32bit, bool
     w.buffer = std::make_shared<DeviceBuffer>(bytes);
     if (transpose && t.numel()) {
         // turned on the device: on the host it costs as much as reading the file (28 M floats: 60 to 200 ms)
-        DeviceBuffer raw(bytes);
-        cuda_check(cudaMemcpy(raw.get(), src, bytes, cudaMemcpyHostToDevice), "copying a weight to the device");
-        const int code = SANDY_KERNEL(elementwise, sandy_transpose)(raw.get(), w.buffer->get(), rows, cols, (int)esz, nullptr);
+        TransposeStage own, *stage = own.outer() ? own.outer() : &own;
+        void* raw = stage->room(bytes);
+        cuda_check(cudaMemcpy(raw, src, bytes, cudaMemcpyHostToDevice), "copying a weight to the device");
+        const int code = SANDY_KERNEL(elementwise, sandy_transpose)(raw, w.buffer->get(), rows, cols, (int)esz, nullptr);
         if (code) throw KernelError("transposing a weight: code " + std::to_string(code));
         cuda_check(cudaStreamSynchronize(nullptr), "transposing a weight");
     } else if (t.numel()) {

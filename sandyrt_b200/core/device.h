@@ -90,6 +90,28 @@ struct DeviceWeight {
 DeviceWeight to_device(const HostTensor& t, DType compute, bool keep_32bit = false, bool transpose = false,
                        bool as_rows = true);
 
+// While one lives, the weights that its thread has turned on the device pass through one buffer, as large as the largest of
+// them, instead of one each (an allocation and its release cost as much as the copy).
+class TransposeStage {
+public:
+    TransposeStage() : outer_(current_) { current_ = this; }
+    ~TransposeStage() { current_ = outer_; }
+    TransposeStage(const TransposeStage&) = delete;
+    TransposeStage& operator=(const TransposeStage&) = delete;
+    TransposeStage* outer() const { return outer_; }
+    void* room(size_t bytes) {
+        if (buffer_.bytes() < bytes) {
+            buffer_ = DeviceBuffer();
+            buffer_ = DeviceBuffer(bytes);
+        }
+        return buffer_.get();
+    }
+private:
+    static thread_local TransposeStage* current_;
+    TransposeStage* outer_;
+    DeviceBuffer buffer_;
+};
+
 // Named scratch tensors that keep their address from step to step (so that a captured CUDA graph
 // stays valid) and only ever grow.
 class Workspace {

@@ -70,6 +70,7 @@ TensorRequests Model::tensor_requests() const {
 }
 
 void Model::bind(const TensorMap& tensors, DType dtype) {
+    TransposeStage stage;
     if (dtype != DType::F32 && dtype != DType::BF16) throw ValueError("compute dtype must be float32 or bfloat16");
     dtype_ = dtype;
     for (const PartRef& p : parts()) {
