@@ -498,6 +498,10 @@ constexpr int kClusterMaxSplits = 8;
 // 1 x 12 pairs 356 against 333 us, the register kernel starting sooner.
 constexpr int kBulkMinPairs = 256;
 
+// Single tokens of a mixed step from which they leave the prompt kernel for a launch of the decode kernel (GPT-2 medium, four layers,
+// 32 of them behind 100 to 700 tokens beside a portion of 480: a step 579 -> 530 us; fewer than eight cost less than the launch).
+constexpr int kSinglesApart = 8;
+
 bool decode_head_dim(DType dt, int d) {
     if (d == 16 || d == 32 || d == 64 || d == 128) return true;
     return d == 256 && dt == DType::BF16;
@@ -538,12 +542,29 @@ void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const K
     if (s.max_q_len > 1 && q.dtype == DType::BF16 && d <= 128) {
         static const bool use_tc = env_int("SANDYRT_PREFILL_TC", 1) != 0;     // 0 keeps every head size on the mma.sync kernel
         if (use_tc && d == 64 && !db) {                       // (the tcgen05 kernel has no form for a bias by distance)
-            static auto fn = SANDY_KERNEL(attention_prefill_tc, sandy_prefill_attention_tc_rules);
+            // Single tokens beside portions: a tile of 128 queries with one row in it costs as much as a full one, so where a
+            // step holds enough of them they go to the decode kernel.  What is known of a step that a recorded graph may
+            // serve again is its tokens, its requests and its longest portion: at most so many requests bring one token.
+            const int singles = s.n_seqs - (T - s.n_seqs + s.max_q_len - 2) / (s.max_q_len - 1);
+            const int seen = window > 0 ? std::min(window + keep, s.max_blocks * c.page_size) : s.max_blocks * c.page_size;
+            const int splits = singles > 0 ? std::min(decode_splits(singles, n_heads, seen), kClusterMaxSplits) : 1;
+            static auto max_keys_fn = SANDY_KERNEL(attention_decode_mma, sandy_decode_attention_mma_max_keys);
+            const bool apart = !ruled && singles >= kSinglesApart && 2 * singles >= s.n_seqs && s.n_seqs <= 65535 && seen <= max_keys_fn(splits, c.page_size);
+            static auto fn = SANDY_KERNEL(attention_prefill_tc, sandy_prefill_attention_tc_portions);
             OpTimer timer(l, "attention, prompt (tcgen05)", attn_bytes, attn_flops);
             const int code = fn(q.data, (int)q.ld, c.k, c.v, c.page_stride, s.block_table, s.max_blocks, s.q_start, s.kv_before,
                                 out.data, (int)out.ld, s.n_seqs, s.max_q_len, n_heads, hkv, d, c.page_size, scale, &rules,
-                                c.num_pages, l.kernel_status, l.stream);
-            if (code != -1) { check(code, "prefill_attention_tc" + shape); return; }
+                                c.num_pages, apart ? 2 : 1, l.kernel_status, l.stream);
+            if (code != -1) {
+                check(code, "prefill_attention_tc" + shape);
+                if (!apart) return;
+                static auto single = SANDY_KERNEL(attention_decode_mma, sandy_decode_attention_mma_single);
+                check(single(q.data, (int)q.ld, c.k, c.v, c.page_stride, s.block_table, s.max_blocks, s.q_start, s.kv_before, out.data,
+                             (int)out.ld, s.n_seqs, n_heads, hkv, d, c.page_size, scale, &rules, splits, c.num_pages, seen,
+                             l.kernel_status, l.stream),
+                      "decode_attention_mma_single" + shape);
+                return;
+            }
         }
         static auto fn = SANDY_KERNEL(attention_prefill, sandy_prefill_attention_rules);
         OpTimer timer(l, "attention, prompt (mma.sync)", attn_bytes, attn_flops);

@@ -90,7 +90,7 @@ decode_attention_mma_kernel(const bf16* __restrict__ q, int ld_q, const bf16* __
                             bf16* __restrict__ out, int ld_out, int n_heads, int n_kv_heads, int page_size, float scale,
                             int window, int num_splits, int num_pages, const float* __restrict__ sink,
                             const float* __restrict__ out_gate, int keep_first, const bf16* __restrict__ elem_gate,
-                            int ld_elem_gate, int gate_dim, int* __restrict__ status) {
+                            int ld_elem_gate, int gate_dim, const int* __restrict__ single_of, int* __restrict__ status) {
     // a warp's own stages: [stage][keys | values][16 rows of 128 bytes]
     __shared__ __align__(128) uint8_t st[WARPS][STAGES][2][GROUP_BYTES];
     __shared__ int s_pages[MAX_PAGES];
@@ -99,15 +99,27 @@ decode_attention_mma_kernel(const bf16* __restrict__ q, int ld_q, const bf16* __
     __shared__ float cl_all[MAX_CLUSTER_SPLITS][D + 2];   // in the cluster's first block: every split's (output, max, sum)
 
     pdl_launch_dependents();
+    // With single_of (q_start of a step of mixed requests) blockIdx.z is a request, positions are the requests' first, and only
+    // requests that bring one token are taken; all blocks of a cluster leave together.
+    int t = blockIdx.z, s;
+    if (single_of) {
+        s = t;
+        t = single_of[s];
+        if (single_of[s + 1] - t != 1) {
+            pdl_wait();                                 // a kernel ends only after the one before it has
+            return;
+        }
+    } else {
+        s = token_seq[t];
+    }
     const bool in_cluster = num_splits > 1;
     // A block may write into another block's shared memory only once that block is running: every
     // block says so here, and waits for the others only when it has its partial state to hand over.
     if (in_cluster) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    const int split = blockIdx.x, h = blockIdx.y, t = blockIdx.z;
+    const int split = blockIdx.x, h = blockIdx.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, tq = lane & 3;
-    const int s = token_seq[t];
-    const int pos = positions[t];
+    const int pos = positions[blockIdx.z];
     const int kvh = h / (n_heads / n_kv_heads);
     const VisibleKeys seen = visible_keys(pos, window, keep_first, 0);
     const int n_keys = seen.n;
@@ -355,18 +367,18 @@ SANDY_API int sandy_decode_attention_mma_max_keys(int num_splits, int page_size)
 // Arguments as sandy_decode_attention_cluster (attention_decode.cu); bfloat16, heads of 64, 1 <= num_splits <= 8;
 // max_keys: the longest visible range of any token of the launch (checked against the block's table of pages).
 // No form for capped scores, chunks of positions or a bias by distance.
-SANDY_API int sandy_decode_attention_mma_rules(const void* q, int ld_q, const void* k_cache, const void* v_cache,
+static int launch_mma(const void* q, int ld_q, const void* k_cache, const void* v_cache,
                                              long long page_stride, const int* block_table, int max_blocks,
                                              const int* token_seq, const int* positions, void* out, int ld_out, int n_tokens,
                                              int n_heads, int n_kv_heads, int head_dim, int page_size, float scale,
                                              const SandyAttentionRules* rules, int num_splits, int num_pages, int max_keys,
-                                             int* status, cudaStream_t stream) {
+                                             const int* single_of, int* status, cudaStream_t stream) {
     if (n_tokens == 0) return SANDY_OK;
     if (!rules) return SANDY_ERR_ARGUMENT;
     if (rules->softcap != 0.0f || rules->chunk || rules->dist_bias || rules->keep_first < 0 || (rules->elem_gate && rules->gate_dim < 1))
         return SANDY_ERR_UNSUPPORTED;
     const int window = rules->window;
-    if (!q || !k_cache || !v_cache || !block_table || !token_seq || !positions || !out) return SANDY_ERR_ARGUMENT;
+    if (!q || !k_cache || !v_cache || !block_table || !(token_seq || single_of) || !positions || !out) return SANDY_ERR_ARGUMENT;
     if (head_dim != D || num_splits < 1 || num_splits > MAX_CLUSTER_SPLITS) return SANDY_ERR_UNSUPPORTED;
     if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0 || page_size <= 0 || window < 0) return SANDY_ERR_UNSUPPORTED;
     if (n_heads > 65535 || n_tokens > 65535) return SANDY_ERR_UNSUPPORTED;
@@ -399,8 +411,31 @@ SANDY_API int sandy_decode_attention_mma_rules(const void* q, int ld_q, const vo
                                              (const bf16*)v_cache, page_stride, block_table, max_blocks, token_seq, positions,
                                              (bf16*)out, ld_out, n_heads, n_kv_heads, page_size, scale, window, num_splits,
                                              num_pages, rules->sink, rules->out_gate, rules->keep_first,
-                                             (const bf16*)rules->elem_gate, rules->ld_elem_gate, rules->gate_dim, status);
+                                             (const bf16*)rules->elem_gate, rules->ld_elem_gate, rules->gate_dim, single_of, status);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+SANDY_API int sandy_decode_attention_mma_rules(const void* q, int ld_q, const void* k_cache, const void* v_cache,
+                                             long long page_stride, const int* block_table, int max_blocks,
+                                             const int* token_seq, const int* positions, void* out, int ld_out, int n_tokens,
+                                             int n_heads, int n_kv_heads, int head_dim, int page_size, float scale,
+                                             const SandyAttentionRules* rules, int num_splits, int num_pages, int max_keys,
+                                             int* status, cudaStream_t stream) {
+    return launch_mma(q, ld_q, k_cache, v_cache, page_stride, block_table, max_blocks, token_seq, positions, out, ld_out, n_tokens,
+                      n_heads, n_kv_heads, head_dim, page_size, scale, rules, num_splits, num_pages, max_keys, nullptr, status, stream);
+}
+
+// The same for a step of mixed requests: takes the requests that bring one token (q_start [n_seqs + 1], kv_before [n_seqs]) and
+// leaves the others' rows alone.
+SANDY_API int sandy_decode_attention_mma_single(const void* q, int ld_q, const void* k_cache, const void* v_cache,
+                                                long long page_stride, const int* block_table, int max_blocks, const int* q_start,
+                                                const int* kv_before, void* out, int ld_out, int n_seqs, int n_heads,
+                                                int n_kv_heads, int head_dim, int page_size, float scale,
+                                                const SandyAttentionRules* rules, int num_splits, int num_pages, int max_keys,
+                                                int* status, cudaStream_t stream) {
+    if (!q_start) return SANDY_ERR_ARGUMENT;
+    return launch_mma(q, ld_q, k_cache, v_cache, page_stride, block_table, max_blocks, nullptr, kv_before, out, ld_out, n_seqs, n_heads,
+                      n_kv_heads, head_dim, page_size, scale, rules, num_splits, num_pages, max_keys, q_start, status, stream);
 }
 
 // The same without kept first keys or a gate by element.

@@ -170,7 +170,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
                             const int* __restrict__ kv_before, bf16* __restrict__ out, int ld_out, int n_heads,
                             int n_kv_heads, int page_size, float scale, int window, float softcap, int chunk,
                             int num_pages, int use_tma, const float* __restrict__ sink, const float* __restrict__ out_gate,
-                            int keep_first, const bf16* __restrict__ elem_gate, int ld_elem_gate, int gate_dim,
+                            int keep_first, const bf16* __restrict__ elem_gate, int ld_elem_gate, int gate_dim, int min_q_len,
                             int* __restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ int s_table[TABLE_SMEM];
@@ -188,7 +188,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     const int qs = q_start[s];
     const int q_len = q_start[s + 1] - qs;
     const int n_tiles = (q_len + BM - 1) / BM;
-    if ((int)blockIdx.x >= n_tiles) return;
+    if ((int)blockIdx.x >= n_tiles || q_len < min_q_len) return;
     const int tile = n_tiles - 1 - blockIdx.x;         // the tiles with the most keys start first
     const int t0 = tile * BM;
     const int rows_valid = min(BM, q_len - t0);
@@ -584,13 +584,14 @@ bool get_page_map(const void* cache, long long page_stride, int num_pages, int n
 }  // namespace
 
 // Arguments as sandy_prefill_attention (attention_prefill.cu).  Heads of 64 only; out and q rows
-// must be 16-byte aligned.  SANDY_ERR_UNSUPPORTED for everything else: the caller then takes the
+// must be 16-byte aligned.  Requests that bring fewer than min_q_len tokens are left out (one at least has to bring as many:
+// a kernel of blocks that all leave at once would not wait for the one before it).  SANDY_ERR_UNSUPPORTED for everything else: the caller then takes the
 // mma.sync kernel.
-SANDY_API int sandy_prefill_attention_tc_rules(const void* q, int ld_q, const void* k_cache, const void* v_cache,
+SANDY_API int sandy_prefill_attention_tc_portions(const void* q, int ld_q, const void* k_cache, const void* v_cache,
                                          long long page_stride, const int* block_table, int max_blocks,
                                          const int* q_start, const int* kv_before, void* out, int ld_out, int n_seqs,
                                          int max_q_len, int n_heads, int n_kv_heads, int head_dim, int page_size,
-                                         float scale, const SandyAttentionRules* rules, int num_pages, int* status,
+                                         float scale, const SandyAttentionRules* rules, int num_pages, int min_q_len, int* status,
                                          cudaStream_t stream) {
     if (n_seqs == 0 || max_q_len == 0) return SANDY_OK;
     if (!rules) return SANDY_ERR_ARGUMENT;
@@ -633,7 +634,19 @@ SANDY_API int sandy_prefill_attention_tc_rules(const void* q, int ld_q, const vo
                         (const bf16*)k_cache, (const bf16*)v_cache, page_stride, block_table, max_blocks, q_start,
                         kv_before, (bf16*)out, ld_out, n_heads, n_kv_heads, page_size, scale, window, softcap, chunk, num_pages,
                         use_tma, rules->sink, rules->out_gate, rules->keep_first, (const bf16*)rules->elem_gate,
-                        rules->ld_elem_gate, rules->gate_dim, status);
+                        rules->ld_elem_gate, rules->gate_dim, min_q_len, status);
+}
+
+// All requests.
+SANDY_API int sandy_prefill_attention_tc_rules(const void* q, int ld_q, const void* k_cache, const void* v_cache,
+                                         long long page_stride, const int* block_table, int max_blocks,
+                                         const int* q_start, const int* kv_before, void* out, int ld_out, int n_seqs,
+                                         int max_q_len, int n_heads, int n_kv_heads, int head_dim, int page_size,
+                                         float scale, const SandyAttentionRules* rules, int num_pages, int* status,
+                                         cudaStream_t stream) {
+    return sandy_prefill_attention_tc_portions(q, ld_q, k_cache, v_cache, page_stride, block_table, max_blocks, q_start, kv_before,
+                                               out, ld_out, n_seqs, max_q_len, n_heads, n_kv_heads, head_dim, page_size, scale,
+                                               rules, num_pages, 1, status, stream);
 }
 
 // The same without kept first keys or a gate by element.

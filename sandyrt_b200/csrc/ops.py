@@ -417,6 +417,28 @@ def prefill_attention(q, k_cache, v_cache, block_table, q_start, kv_before, out,
     _check(code, f"prefill_attention(H={n_heads},Hkv={hkv},D={d})")
 
 
+def mixed_attention(q, k_cache, v_cache, block_table, q_start, kv_before, out, *, sink=None, out_gate=None, n_heads: int,
+                    max_q_len: int, scale: float, window: int = 0, keep_first: int = 0, elem_gate=None, num_splits: int = 1) -> None:
+    """Attention of a step of portions and single tokens in two launches (bfloat16, heads of 64; at least one portion): the
+    portions on the tcgen05 prompt kernel, the single tokens on the mma.sync decode kernel."""
+    _cuda(q, k_cache, v_cache, block_table, q_start, kv_before, out, sink, out_gate)
+    hkv, ps, d, page_stride, num_pages = _cache_args(k_cache, v_cache)
+    if q.dtype != torch.bfloat16 or d != 64 or out.shape != q.shape or q.stride(1) != 1 or out.stride(1) != 1 or max_q_len < 2:
+        raise UnsupportedShape("mixed_attention: bfloat16, heads of 64 and a portion of two tokens or more")
+    _i32(block_table, "block_table"); _i32(q_start, "q_start"); _i32(kv_before, "kv_before")
+    S, status = kv_before.numel(), _p(kernel_status(q.device))
+    rules = _rules(q, n_heads, window, keep_first, sink=sink, out_gate=out_gate, elem_gate=elem_gate)
+    head = (_p(q), ctypes.c_int(q.stride(0)), _p(k_cache), _p(v_cache), ctypes.c_longlong(page_stride), _p(block_table),
+            ctypes.c_int(block_table.shape[1]), _p(q_start), _p(kv_before), _p(out), ctypes.c_int(out.stride(0)), ctypes.c_int(S))
+    sizes = (ctypes.c_int(n_heads), ctypes.c_int(hkv), ctypes.c_int(d), ctypes.c_int(ps), ctypes.c_float(scale), rules)
+    code = load_library("attention_prefill_tc").sandy_prefill_attention_tc_portions(
+        *head, ctypes.c_int(max_q_len), *sizes, ctypes.c_int(num_pages), ctypes.c_int(2), status, _stream())
+    _check(code, f"prefill_attention_tc(H={n_heads},Hkv={hkv},D={d})")
+    code = load_library("attention_decode_mma").sandy_decode_attention_mma_single(
+        *head, *sizes, ctypes.c_int(num_splits), ctypes.c_int(num_pages), ctypes.c_int(block_table.shape[1] * ps), status, _stream())
+    _check(code, f"decode_attention_mma(H={n_heads},Hkv={hkv},page={ps},splits={num_splits})")
+
+
 def prefill_attention_f32(q, k_cache, v_cache, block_table, q_start, kv_before, out, *, sink=None, out_gate=None, n_heads: int,
                           max_q_len: int, scale: float, window: int = 0, softcap: float = 0.0, chunk: int = 0, dist_bias=None,
                           keep_first: int = 0, elem_gate=None) -> None:

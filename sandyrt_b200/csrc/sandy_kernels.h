@@ -214,6 +214,16 @@ int sandy_prefill_attention_tc_rules(const void* q, int ld_q, const void* k_cach
                                      const int* block_table, int max_blocks, const int* q_start, const int* kv_before, void* out,
                                      int ld_out, int n_seqs, int max_q_len, int n_heads, int n_kv_heads, int head_dim, int page_size,
                                      float scale, const SandyAttentionRules* rules, int num_pages, int* status, cudaStream_t stream);
+int sandy_prefill_attention_tc_portions(const void* q, int ld_q, const void* k_cache, const void* v_cache, long long page_stride,
+                                        const int* block_table, int max_blocks, const int* q_start, const int* kv_before, void* out,
+                                        int ld_out, int n_seqs, int max_q_len, int n_heads, int n_kv_heads, int head_dim,
+                                        int page_size, float scale, const SandyAttentionRules* rules, int num_pages, int min_q_len,
+                                        int* status, cudaStream_t stream);
+int sandy_decode_attention_mma_single(const void* q, int ld_q, const void* k_cache, const void* v_cache, long long page_stride,
+                                      const int* block_table, int max_blocks, const int* q_start, const int* kv_before, void* out,
+                                      int ld_out, int n_seqs, int n_heads, int n_kv_heads, int head_dim, int page_size, float scale,
+                                      const SandyAttentionRules* rules, int num_splits, int num_pages, int max_keys, int* status,
+                                      cudaStream_t stream);
 int sandy_decode_attention_shared_rules(const void* q, int ld_q, const void* k_cache, const void* v_cache, long long page_stride,
                                         const int* block_table, int max_blocks, const int* token_seq, const int* positions, void* out,
                                         int ld_out, int n_tokens, int n_heads, int n_kv_heads, int head_dim, int page_size, float scale,
