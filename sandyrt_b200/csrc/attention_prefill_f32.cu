@@ -180,6 +180,7 @@ prefill_attention_f32_kernel(const PromptArgs p) {
             const bool whole = __all_sync(0xffffffffu, !ruled && found && start + BKEYS - 1 <= pos0);
             bool rose = false;
             float corr[8];
+            unsigned hidden = 0;                    // bit 8 j + i: query i does not see key j, whatever its score is
 #pragma unroll
             for (int i = 0; i < 8; i++) {
 #pragma unroll
@@ -199,6 +200,7 @@ prefill_attention_f32_kernel(const PromptArgs p) {
                         if (r.softcap > 0.0f) x = r.softcap * tanhf(x / r.softcap);
                         if (r.dist_bias && seen) x += r.dist_bias[(size_t)head * r.n_dist + min(pos - key, r.n_dist - 1)];
                         x = seen ? x : -INFINITY;
+                        hidden |= seen ? 0u : 1u << (8 * j + i);
                         s[i][0] = j == 0 ? x : s[i][0];
                         s[i][1] = j == 1 ? x : s[i][1];
                         s[i][2] = j == 2 ? x : s[i][2];
@@ -216,8 +218,15 @@ prefill_attention_f32_kernel(const PromptArgs p) {
                 rose |= m_new != m[i];
                 m[i] = m_new;
 #pragma unroll
-                for (int j = 0; j < 4; j++) s[i][j] = s[i][j] > -INFINITY ? expf(s[i][j] - base) : NOT_SEEN;
+                for (int j = 0; j < 4; j++) s[i][j] = expf(s[i][j] - base);      // (a score that is NaN stays one)
                 l[i] = l[i] * corr[i] + ((s[i][0] + s[i][1]) + (s[i][2] + s[i][3]));
+            }
+            if (!whole) {
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        if (hidden >> (8 * j + i) & 1) s[i][j] = NOT_SEEN;
             }
             if (__any_sync(0xffffffffu, rose)) {
 #pragma unroll

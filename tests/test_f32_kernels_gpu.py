@@ -110,6 +110,54 @@ def test_a_value_that_is_not_finite_reaches_only_the_queries_that_see_it(D, bad)
     assert (got[:70] - want[:70]).abs().max().item() < 2e-5 and (got[100:] - want[100:]).abs().max().item() < 2e-5
 
 
+def _formula(case, H, scale, window, sink):
+    """[T, H * D] in 64 bits, request by request; a hidden key has no part in a query's sums, whatever it holds."""
+    rows = []
+    for s, (before, n) in enumerate(case["seqs"]):
+        k, v, q = (case[name][s].double() for name in ("dense_k", "dense_v", "qs"))
+        for i in range(n):
+            lo, hi = max(0, before + i + 1 - window) if window else 0, before + i + 1
+            z = torch.einsum("jhd,hd->hj", k[lo:hi], q[i]) * scale
+            if sink is not None:
+                z = torch.cat([z, sink.double().cpu().view(H, 1)], 1)
+            p = torch.softmax(z, 1)[:, :hi - lo]
+            rows.append(torch.einsum("hj,jhd->hd", p, v[lo:hi]).reshape(-1))
+    return torch.stack(rows)
+
+
+@pytest.mark.parametrize("D", [16, 64, 128])
+@pytest.mark.parametrize("window", [0, 90])
+@pytest.mark.parametrize("with_sink", [False, True])
+@pytest.mark.parametrize("bad", ["key", "key and value", "query", "score of minus infinity", "score of minus infinity and value"])
+def test_a_token_that_is_not_finite_reaches_every_query_that_sees_it(D, window, with_sink, bad):
+    """Token 70 of 200: its tile of keys is at the edge for the queries of its own tile and a whole one for those behind it.
+    A NaN score is a NaN in the softmax, and a seen key whose score is minus infinity still brings 0 times its value; what
+    the formula leaves finite stays so."""
+    H, at = 2, 70
+    case = _paged_case(torch.float32, H, H, D, 16, [(0, 200), (0, 70)], seed=3)
+    page = int(case["table"][0, at // 16])
+    if "minus" in bad:                                      # queries above zero, a key of -inf
+        case["q"] = case["q"].abs()
+        case["qs"] = [q.abs() for q in case["qs"]]
+    for name, cache, dense, x in (("query", None, None, None), ("key", "kc", "dense_k", float("nan")),
+                                  ("minus", "kc", "dense_k", -float("inf")), ("value", "vc", "dense_v", float("inf" if "minus" in bad else "nan"))):
+        if name in bad and cache:
+            case[cache][page, :, at % 16] = x
+            case[dense][0][at] = x
+    if bad == "query":
+        case["q"][at] = float("nan")
+        case["qs"][0][at] = float("nan")
+    sink = torch.tensor([0.5, -1.0], device=DEV) if with_sink else None
+    got, general = _both(case, H, {"scale": 0.1, "window": window, "sink": sink})
+    want = _formula(case, H, 0.1, window, sink)
+    assert torch.isnan(want).any() == (bad != "score of minus infinity")
+    assert torch.equal(torch.isnan(got).cpu(), torch.isnan(want))
+    fine = ~torch.isnan(want)
+    assert (got.double().cpu() - want)[fine].abs().max().item() < 2e-5      # the bound of test_prompt_attention_f32
+    if bad != "key":                                        # (the general kernel gives a NaN score no weight)
+        assert torch.equal(torch.isnan(got), torch.isnan(general))
+
+
 # ---- one small matrix per group of rows or columns ---------------------------------------------------------------------
 @pytest.mark.parametrize("sizes,N,K", [([1, 0, 2, 1], 33, 132), ([3, 3, 3], 4, 4), ([64, 65, 0, 127, 1], 130, 100), ([200], 64, 64), ([5, 9], 1000, 768)])
 def test_expert_product_f32(sizes, N, K):
