@@ -36,6 +36,25 @@ def test_gemm_f32(M, N, K, form, splits):
     assert bool(((out.double() - gelu).abs() <= 2 * bound + 1e-6 * (1 + want.abs())).all())     # the slope stays below 1.13
 
 
+@pytest.mark.parametrize("form,splits", [(0, 1), (1, 1), (4, 1), (4, 2)])
+@pytest.mark.parametrize("M,N,K", [(1, 5, 4), (2, 9, 132), (4, 40, 132), (8, 33, 1600), (9, 33, 260)])
+def test_gemm_f32_infinity_at_the_end_of_a_row(M, N, K, form, splits):
+    """An infinite activation among the last four k: plus or minus infinity by the weight's sign, nothing for the other rows."""
+    from sandyrt_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    finite = torch.empty(M, N, device=DEV)
+    ops.gemm_f32(a, w, None, finite, form=form, splits=splits)
+    for at in (K - 4, K - 1):
+        b = a.clone()
+        b[M - 1, at] = float("inf")
+        out = torch.full((M, N), float("nan"), device=DEV)
+        ops.gemm_f32(b, w, None, out, form=form, splits=splits)
+        assert torch.equal(out[M - 1], torch.sign(w[:, at]) * float("inf"))
+        assert torch.equal(out[:M - 1], finite[:M - 1])
+
+
 def test_gemm_f32_refuses_what_it_cannot_load():
     from sandyrt_b200.csrc import ops
 
