@@ -200,6 +200,25 @@ def test_expert_product_f32(sizes, N, K):
     assert bool(((out.double().cpu() - want).abs() <= 2 * torch.relu(z) * off + off ** 2 + 2.0 ** -23 * want).all())
 
 
+@pytest.mark.parametrize("sizes", [[1, 0, 2, 1], [64, 65, 0, 127]])
+@pytest.mark.parametrize("K", [4, 132, 260])
+def test_expert_product_f32_infinity_at_the_end_of_a_row(sizes, K):
+    """As in the dense products, for groups of few rows and of many."""
+    from sandyrt_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(K)
+    n, G, N = sum(sizes), len(sizes), 40
+    a, w = torch.randn(n, K, generator=g), torch.randn(G, N, K, generator=g)
+    start = torch.tensor([0] + list(np.cumsum(sizes)), dtype=torch.int32)
+    r = types.SimpleNamespace(n_experts=G, n_tokens=n, top=1, group_start=start.to(DEV), entry_of_slot=torch.arange(n, dtype=torch.int32).to(DEV))
+    a[n - 1, K - 2] = float("inf")
+    out = torch.full((n, N), float("nan"), device=DEV)
+    ops.expert_product(r, a.to(DEV), w.view(G * N, K).to(DEV), out, gather=True)
+    last = max(i for i, size in enumerate(sizes) if size)
+    assert torch.equal(out[n - 1].cpu(), torch.sign(w[last, :, K - 2]) * float("inf"))
+    assert torch.isfinite(out[:n - 1]).all()
+
+
 @pytest.mark.parametrize("T", [1, 4, 5, 64, 65, 150])
 def test_head_product_f32(T):
     from sandyrt_b200.csrc import ops
