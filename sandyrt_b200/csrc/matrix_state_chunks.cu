@@ -6,10 +6,13 @@
 //                lower triangular system of matrix_state.cu solved for both right-hand sides,
 //                    U = L^-1 (beta v),   W = L^-1 (beta exp(G) k),   u = U - W S0
 //                the rest is linear in the state before the chunk, S0:
-//                    S  = A S0 + N,       A = exp(G_31) I - K'^T W,  N = K'^T U,  K'_j = exp(G_31 - G_j) k_j
+//                    S  = exp(G_31) S0 + (N - A S0),   A = K'^T W,  N = K'^T U,  K'_j = exp(G_31 - G_j) k_j
 //                    o  = Q S0 + P U,     Q_t = exp(G_t) q_t - sum_j P(t, j) W_j,  P(t, j) = r(t, j) (q_t . k_j)
-//                so a chunk costs the walk one [d, d] x [d, columns] product and no triangular system.
-//   delta_chunk_prepare_kernel   a block a (chunk, head, request): A, N, Q, and P U into the output
+//                so a chunk costs the walk one [d, d] x [d, columns] product and no triangular system.  A S0 is summed
+//                by itself: started from N, or with exp(G_31) inside A, each of its 64 products would be rounded at the size
+//                of the whole state (error of the state against 64 bits beside the walk's, mean over 144 settings of length,
+//                keys, write strength and decay: 1.12 times, up to 1.65; so 0.74 times, up to 1.03).
+//   delta_chunk_prepare_kernel   a block a (chunk, head, request): A, N, Q, exp(G_31), and P U into the output
 //   delta_chunk_states_kernel    a block a (request, head, 16 columns) walks the chunks and leaves S0 of each
 //   delta_chunk_output_kernel    a block a (chunk, head, request): the output plus Q S0
 //
@@ -22,7 +25,7 @@
 //
 // All float32, the inputs in the projection's type.  The kernels that walk with everything in one block (matrix_state.cu) spend 9
 // and 6 us a chunk, whatever the head count; they keep sizes above 64.  Alone, us, those -> these: 2 x 1,024 tokens, 12 heads, delta
-// rule 278 -> 113 (52 / 61 / 15), 24 heads 400 -> 199; 3 heads of 64 x 128, matrix memory 179 -> 37; one request of 96 tokens 29 -> 25
+// rule 278 -> 115, 24 heads 400 -> 201; 3 heads of 64 x 128, matrix memory 179 -> 37; one request of 96 tokens 29 -> 25
 // and 22 -> 21, of 64 21 / 23 and 16 / 21.  The walk is bound by its chain (a product of 64 x 64 x 16 and two barriers a chunk), the
 // others by shared-memory loads beside the fmas.
 #include "common.cuh"
@@ -116,9 +119,9 @@ __device__ __forceinline__ void dots(const float* X, const float* Y, float (&out
 __device__ __forceinline__ long long place(int t0, int s, int chunk) { return (long long)(t0 / CC + s + chunk); }
 
 // ---- delta rule ----------------------------------------------------------------------------------------------
-// Of a (place, head): A transposed [column][row] (D * D), Q transposed [row of the state][token] (D * CC), N [D][ep], ep the value
-// size in whole 64s; the states overwrite N.
-__host__ __device__ constexpr long long delta_floats(int ep) { return (long long)D * D + D * CC + (long long)D * ep; }
+// Of a (place, head): -A transposed [column][row] (D * D), Q transposed [row of the state][token] (D * CC), N [D][ep], ep the value
+// size in whole 64s, and exp(G_31) (and 31 floats that keep the parts on 128-byte boundaries); the states overwrite N.
+__host__ __device__ constexpr long long delta_floats(int ep) { return (long long)D * D + D * CC + (long long)D * ep + 32; }
 
 // grid (chunks x 64s of columns, heads, requests), 256 threads.
 __global__ void __launch_bounds__(256, 2)
@@ -238,7 +241,6 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, int ld, const float* _
 #pragma unroll
             for (int r = 0; r < 8; r++) put4(N + (size_t)(i0 + r) * tiles * 64 + col0 + c4, sum[r][0].x, sum[r][0].y, sum[r][1].x, sum[r][1].y);
         } else {
-            const float all = expf(G[CC - 1]);
             float a[4][8];
 #pragma unroll
             for (int r = 0; r < 8; r++) { a[0][r] = sum[r][0].x; a[1][r] = sum[r][0].y; a[2][r] = sum[r][1].x; a[3][r] = sum[r][1].y; }
@@ -246,16 +248,17 @@ delta_chunk_prepare_kernel(const float* __restrict__ qkv, int ld, const float* _
             for (int c = 0; c < 4; c++) {
                 const int i = c4 - D + c;
 #pragma unroll
-                for (int r = 0; r < 8; r++) a[c][r] = (i0 + r == i ? all : 0.0f) - a[c][r];
+                for (int r = 0; r < 8; r++) a[c][r] = -a[c][r];
                 put4(mine + i * D + i0, a[c][0], a[c][1], a[c][2], a[c][3]);
                 put4(mine + i * D + i0 + 4, a[c][4], a[c][5], a[c][6], a[c][7]);
             }
+            if (tid == D / 4) put4(mine + D * D + D * CC + D * tiles * 64, expf(G[CC - 1]), 0.0f, 0.0f, 0.0f);     // the first such thread
         }
     }
     pdl_launch_dependents();
 }
 
-constexpr int WALK_STAGES = 3, WALK_STAGE = D * D + D * COLS;       // floats: A and 16 columns of N
+constexpr int WALK_STAGES = 3, WALK_STAGE = D * D + D * COLS + 32;   // floats: A, 16 columns of N, the decay
 
 // grid (requests, heads, 16s of columns), 128 threads: four rows and two columns of the state each.
 __global__ void __launch_bounds__(128)
@@ -282,6 +285,7 @@ delta_chunk_states_kernel(float* __restrict__ scratch, float* __restrict__ state
                 const int x = tid + u * 128, i = x / (COLS / 4), c4 = x % (COLS / 4) * 4;
                 copy_16(to + D * D + x * 4, from + D * D + D * CC + (size_t)i * ep + col0 + c4);
             }
+            if (tid == 0) copy_16(to + D * D + D * COLS, from + D * D + D * CC + D * ep);
         }
         commit_group();
     };
@@ -291,6 +295,10 @@ delta_chunk_states_kernel(float* __restrict__ scratch, float* __restrict__ state
         const int c = x / D, i = x % D;
         S[i * COLS + c] = (i < d && col0 + c < e) ? St[(size_t)(col0 + c) * d + i] : 0.0f;
     }
+    auto at = [&](int i, int c) { return i < d && col0 + c < e ? St[(size_t)(col0 + c) * d + i] : 0.0f; };
+    float2 own[4];                              // this thread's part of the state
+#pragma unroll
+    for (int r = 0; r < 4; r++) own[r] = make_float2(at(r0 + r, c0), at(r0 + r, c0 + 1));
     for (int c = 0; c < chunks; c++) {
         wait_groups<1>();
         __syncthreads();                        // this chunk's A and N are there, the state is whole
@@ -303,9 +311,13 @@ delta_chunk_states_kernel(float* __restrict__ scratch, float* __restrict__ state
             const int x = tid + u * 128, i = x / (COLS / 4), c4 = x % (COLS / 4) * 4;
             *reinterpret_cast<float4*>(S0 + (size_t)i * ep + col0 + c4) = at4(S + x * 4);
         }
-        float2 acc[4];
+        float2 acc[4], n4[4];
 #pragma unroll
-        for (int r = 0; r < 4; r++) acc[r] = *reinterpret_cast<const float2*>(N + (r0 + r) * COLS + c0);
+        for (int r = 0; r < 4; r++) {
+            acc[r] = make_float2(0.0f, 0.0f);
+            n4[r] = *reinterpret_cast<const float2*>(N + (r0 + r) * COLS + c0);
+        }
+        const float2 decay = make_float2(N[D * COLS], N[D * COLS]);
 #pragma unroll 8
         for (int i = 0; i < D; i++) {
             const float4 a = at4(A + i * D + r0);
@@ -315,9 +327,11 @@ delta_chunk_states_kernel(float* __restrict__ scratch, float* __restrict__ state
             acc[2] = __ffma2_rn(make_float2(a.z, a.z), sv, acc[2]);
             acc[3] = __ffma2_rn(make_float2(a.w, a.w), sv, acc[3]);
         }
+#pragma unroll
+        for (int r = 0; r < 4; r++) own[r] = __ffma2_rn(decay, own[r], __fadd2_rn(n4[r], acc[r]));
         __syncthreads();                        // everyone has read the state
 #pragma unroll
-        for (int r = 0; r < 4; r++) *reinterpret_cast<float2*>(S + (r0 + r) * COLS + c0) = acc[r];
+        for (int r = 0; r < 4; r++) *reinterpret_cast<float2*>(S + (r0 + r) * COLS + c0) = own[r];
     }
     pdl_launch_dependents();
     __syncthreads();
