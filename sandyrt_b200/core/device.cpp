@@ -15,6 +15,18 @@ void cuda_check(cudaError_t e, const char* what) {
 DeviceBuffer::DeviceBuffer(size_t bytes) : bytes_(bytes) {
     cuda_check(cudaMalloc(&ptr_, std::max<size_t>(bytes, 16)), "allocating device memory");
 }
+DeviceBuffer DeviceBuffer::if_there_is_room(size_t bytes) {
+    DeviceBuffer b;
+    const cudaError_t e = cudaMalloc(&b.ptr_, std::max<size_t>(bytes, 16));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();             // answered here: no launch behind this one reports it
+        b.ptr_ = nullptr;
+        return b;
+    }
+    cuda_check(e, "allocating device memory");
+    b.bytes_ = bytes;
+    return b;
+}
 DeviceBuffer::~DeviceBuffer() {
     if (ptr_) cudaFree(ptr_);
 }
@@ -115,11 +127,40 @@ void* Workspace::raw(const std::string& name, size_t bytes) {
         // grow in steps, so that a slowly growing step does not move the buffer every time
         size_t want = std::max<size_t>(bytes, 256);
         if (it != bufs_.end()) want = std::max(want, it->second.bytes() + it->second.bytes() / 2);
-        bufs_[key] = DeviceBuffer(want);
+        DeviceBuffer larger = DeviceBuffer::if_there_is_room(want);
+        if (!larger.get()) {
+            give_back();
+            larger = DeviceBuffer(want);
+        }
+        bufs_[key] = std::move(larger);
         version_++;
         it = bufs_.find(key);
     }
     return it->second.get();
+}
+
+void* Workspace::spare(const std::string& name, size_t bytes) {
+    Spare& s = spares_[name];
+    if (s.buffer.get() && s.buffer.bytes() >= bytes) return s.buffer.get();
+    if (bytes >= s.refused) return nullptr;
+    if (s.buffer.get()) version_++;
+    s.buffer = DeviceBuffer();          // nothing in it outlives the call it was asked for
+    s.buffer = DeviceBuffer::if_there_is_room(bytes);
+    if (s.buffer.get()) version_++;
+    else s.refused = bytes;
+    return s.buffer.get();
+}
+
+bool Workspace::give_back() {
+    bool any = false;
+    for (auto& [name, s] : spares_)
+        if (s.buffer.get()) {
+            s.refused = std::min(s.refused, s.buffer.bytes());
+            s.buffer = DeviceBuffer();
+            any = true;
+        }
+    if (any) version_++;
+    return any;
 }
 
 }  // namespace sandy

@@ -47,6 +47,7 @@ class DeviceBuffer {
 public:
     DeviceBuffer() = default;
     explicit DeviceBuffer(size_t bytes);
+    static DeviceBuffer if_there_is_room(size_t bytes);     // empty (get() null) where the device has no memory left
     ~DeviceBuffer();
     DeviceBuffer(DeviceBuffer&& o) noexcept : ptr_(o.ptr_), bytes_(o.bytes_) { o.ptr_ = nullptr; o.bytes_ = 0; }
     DeviceBuffer& operator=(DeviceBuffer&& o) noexcept;
@@ -118,9 +119,18 @@ class Workspace {
 public:
     Tensor get(const std::string& name, int64_t rows, int64_t cols, DType dtype);
     void* raw(const std::string& name, size_t bytes);
+    // A buffer that a step can do without: null where the device has no room for it, which is remembered (so much is not asked
+    // for again).  It is given back when a buffer that a step cannot do without finds no room.
+    void* spare(const std::string& name, size_t bytes);
     uint64_t version() const { return version_; }      // bumped whenever a buffer moves; recorded graphs check it
 private:
+    struct Spare {
+        DeviceBuffer buffer;
+        size_t refused = SIZE_MAX;      // no room was found for this much
+    };
+    bool give_back();
     std::map<std::pair<std::string, int>, DeviceBuffer> bufs_;
+    std::map<std::string, Spare> spares_;
     uint64_t version_ = 0;
 };
 

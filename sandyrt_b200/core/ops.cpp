@@ -1136,7 +1136,7 @@ void embed_bigram(const Launch& l, const StepSeqs& s, const int* ids, const int*
 namespace {
 // Scratch of the recurrences that form all chunks side by side (matrix_state_chunks.cu), or null where a step stays with the
 // kernels that walk its chunks one by one: heads above 64, portions below 96 tokens (alone, us, walk / side by side: 64 tokens 21 /
-// 23 and 16 / 21, 96 tokens 29 / 25 and 22 / 21), and steps whose scratch would pass half a gigabyte.
+// 23 and 16 / 21, 96 tokens 29 / 25 and 22 / 21), and steps whose scratch would pass half a gigabyte or finds no room on the device.
 float* chunk_scratch(int kind, const StepSeqs& s, int n_heads, int qk_dim, int v_dim, int max_q_len, Workspace& ws) {
     constexpr int kWideFrom = 96;
     constexpr long long kMostFloats = 128ll << 20;
@@ -1144,7 +1144,7 @@ float* chunk_scratch(int kind, const StepSeqs& s, int n_heads, int qk_dim, int v
     static auto need = SANDY_KERNEL(matrix_state_chunks, sandy_matrix_chunks_scratch);
     const long long floats = need(kind, s.n_tokens, s.n_seqs, n_heads, v_dim);
     if (floats > kMostFloats) return nullptr;
-    return (float*)ws.raw("matrix_chunks", (size_t)floats * sizeof(float));
+    return (float*)ws.spare("matrix_chunks", (size_t)floats * sizeof(float));
 }
 }  // namespace
 
