@@ -1007,7 +1007,13 @@ SANDY_EXPORT int sandy_engine_synchronize(void* engine) {
 }
 SANDY_EXPORT void* sandy_engine_stream(void* engine) { return ((EngineBox*)engine)->engine->stream(); }
 SANDY_EXPORT int sandy_engine_release(void* engine, long long rid) {
-    return guarded([&]() { ((EngineBox*)engine)->engine->release((RequestId)rid); return 0; }, 1);
+    return guarded(
+        [&]() {
+            if (!engine) throw ValueError("a null handle was given for an 'engine'");
+            ((EngineBox*)engine)->engine->release((RequestId)rid);
+            return 0;
+        },
+        1);
 }
 SANDY_EXPORT int sandy_engine_mark(void* engine, int which) {
     return guarded(

@@ -122,8 +122,9 @@ int sandy_engine_decode_burst_async(void* engine, int n_requests, const long lon
 int sandy_engine_burst_tokens(void* engine, int burst, int* out);      /* out: [n_steps, n_requests] */
 int sandy_engine_synchronize(void* engine);
 void* sandy_engine_stream(void* engine);
-/* device time in milliseconds between two marks on the engine's stream */
+/* gives a request's pages and state slot back: 0, or 1 and an error (an unknown request, a null engine) */
 int sandy_engine_release(void* engine, long long rid);
+/* device time in milliseconds between two marks on the engine's stream */
 int sandy_engine_mark(void* engine, int which);
 /* Keeps the engine's stream busy for so many microseconds (a kernel that only waits), so that what the
    host queues meanwhile runs back to back behind it: for timing the device's share of a step. */

@@ -1,6 +1,9 @@
 """The cache manager's host side: no page lost, held twice or freed twice, under random
 orders of requests; groups with windows give pages back; state slots (no GPU)."""
+import os
 import random
+import subprocess
+import sys
 
 import pytest
 
@@ -187,3 +190,13 @@ def test_small_product_rule():
     assert small_gemm_kernel(8, 1600, 6400) == "split_k" and small_gemm_kernel(8, 1024, 4096) == "streaming"
     assert small_gemm_kernel(64, 4800, 1600) == "split_k" and small_gemm_kernel(32, 4800, 1600) == "streaming"
     assert small_gemm_kernel(64, 3072, 1024) == "streaming"
+
+
+def test_releasing_on_a_null_engine_is_an_error_and_no_crash():
+    """In a process of its own: a crash there ends that process alone."""
+    code = ("import ctypes\nfrom sandyrt_b200 import core\n"
+            "assert core.lib().sandy_engine_release(None, ctypes.c_longlong(0)) == 1\n"
+            "try:\n    core.raise_last_error()\nexcept ValueError as e:\n    assert 'null handle' in str(e)\n    print('refused')\n")
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                          cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert done.returncode == 0 and "refused" in done.stdout, (done.returncode, done.stderr[-500:])
