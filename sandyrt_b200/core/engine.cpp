@@ -254,6 +254,12 @@ Engine::Prepared Engine::prepare(const std::vector<StepEntry>& entries, const st
     c.host_slots = slots;
     c.max_q_len = max_q;
     c.max_kv_len = max_kv + extra;
+    // What the attention of a mixed step chooses its launches by (bfloat16 only).  Part of the graph's key, so rounded down: nothing
+    // below eight, then powers of two.
+    if (dtype_ == DType::BF16 && max_q > 1) {
+        const int singles = (int)std::count(q_lens.begin(), q_lens.end(), 1);
+        for (int n = 8; n <= singles; n *= 2) c.n_single = n;
+    }
     c.launch.stream = stream_;
     c.launch.status = (int*)status_.get();
     c.launch.kernel_status = (int*)status_.get() + 1;
@@ -269,7 +275,7 @@ Engine::Prepared Engine::prepare(const std::vector<StepEntry>& entries, const st
     // steps always do, prompt steps do when the token budget is filled the same way.  A burst is
     // recorded whole (all its steps in one graph), in two copies used in turn: a graph that is
     // launched again while it still runs makes the host wait for it.
-    p.key = Key{T, S, R, max_q, max_blocks, sampling ? 1 : 0, n_burst, n_burst ? burst_flip_ : 0, staging_->generation};
+    p.key = Key{T, S, R, max_q, max_blocks, sampling ? 1 : 0, n_burst, n_burst ? burst_flip_ : 0, staging_->generation, c.n_single};
     return p;
 }
 

@@ -489,6 +489,15 @@ int decode_splits(int n_tokens, int n_heads, int max_kv, int sms) {
     return (n == 6 || n == 7) ? 5 : n;
 }
 
+// From how many (token, head) pairs on the single tokens of a mixed step leave the prompt kernel, where each takes a tile of 128 queries with one
+// row in it, for a launch of the decode kernel.  Alone, us, one launch / two, contexts of about 100, 400 and 900 tokens beside a portion
+// of 480: 12 heads x 8 tokens 14.3 / 16.9, 15.9 / 18.0, 23.6 / 20.0; x 16 17.9 / 18.9, 20.1 / 21.3, 27.9 / 28.2; x 32 25.0 / 24.2, 31.5 /
+// 28.6, 46.7 / 40.0; 16 heads x 8 15.1 / 18.0, 16.8 / 19.4, 24.9 / 21.8; x 16 20.6 / 20.4, 25.9 / 23.7, 39.0 / 31.7; 25 heads x 12 22.4 /
+// 21.3, 28.8 / 25.0, 42.1 / 34.6.  Tables of up to 128 keys (contexts of 100, a portion of 64): 16 heads x 16 8.7 / 11.5, x 32 15.7 /
+// 13.3; 12 heads x 32 13.7 / 13.8; 25 heads x 16 13.8 / 12.3.  How many portions there are makes no difference to that (16 heads x 16
+// beside 4, 8, 16 and 32 portions of 32 tokens: 16.5 / 15.1, 17.7 / 15.3, 21.6 / 17.0, 27.2 / 23.8).
+bool singles_apart(int singles, int n_heads, int seen_keys) { return singles * n_heads >= (seen_keys > 128 ? 256 : 384); }
+
 namespace {
 constexpr int kClusterMaxSplits = 8;
 // From this many (token, head) pairs on, a decode step's attention streams pages through shared
@@ -497,10 +506,6 @@ constexpr int kClusterMaxSplits = 8;
 // but a whole decode step of 8 x 12 pairs (its cache fits in L2) took 414 against 400 us and one of
 // 1 x 12 pairs 356 against 333 us, the register kernel starting sooner.
 constexpr int kBulkMinPairs = 256;
-
-// Single tokens of a mixed step from which they leave the prompt kernel for a launch of the decode kernel (GPT-2 medium, four layers,
-// 32 of them behind 100 to 700 tokens beside a portion of 480: a step 579 -> 530 us; fewer than eight cost less than the launch).
-constexpr int kSinglesApart = 8;
 
 bool decode_head_dim(DType dt, int d) {
     if (d == 16 || d == 32 || d == 64 || d == 128) return true;
@@ -542,14 +547,11 @@ void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const K
     if (s.max_q_len > 1 && q.dtype == DType::BF16 && d <= 128) {
         static const bool use_tc = env_int("SANDYRT_PREFILL_TC", 1) != 0;     // 0 keeps every head size on the mma.sync kernel
         if (use_tc && d == 64 && !db) {                       // (the tcgen05 kernel has no form for a bias by distance)
-            // Single tokens beside portions: a tile of 128 queries with one row in it costs as much as a full one, so where a
-            // step holds enough of them they go to the decode kernel.  What is known of a step that a recorded graph may
-            // serve again is its tokens, its requests and its longest portion: at most so many requests bring one token.
-            const int singles = s.n_seqs - (T - s.n_seqs + s.max_q_len - 2) / (s.max_q_len - 1);
+            const int singles = s.n_single;
             const int seen = window > 0 ? std::min(window + keep, s.max_blocks * c.page_size) : s.max_blocks * c.page_size;
             const int splits = singles > 0 ? std::min(decode_splits(singles, n_heads, seen), kClusterMaxSplits) : 1;
             static auto max_keys_fn = SANDY_KERNEL(attention_decode_mma, sandy_decode_attention_mma_max_keys);
-            const bool apart = !ruled && singles >= kSinglesApart && 2 * singles >= s.n_seqs && s.n_seqs <= 65535 && seen <= max_keys_fn(splits, c.page_size);
+            const bool apart = !ruled && singles_apart(singles, n_heads, seen) && s.n_seqs <= 65535 && seen <= max_keys_fn(splits, c.page_size);
             static auto fn = SANDY_KERNEL(attention_prefill_tc, sandy_prefill_attention_tc_portions);
             OpTimer timer(l, "attention, prompt (tcgen05)", attn_bytes, attn_flops);
             const int code = fn(q.data, (int)q.ld, c.k, c.v, c.page_stride, s.block_table, s.max_blocks, s.q_start, s.kv_before,

@@ -124,6 +124,7 @@ void kv_append(const Launch& l, const Tensor& k_src, const Tensor& v_src, const 
 // What an attention launch needs to know about the step.
 struct AttentionStep {
     int n_tokens = 0, n_seqs = 0, max_q_len = 0;
+    int n_single = 0;       // at least so many requests beside portions bring one token (the launches' shapes may depend on it)
     const int* token_seq = nullptr;
     const int* positions = nullptr;
     const int* q_start = nullptr;
@@ -165,6 +166,9 @@ constexpr int64_t kSharedKvMinTriples = 40000;      // tokens x heads x keys (th
 void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const KVView& cache, Tensor& out, int n_heads,
                float scale, int window, Workspace& ws, const AttentionExtras* extras = nullptr);
 int decode_splits(int n_tokens, int n_heads, int max_kv, int sms = 0);
+// Whether a mixed step's single tokens take a launch of the decode kernel of their own (bfloat16, heads of 64); seen_keys: the most
+// keys a token may see.
+bool singles_apart(int singles, int n_heads, int seen_keys);
 
 // ---- RMS norms and what goes with them (rmsnorm.cu, elementwise.cu) ------------------------------------------
 struct StepSeqs {                                                  // the step's requests, as kernels with a state per request need them

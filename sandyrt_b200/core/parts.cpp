@@ -10,6 +10,7 @@ ops::AttentionStep StepContext::attention_step(int group, int window, int keep_f
     s.n_tokens = n_tokens;
     s.n_seqs = n_seqs;
     s.max_q_len = max_q_len;
+    s.n_single = n_single;
     s.token_seq = token_seq;
     s.positions = positions;
     s.q_start = q_start;

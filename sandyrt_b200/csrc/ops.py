@@ -263,6 +263,13 @@ def paged_attention(q, k_cache, v_cache, block_table, token_seq, positions, out,
 _DECODE_HEAD_DIMS = {torch.bfloat16: (16, 32, 64, 128, 256), torch.float32: (16, 32, 64, 128)}
 
 
+def singles_apart(singles: int, n_heads: int, seen_keys: int) -> bool:
+    """Whether a mixed step's single tokens take a launch of the decode kernel of their own (bfloat16, heads of 64)."""
+    from .. import core
+
+    return core.call("global", None, "singles_apart", singles=singles, n_heads=n_heads, seen_keys=seen_keys)
+
+
 def decode_splits(n_tokens: int, n_heads: int, max_kv: int, sms: Optional[int] = None) -> int:
     """How many blocks share the keys of one (token, head) pair in a decode step (the host library's
     rule, core/ops.cpp): about four blocks an SM in all, more where a block would walk more than some 256

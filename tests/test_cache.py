@@ -177,6 +177,16 @@ def test_decode_splits_at_the_measured_points():
     assert at(64, 600, heads=25) == 1           # GPT-2 xl, 64 requests: one block a pair
 
 
+def test_single_tokens_take_a_launch_of_their_own_where_it_was_measured_faster():
+    """The rule's answers where both were timed (a launch over everything against two)."""
+    from sandyrt_b200.csrc.ops import singles_apart
+
+    at = lambda singles, heads, keys: singles_apart(singles, heads, keys)
+    assert not any(at(n, h, 512) for n, h in ((0, 16), (8, 6), (32, 6), (8, 12), (16, 12), (8, 16)))
+    assert all(at(n, h, 512) for n, h in ((64, 6), (32, 12), (16, 16), (32, 16), (16, 25)))
+    assert not at(16, 16, 128) and at(32, 16, 128) and at(32, 12, 128) and at(16, 25, 128)
+
+
 def test_small_product_rule():
     """Which kernel takes a product of up to 64 rows is a rule of its shape (the kernels add in different
     orders, so it must not depend on a timing)."""

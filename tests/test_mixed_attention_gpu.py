@@ -28,3 +28,98 @@ def test_portions_and_single_tokens(H, Hkv, page_size, window, keep, splits, seq
     ops.check_kernel_status(DEV)
     want = _want(case, H, Hkv, 0.1, window, keep, bool(keep), None if gate is None else gate.double().cpu(), 59)
     assert (out.double().cpu() - want).abs().max().item() < ATT_TOL[torch.bfloat16] * 1.5
+
+
+# ---- through the engine -----------------------------------------------------------------------------------------
+HEADS, WIDTH, LAYERS, VOCAB = 16, 1024, 2, 301
+
+
+@pytest.fixture(scope="module")
+def wide(tmp_path_factory):
+    from conftest import make_model_dir
+    from plain_gpt2 import PlainGPT2
+
+    folder = make_model_dir(dict(architectures=["GPT2LMHeadModel"], model_type="gpt2", n_layer=LAYERS, n_embd=WIDTH, n_head=HEADS, n_inner=512,
+                                 vocab_size=VOCAB, n_positions=512, layer_norm_epsilon=1e-5, activation_function="gelu_new"),
+                            str(tmp_path_factory.mktemp("mixed") / "model"), seed=8)
+    return folder, PlainGPT2(folder, "bf16")
+
+
+class _Running:
+    """An engine and what its requests have been fed."""
+
+    def __init__(self, wide, contexts, seed):
+        from sandyrt_b200.engine.step import Engine
+        from sandyrt_b200.models.model import load_model
+
+        self.plain = wide[1]
+        self.eng = Engine(load_model(wide[0], device="cuda:0", dtype=torch.bfloat16), max_tokens=8192, max_requests=48)
+        self.eng.cache.device_caches.poison()
+        self.rng = np.random.default_rng(seed)
+        self.fed = {}
+        for r, n in enumerate(contexts):
+            self.step([(r, n)], check=False)
+
+    def step(self, portions, check=True):
+        """portions: (request, tokens) in the step's order; every request's last row against the plain model's."""
+        from sandyrt_b200.engine.step import StepEntry
+
+        entries = []
+        for r, n in portions:
+            ids = self.rng.integers(0, VOCAB, size=n).tolist()
+            self.fed[r] = self.fed.get(r, []) + ids
+            entries.append(StepEntry(r, ids, [n - 1]))
+        got = self.eng.step(entries).cpu().double().numpy()
+        if check:
+            for (r, n), row in zip(portions, got):
+                want = self.plain.logits(self.fed[r], [len(self.fed[r]) - 1])[0].astype(np.float64)
+                # two layers of bfloat16 roundings in another order: 5e-3 of the row; a row that no launch wrote is off by its size
+                assert np.linalg.norm(row - want) < 2e-2 * np.linalg.norm(want), (r, n, portions)
+        return self.eng.last_launches
+
+
+def _contexts(n):
+    return [3 + 7 * i % 61 for i in range(n - 1)] + [150]           # one behind a table of more than 128 keys
+
+
+@pytest.mark.parametrize("singles", [15, 16, 20, 33])
+def test_engine_steps_of_single_tokens_beside_a_portion(wide, singles):
+    """Below and from 256 (token, head) pairs on; the same counts with the portion first, last and in the middle, so that one
+    recording serves requests that have changed places."""
+    run = _Running(wide, _contexts(singles), seed=singles)
+    launches, replays = [], run.eng.graph_replays
+    for step, at in enumerate((singles, 0, singles // 2, 1)):
+        portions = [(r, 1) for r in range(singles)]
+        portions.insert(at, (f"new {step}", 37))
+        launches.append(run.step(portions))
+        run.eng.release(f"new {step}")
+    assert run.eng.graph_replays - replays == 3 and len(set(launches)) == 1
+    alone = _Running(wide, [3], seed=1)
+    one = alone.step([(0, 1), ("new", 37)])
+    assert launches[0] - one == (LAYERS if singles >= 16 else 0)
+
+
+def test_engine_step_without_single_tokens_takes_no_second_launch(wide):
+    """Ragged prompts whose counts would allow for many single tokens, beside prompts with as many tokens and no room for one."""
+    run = _Running(wide, [2], seed=5)
+    launches = []
+    for lengths in ([270] + [20] * 24, [30] * 25):
+        for time in range(2):                               # (a product's first step at a new size tries its kernels)
+            requests = [f"{time} {i}" for i in range(25)]
+            n = run.step(list(zip(requests, lengths)))
+            for r in requests:
+                run.eng.release(r)
+                del run.fed[r]
+        launches.append(n)
+    assert launches[0] == launches[1]
+
+
+def test_engine_recording_is_not_shared_by_steps_with_and_without_single_tokens(wide):
+    """Equal tokens, requests and longest portion: sixteen single tokens beside two portions, then portions alone."""
+    run = _Running(wide, [150] + [4] * 17, seed=6)
+    for _ in range(2):
+        run.step([(r, 1) for r in range(16)] + [(16, 40), (17, 24)])
+    for _ in range(2):
+        run.step([(0, 40)] + [(r, 2) for r in range(1, 7)] + [(r, 3) for r in range(7, 13)] + [(r, 2) for r in range(13, 18)])
+    for _ in range(2):
+        run.step([(r, 1) for r in range(2, 18)] + [(1, 24), (0, 40)])
