@@ -344,8 +344,8 @@ int launch_stream(const Product& p, cudaStream_t stream) {
     return sandy_launch(gemm_f32_stream_kernel<MB, AHEAD, BLOCKS>, grid, block, 0, stream, p);
 }
 
-// Up to here the weights are streamed (alone, weights from HBM, us, stream / best tile: 24 rows 768 x 768 4.8 / 6.0, 3,072 x
-// 768 10.1 / 11.5, 768 x 3,072 10.8 / 15.3, 50,257 x 768 129 / 126; 32 rows 6.8 / 6.0, 17.3 / 11.6, 18.8 / 15.4, 171 / 128).
+// Up to here the weights are streamed (alone, weights from HBM, us, stream / best tile: 24 rows 768 x 768 4.0 / 5.7, 3,072 x
+// 768 8.4 / 11.4, 768 x 3,072 8.9 / 15.3, 50,257 x 768 99 / 120; 28 rows 5.7 / 5.8, 12.7 / 11.5, 14.7 / 15.4, 125 / 121).
 constexpr int STREAM_MAX_ROWS = 24;
 
 // SMs that clusters of s blocks, one block an SM, can cover: groups of SMs that share a crossbar are not all multiples of s
