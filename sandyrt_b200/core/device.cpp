@@ -120,6 +120,24 @@ Tensor Workspace::get(const std::string& name, int64_t rows, int64_t cols, DType
     return t;
 }
 
+std::vector<Tensor> Workspace::get_together(const std::string& name, int64_t rows, const std::vector<std::pair<int64_t, DType>>& cols) {
+    std::vector<size_t> at;
+    size_t bytes = 0;
+    for (const auto& [n, dtype] : cols) {
+        at.push_back(bytes);
+        bytes += ((size_t)(rows * n) * dtype_size(dtype) + 255) / 256 * 256;
+    }
+    char* base = (char*)raw(name, bytes);
+    std::vector<Tensor> out(cols.size());
+    for (size_t i = 0; i < cols.size(); i++) {
+        out[i].data = base + at[i];
+        out[i].dtype = cols[i].second;
+        out[i].rows = rows;
+        out[i].cols = out[i].ld = cols[i].first;
+    }
+    return out;
+}
+
 void* Workspace::raw(const std::string& name, size_t bytes) {
     auto key = std::make_pair(name, 0);
     auto it = bufs_.find(key);

@@ -504,14 +504,14 @@ public:
         const int64_t tail_off = (int64_t)H_ * e_ * d_;
         ops::StepSeqs seqs{ctx.n_tokens, ctx.n_seqs, ctx.token_seq, ctx.q_start, ctx.seq_slots};
         ops::DeltaShape ds{H_, G_, d_, e_, taps_};
-        Tensor qkv = ws.get("delta_qkv", T, channels_, DType::F32);
-        Tensor bg = ws.get("delta_gates", T, 2 * H_, DType::F32);
+        const int64_t He = (int64_t)H_ * e_;
+        std::vector<Tensor> parts = ws.get_together("delta_rows", T, {{channels_, DType::F32}, {2 * H_, DType::F32}, {He, DType::F32},
+                                                                      {He, ctx.compute_dtype}});
+        Tensor &qkv = parts[0], &bg = parts[1], &read = parts[2], &normed = parts[3];
         ops::delta_prepare(l, seqs, ds, wide, conv_.view, &gates, (const float*)a_log_.view.data, (const float*)dt_bias_.view.data,
                            state, tail_off, 1.0f / std::sqrt((float)d_), qkv, &bg, ctx.max_q_len);
         if (ctx.max_q_len != 1) ops::conv_tail(l, seqs, ds, wide, state, tail_off);
-        Tensor read = ws.get("mix_read", T, (int64_t)H_ * e_, DType::F32);
         ops::delta_scan(l, seqs, ds, qkv, bg, state, read, ctx.max_q_len, *ctx.workspace);
-        Tensor normed = ws.get("delta_normed", T, (int64_t)H_ * e_, ctx.compute_dtype);
         Tensor out_gate = wide.col_range(channels_, n_wide_);
         ops::head_norm_gate(l, read, &gain_.view, &out_gate, ops::GateAct::Silu, 1.0f, eps_, H_, normed);
         out_.run(ctx, nullptr, &normed, x, ops::Act::None, ctx.overwrite ? nullptr : &x);
