@@ -260,8 +260,6 @@ Engine::Prepared Engine::prepare(const std::vector<StepEntry>& entries, const st
         const int singles = (int)std::count(q_lens.begin(), q_lens.end(), 1);
         for (int n = 8; n <= singles; n *= 2) c.n_single = n;
     }
-    // Likewise the attention of float32 portions: up to 32 keys, up to 48, or more.
-    if (dtype_ == DType::F32 && max_q > 1) c.few_keys = c.max_kv_len <= 32 ? 32 : c.max_kv_len <= 48 ? 48 : 0;
     c.launch.stream = stream_;
     c.launch.status = (int*)status_.get();
     c.launch.kernel_status = (int*)status_.get() + 1;
@@ -277,7 +275,7 @@ Engine::Prepared Engine::prepare(const std::vector<StepEntry>& entries, const st
     // steps always do, prompt steps do when the token budget is filled the same way.  A burst is
     // recorded whole (all its steps in one graph), in two copies used in turn: a graph that is
     // launched again while it still runs makes the host wait for it.
-    p.key = Key{T, S, R, max_q, max_blocks, sampling ? 1 : 0, n_burst, n_burst ? burst_flip_ : 0, staging_->generation, c.n_single, c.few_keys};
+    p.key = Key{T, S, R, max_q, max_blocks, sampling ? 1 : 0, n_burst, n_burst ? burst_flip_ : 0, staging_->generation, c.n_single};
     return p;
 }
 

@@ -125,7 +125,7 @@ public:
     size_t recorded_graphs() const { return graphs_.size(); }
 
 private:
-    using Key = std::array<long long, 11>;
+    using Key = std::array<long long, 10>;
     struct Prepared {
         StepContext ctx;
         int* sample = nullptr;             // device: [temperature R | top_k R | top_p R | uniform R]

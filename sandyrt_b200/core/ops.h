@@ -125,7 +125,6 @@ void kv_append(const Launch& l, const Tensor& k_src, const Tensor& v_src, const 
 struct AttentionStep {
     int n_tokens = 0, n_seqs = 0, max_q_len = 0;
     int n_single = 0;       // at least so many requests beside portions bring one token (the launches' shapes may depend on it)
-    int few_keys = 0;       // beside portions no request has more keys than this; 0: nothing is known but the table's width
     const int* token_seq = nullptr;
     const int* positions = nullptr;
     const int* q_start = nullptr;
@@ -170,8 +169,6 @@ int decode_splits(int n_tokens, int n_heads, int max_kv, int sms = 0);
 // Whether a mixed step's single tokens take a launch of the decode kernel of their own (bfloat16, heads of 64); seen_keys: the most
 // keys a token may see.
 bool singles_apart(int singles, int n_heads, int seen_keys);
-// Whether float32 prompt portions stay with the general attention kernel; keys: the most a token may see.
-bool prompt_f32_general(int head_dim, int n_tokens, int n_heads, int keys);
 
 // ---- RMS norms and what goes with them (rmsnorm.cu, elementwise.cu) ------------------------------------------
 struct StepSeqs {                                                  // the step's requests, as kernels with a state per request need them

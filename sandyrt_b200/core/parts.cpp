@@ -11,7 +11,6 @@ ops::AttentionStep StepContext::attention_step(int group, int window, int keep_f
     s.n_seqs = n_seqs;
     s.max_q_len = max_q_len;
     s.n_single = n_single;
-    s.few_keys = few_keys;
     s.token_seq = token_seq;
     s.positions = positions;
     s.q_start = q_start;

@@ -187,16 +187,6 @@ def test_single_tokens_take_a_launch_of_their_own_where_it_was_measured_faster()
     assert not at(16, 16, 128) and at(32, 16, 128) and at(32, 12, 128) and at(16, 25, 128)
 
 
-def test_float32_portions_take_the_attention_kernel_that_was_measured_faster():
-    """The rule's answers where both kernels were timed alone."""
-    from sandyrt_b200.csrc.ops import prompt_f32_general
-
-    assert all(prompt_f32_general(d, n, h, k) for d, n, h, k in ((64, 8, 12, 32), (64, 16, 12, 32), (128, 16, 12, 32), (64, 128, 12, 32),
-                                                                 (16, 33, 4, 48), (16, 71, 4, 48)))
-    assert not any(prompt_f32_general(d, n, h, k) for d, n, h, k in ((16, 100, 4, 128), (16, 64, 4, 128), (64, 48, 12, 48), (64, 8, 12, 128),
-                                                                     (64, 256, 12, 32)))
-
-
 def test_small_product_rule():
     """Which kernel takes a product of up to 64 rows is a rule of its shape (the kernels add in different
     orders, so it must not depend on a timing)."""
