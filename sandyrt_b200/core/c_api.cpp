@@ -303,6 +303,8 @@ Json call_global(const std::string& m, const Json& a) {
     }
     if (m == "singles_apart")
         return Json(ops::singles_apart((int)a.at("singles").as_int(), (int)a.at("n_heads").as_int(), (int)a.at("seen_keys").as_int()));
+    if (m == "prompt_f32_general")
+        return Json(ops::prompt_f32_general((int)a.at("head_dim").as_int(), (int)a.at("max_q_len").as_int(), (int)a.at("table_keys").as_int()));
     if (m == "decode_splits")
         return Json(ops::decode_splits((int)a.at("n_tokens").as_int(), (int)a.at("n_heads").as_int(), (int)a.at("max_kv").as_int(), (int)geti(a, "sms", 0)));
     if (m == "small_gemm_kernel")                     // {"M", "N", "K"} -> "split_k" | "streaming": the rule for products of up to 64 rows

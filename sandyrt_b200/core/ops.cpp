@@ -498,6 +498,15 @@ int decode_splits(int n_tokens, int n_heads, int max_kv, int sms) {
 // beside 4, 8, 16 and 32 portions of 32 tokens: 16.5 / 15.1, 17.7 / 15.3, 21.6 / 17.0, 27.2 / 23.8).
 bool singles_apart(int singles, int n_heads, int seen_keys) { return singles * n_heads >= (seen_keys > 128 ? 256 : 384); }
 
+// The general kernel starts at once and then takes 0.2 to 0.4 us a key; the prompt kernel brings a tile of 64 keys whatever it needs
+// of it.  Alone, us, general / prompt kernel, one prompt of 16, 32, 48 and 64 tokens: 4 heads of 16 6.6 / 13.0, 9.8 / 13.5, 13.8 / 14.2,
+// 17.0 / 14.9; of 32 7.1 / 13.0, 10.6 / 13.6, 15.2 / 14.3, 18.5 / 14.9; 12 heads of 64 9.3 / 13.6, 14.0 / 14.3, 20.7 / 14.8, 25.8 /
+// 15.8; and 16 tokens behind 100 and 500: 4 heads of 16 28.4 / 19.9, 118 / 60, 12 heads of 64 43.7 / 21.4, 182 / 68.  What decides is
+// the keys a request has, and a recorded step serves every division of its tokens, so only the longest portion and the table's
+// width are known here.  Portions above 48 tokens have more keys than that.  Below, on tables of up to 128 keys, small heads stand to
+// lose 9 us behind a context and 6 without, heads of 64 22 and 4: those take the prompt kernel.
+bool prompt_f32_general(int head_dim, int max_q_len, int table_keys) { return head_dim <= 32 && max_q_len <= 48 && table_keys <= 128; }
+
 namespace {
 constexpr int kClusterMaxSplits = 8;
 // From this many (token, head) pairs on, a decode step's attention streams pages through shared
@@ -576,11 +585,8 @@ void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const K
               "prefill_attention" + shape);
         return;
     }
-    // float32 prompts.  The general kernel keeps heads above 128, and small heads on tables of few keys: it starts at once and
-    // then takes 0.2 to 0.4 us a key, where the prompt kernel brings a tile of 64 keys whatever it needs of it.  Alone, us, general /
-    // prompt kernel: 4 heads of 16, prompts of 8 tokens 4.6 / 10.8, of 16 6.7 / 13.0, of 33 11.1 / 14.0, of 64 16.8 / 14.8, of 100
-    // 26.3 / 19.7; 12 heads of 64: 7.0 / 11.5, 9.5 / 13.7, 18.0 / 14.7, 25.5 / 15.6, 44.7 / 21.3.
-    if (s.max_q_len > 1 && q.dtype == DType::F32 && d <= 128 && (d > 32 || s.max_blocks * c.page_size > 128)) {
+    // float32 prompts (the general kernel also keeps heads above 128)
+    if (s.max_q_len > 1 && q.dtype == DType::F32 && d <= 128 && !prompt_f32_general(d, s.max_q_len, s.max_blocks * c.page_size)) {
         static auto fn = SANDY_KERNEL(attention_prefill_f32, sandy_prefill_attention_f32_rules);
         OpTimer timer(l, "attention, prompt (float32)", attn_bytes, attn_flops);
         const int code = fn((const float*)q.data, (int)q.ld, (const float*)c.k, (const float*)c.v, c.page_stride, s.block_table,

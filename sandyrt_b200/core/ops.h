@@ -169,6 +169,8 @@ int decode_splits(int n_tokens, int n_heads, int max_kv, int sms = 0);
 // Whether a mixed step's single tokens take a launch of the decode kernel of their own (bfloat16, heads of 64); seen_keys: the most
 // keys a token may see.
 bool singles_apart(int singles, int n_heads, int seen_keys);
+// Whether float32 prompt portions stay with the general attention kernel; table_keys: the keys the block table has room for.
+bool prompt_f32_general(int head_dim, int max_q_len, int table_keys);
 
 // ---- RMS norms and what goes with them (rmsnorm.cu, elementwise.cu) ------------------------------------------
 struct StepSeqs {                                                  // the step's requests, as kernels with a state per request need them

@@ -270,6 +270,13 @@ def singles_apart(singles: int, n_heads: int, seen_keys: int) -> bool:
     return core.call("global", None, "singles_apart", singles=singles, n_heads=n_heads, seen_keys=seen_keys)
 
 
+def prompt_f32_general(head_dim: int, max_q_len: int, table_keys: int) -> bool:
+    """Whether float32 prompt portions stay with the general attention kernel; table_keys: the keys the block table has room for."""
+    from .. import core
+
+    return core.call("global", None, "prompt_f32_general", head_dim=head_dim, max_q_len=max_q_len, table_keys=table_keys)
+
+
 def decode_splits(n_tokens: int, n_heads: int, max_kv: int, sms: Optional[int] = None) -> int:
     """How many blocks share the keys of one (token, head) pair in a decode step (the host library's
     rule, core/ops.cpp): about four blocks an SM in all, more where a block would walk more than some 256

@@ -187,6 +187,14 @@ def test_single_tokens_take_a_launch_of_their_own_where_it_was_measured_faster()
     assert not at(16, 16, 128) and at(32, 16, 128) and at(32, 12, 128) and at(16, 25, 128)
 
 
+def test_float32_portions_take_the_attention_kernel_that_was_measured_faster():
+    """The rule's answers where both kernels were timed alone, as far as a recorded step's counts tell."""
+    from sandyrt_b200.csrc.ops import prompt_f32_general
+
+    assert all(prompt_f32_general(d, n, 128) for d, n in ((16, 8), (16, 33), (32, 32), (16, 48)))
+    assert not any(prompt_f32_general(d, n, k) for d, n, k in ((16, 64, 128), (16, 100, 128), (32, 64, 128), (16, 16, 256), (64, 48, 128), (128, 100, 128)))
+
+
 def test_small_product_rule():
     """Which kernel takes a product of up to 64 rows is a rule of its shape (the kernels add in different
     orders, so it must not depend on a timing)."""

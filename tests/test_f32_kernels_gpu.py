@@ -177,6 +177,38 @@ def test_a_token_that_is_not_finite_reaches_every_query_that_sees_it(D, window, 
         assert torch.equal(torch.isnan(got), torch.isnan(general))
 
 
+@pytest.mark.parametrize("name", ["A", "C"])
+def test_float32_portions_on_both_sides_of_the_rule(model_dirs, plain_models, name):
+    """Heads of 16 and 48: prompts of 32 to 100 tokens (48 is the last that the general kernel keeps) and portions behind a context,
+    alone and together; the same step again is a replay."""
+    from sandyrt_b200.engine.step import Engine, StepEntry
+    from sandyrt_b200.models.model import load_model
+    from test_replay_gpu import _close
+
+    plain = plain_models(name, "f32")
+    eng = Engine(load_model(model_dirs[name], device="cuda:0", dtype=torch.float32), max_tokens=512, max_requests=8)
+    eng.cache.device_caches.poison()
+    ids = np.random.default_rng(4).integers(0, 512, size=100).tolist()
+
+    def step(parts):
+        out = eng.step([StepEntry(r, ids[a:b], list(range(b - a))) for r, a, b in parts]).cpu().numpy()
+        at = 0
+        for r, a, b in parts:
+            _close(out[at:at + b - a], plain.logits(ids[:b])[a:], "float32", f"{name} {parts}")
+            at += b - a
+
+    for n in (32, 48, 49, 64, 100):
+        for _ in range(3):
+            step([("r", 0, n)])
+            eng.release("r")
+    step([("a", 0, 31), ("b", 0, 5), ("c", 0, 17)])
+    for b in range(31, 63, 4):                          # portions of four tokens, from 35 keys to 63
+        step([("a", b, b + 4)])
+    for n in (5, 9, 13, 17, 21, 25, 29, 33):
+        step([("b", n, n + 4), ("c", 12 + n, 16 + n)])
+    assert eng.graph_replays >= 4
+
+
 # ---- one small matrix per group of rows or columns ---------------------------------------------------------------------
 @pytest.mark.parametrize("sizes,N,K", [([1, 0, 2, 1], 33, 132), ([3, 3, 3], 4, 4), ([64, 65, 0, 127, 1], 130, 100), ([200], 64, 64), ([5, 9], 1000, 768)])
 def test_expert_product_f32(sizes, N, K):
