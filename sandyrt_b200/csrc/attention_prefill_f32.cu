@@ -8,7 +8,7 @@
 // fmas.  Scores pair two entries of the head (queries and keys run along it), the output pairs two columns.  Keys and values
 // come by cp.async from the request's pages, values under the scores, the next keys under the output; for heads above 64 the
 // probabilities take the keys' place, so that two blocks fit an SM.
-// Alone, us, the general kernel -> this one: two prompts of 1,024 tokens, 12 heads of 64: 1,618 -> 154 (21 TFLOP/s of the pairs a
+// Alone, us, the general kernel -> this one: two prompts of 1,024 tokens, 12 heads of 64: 1,607 -> 132 (24 TFLOP/s of the pairs a
 // causal mask leaves); four of 100 to 412 tokens, 12 heads of 128 on one key/value head: 470 -> 99; 32 single tokens behind
 // 100 to 700 beside a portion of 480, 16 heads of 64: 573 -> 119.  What is left is instructions beside the fmas (softmax, loads
 // from shared memory) and, in short steps, a block's serial start.

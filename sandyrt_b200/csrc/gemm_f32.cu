@@ -9,8 +9,8 @@
 // fixed by the launch's shape (M, N, K), never by the other rows' values.
 //
 // Measured alone, weights from HBM, against the general kernel (gemm_simt.cu), us: 8 rows, 2,304 x 768 94 -> 4.1, 768 x 3,072
-// 361 -> 5.2, 50,257 x 768 242 -> 46 (3.4 TB/s); 2,048 rows, 2,304 x 768 239 -> 164, 768 x 768 98 -> 68, 3,072 x 768 327 ->
-// 227, 768 x 3,072 379 -> 240 (44 TFLOP/s of the 74 the fma units could do: with three 64-bit operands a packed fma takes
+// 361 -> 5.2, 50,257 x 768 242 -> 46 (3.4 TB/s); 2,048 rows, 2,304 x 768 239 -> 164, 768 x 768 98 -> 68, 3,072 x 768 328 ->
+// 246, 768 x 3,072 379 -> 240 (44 TFLOP/s of the 74 the fma units could do: with three 64-bit operands a packed fma takes
 // about three cycles of the register file, not two).
 //
 // Two kernels:

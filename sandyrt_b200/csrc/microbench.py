@@ -4,6 +4,10 @@
     python -m sandyrt_b200.csrc.microbench gemm [--rows 2048] [--width 768] [--inner 3072] [--layers 48] [--k-sweep]
     python -m sandyrt_b200.csrc.microbench prefill-attention [--heads 12] [--page-size 16] [--shape 2x1024+0 ...]
     python -m sandyrt_b200.csrc.microbench grouped [--tokens 2048 8] [--experts 16] [--top 2] [--width 1536] [--inner 2048]
+    python -m sandyrt_b200.csrc.microbench gemm-f32 [--rows 1 8 24 2048] [--shape 2304x768 ...]
+    python -m sandyrt_b200.csrc.microbench attention-f32 [--heads 12] [--head-dim 64] [--shape 2x1024+0 ...]
+    python -m sandyrt_b200.csrc.microbench mixed-attention [--heads 16] [--context 400] [--portions 1x480] [--singles 8 16 32]
+    python -m sandyrt_b200.csrc.microbench recurrences [--lengths 1024 1024] [--heads 12]
 
 decode-attention: the register kernel and the bulk-copy kernel of single-token attention on
 several (tokens, context) shapes.  Each timing replays a graph of one launch per distinct cache
@@ -220,6 +224,113 @@ def grouped(a) -> int:
     return 0
 
 
+def gemm_f32(a) -> int:
+    """The float32 product beside the general kernel, on distinct weights that together exceed L2."""
+    dev = torch.device("cuda:0")
+    for M in a.rows:
+        for shape in a.shape:
+            N, K = (int(v) for v in shape.split("x"))
+            x, out = torch.randn(M, K, device=dev), torch.empty(M, N, device=dev)
+            ws = [torch.randn(N, K, device=dev) for _ in range(max(1, min(24, 300_000_000 // (4 * N * K))))]
+            us = [_time_graph(lambda l: ops.gemm_f32(x, ws[l], None, out), len(ws)),
+                  _time_graph(lambda l: ops.gemm_simt(x, ws[l], None, out, w_out_in=True), len(ws))]
+            print(f"{M:5d} rows {N:6d} x {K:5d}: {us[0]:8.1f} us  {4e-3 * N * K / us[0]:6.0f} GB/s  {2e-6 * M * N * K / us[0]:5.1f} TFLOP/s"
+                  f"   general kernel {us[1]:8.1f} us", flush=True)
+    return 0
+
+
+def _cache(dev, H, D, ps, seqs, dtype):
+    """Queries and cache of requests (tokens before, new tokens); the table's width as the engine has it, in steps of 8 pages."""
+    g = torch.Generator(device=dev).manual_seed(0)
+    blocks = [-(-(b + n) // ps) for b, n in seqs]
+    table = torch.full((len(seqs), -(-max(blocks) // 8) * 8), -1, dtype=torch.int32)
+    at = 0
+    for i, n in enumerate(blocks):
+        table[i, :n] = torch.arange(at, at + n)
+        at += n
+    kc, vc = (torch.randn(at, H, ps, D, generator=g, device=dev).to(dtype) for _ in range(2))
+    T = sum(n for _, n in seqs)
+    q = torch.randn(T, H * D, generator=g, device=dev).to(dtype)
+    start = torch.tensor([0] + [n for _, n in seqs]).cumsum(0).to(torch.int32).to(dev)
+    before = torch.tensor([b for b, _ in seqs], dtype=torch.int32, device=dev)
+    seq = torch.repeat_interleave(torch.arange(len(seqs)), torch.tensor([n for _, n in seqs])).to(torch.int32).to(dev)
+    pos = torch.cat([torch.arange(b, b + n) for b, n in seqs]).to(torch.int32).to(dev)
+    return q, kc, vc, table.to(dev), start, before, seq, pos
+
+
+def attention_f32(a) -> int:
+    """Prompt portions in float32: the general kernel and the prompt kernel."""
+    for shape in a.shape:
+        reqs, rest = shape.split("x")
+        new, cached = (int(v) for v in rest.split("+"))
+        q, kc, vc, table, start, before, seq, pos = _cache("cuda:0", a.heads, a.head_dim, a.page_size, [(cached, new)] * int(reqs), torch.float32)
+        out, kw = torch.empty_like(q), dict(n_heads=a.heads, scale=a.head_dim ** -0.5)
+        general = _time_graph(lambda l: ops.paged_attention(q, kc, vc, table, seq, pos, out, **kw), 10)
+        tiles = _time_graph(lambda l: ops.prefill_attention_f32(q, kc, vc, table, start, before, out, max_q_len=new, **kw), 10)
+        print(f"{a.heads} heads of {a.head_dim}, {shape:>10}: general {general:8.1f} us  prompt kernel {tiles:8.1f} us", flush=True)
+    return 0
+
+
+def mixed_attention(a) -> int:
+    """Single tokens beside portions, bfloat16, heads of 64: one launch over everything and two."""
+    reqs, new = (int(v) for v in a.portions.split("x"))
+    for n in a.singles:
+        spread = a.context // 2
+        seqs = [(a.context - spread // 2 + spread * i // max(n - 1, 1), 1) for i in range(n)] + [(0, new)] * reqs
+        q, kc, vc, table, start, before, _, _ = _cache("cuda:0", a.heads, 64, 16, seqs, torch.bfloat16)
+        out, keys = torch.empty_like(q), table.shape[1] * 16
+        kw = dict(n_heads=a.heads, max_q_len=new, scale=0.125)
+        one = _time_graph(lambda l: ops.prefill_attention(q, kc, vc, table, start, before, out, **kw), 10)
+        splits = min(8, ops.decode_splits(n, a.heads, keys))
+        two = _time_graph(lambda l: ops.mixed_attention(q, kc, vc, table, start, before, out, num_splits=splits, **kw), 10)
+        print(f"{a.heads} heads, {n:3d} tokens behind about {a.context} beside {a.portions}: one launch {one:6.1f} us  two {two:6.1f} us  "
+              f"(taken: {'two' if ops.singles_apart(n, a.heads, keys) else 'one'})", flush=True)
+    return 0
+
+
+def recurrences(a) -> int:
+    """Delta rule (heads of 64) and matrix memory (a quarter of the heads, 64 x 128) over prompts: chunks walked one by one and side by
+    side; and the delta rule's errors against 64 bits in the 2-norm (read-outs, state), from an empty state."""
+    dev = torch.device("cuda:0")
+    H, T, d = a.heads, sum(a.lengths), 64
+    g = torch.Generator(device=dev).manual_seed(0)
+    rand = lambda *shape: torch.randn(*shape, generator=g, device=dev)
+    start = torch.tensor([0] + a.lengths).cumsum(0).to(torch.int32).to(dev)
+    slots = torch.arange(len(a.lengths), dtype=torch.int32, device=dev)
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    q, k, v = unit(rand(T, H, d)) / 8, unit(torch.nn.functional.silu(rand(T, H, d))), rand(T, H, d)
+    bg = torch.cat([torch.rand(T, H, generator=g, device=dev), -0.1 * torch.rand(T, H, generator=g, device=dev)], 1)
+    qkv = torch.cat([x.reshape(T, -1) for x in (q, k, v)], 1)
+    want, S = torch.empty(T, H, d, dtype=torch.float64, device=dev), None
+    states = []
+    for t in range(T):
+        if t in start.tolist():
+            S = torch.zeros(H, d, d, dtype=torch.float64, device=dev)
+        S = S * torch.exp(bg[t, H:].double()).view(H, 1, 1)
+        u = bg[t, :H].double().view(H, 1) * (v[t].double() - torch.einsum("hed,hd->he", S, k[t].double()))
+        S = S + u.unsqueeze(2) * k[t].double().unsqueeze(1)
+        want[t] = torch.einsum("hed,hd->he", S, q[t].double())
+        if t + 1 in start.tolist():
+            states.append(S)
+    off = lambda x, y: ((x.double() - y).norm() / y.norm()).item()
+    kw = dict(long_from=8, max_q_len=max(a.lengths))
+    for form in ("walk", "chunks"):
+        state, out = torch.zeros(len(a.lengths), H * d * d, device=dev), torch.empty(T, H * d, device=dev)
+        go = lambda l: ops.delta_scan(qkv, bg, state, start, slots, out, n_heads=H, n_qk_heads=H, qk_dim=d, v_dim=d, form=form, **kw)
+        go(0)
+        errors = off(out.view(T, H, d), want), off(state.view(-1, H, d, d), torch.stack(states))
+        print(f"delta rule, {H} heads, {a.lengths}, {form:6s}: {_time_graph(go, 10):8.1f} us  errors {errors[0]:.1e} {errors[1]:.1e}", flush=True)
+    H = max(1, H // 4)
+    proj, gates = rand(T, H * (2 * d + 128)).to(torch.bfloat16), rand(T, 2 * H)
+    bias = torch.cat([torch.zeros(H), torch.full((H,), 4.0)]).to(dev)
+    for form in ("walk", "chunks"):
+        state, out = torch.zeros(len(a.lengths), H * (128 * d + 8 * d + 8), device=dev), torch.empty(T, H * 128, device=dev)
+        go = lambda l: ops.mlstm_scan(proj, 0, H * d, 2 * H * d, gates, bias, state, start, slots, out, cap=12.0, q_scale=0.125, n_heads=H,
+                                      qk_dim=d, v_dim=128, form=form, **kw)
+        print(f"matrix memory, {H} heads, {a.lengths}, {form:6s}: {_time_graph(go, 10):8.1f} us", flush=True)
+    return 0
+
+
 def main(argv=None) -> int:
     ap = argparse.ArgumentParser(prog="sandyrt_b200.csrc.microbench")
     sub = ap.add_subparsers(dest="cmd", required=True)
@@ -253,6 +364,26 @@ def main(argv=None) -> int:
     gr.add_argument("--heads", type=int, default=24)
     gr.add_argument("--layers", type=int, default=4, help="distinct sets of weights (together larger than L2)")
     gr.set_defaults(fn=grouped)
+    gf = sub.add_parser("gemm-f32")
+    gf.add_argument("--rows", type=int, nargs="+", default=[1, 8, 24, 2048])
+    gf.add_argument("--shape", nargs="+", default=["2304x768", "768x768", "3072x768", "768x3072", "50257x768"], help="outputs x inputs")
+    gf.set_defaults(fn=gemm_f32)
+    af = sub.add_parser("attention-f32")
+    af.add_argument("--heads", type=int, default=12)
+    af.add_argument("--head-dim", type=int, default=64)
+    af.add_argument("--page-size", type=int, default=16)
+    af.add_argument("--shape", nargs="+", default=["2x1024+0", "1x16+0", "1x32+0", "1x48+0", "1x64+0", "8x16+0", "1x16+100"], help="REQUESTSxNEW+CACHED")
+    af.set_defaults(fn=attention_f32)
+    mx = sub.add_parser("mixed-attention")
+    mx.add_argument("--heads", type=int, default=16)
+    mx.add_argument("--context", type=int, default=400)
+    mx.add_argument("--portions", default="1x480", help="PORTIONSxTOKENS")
+    mx.add_argument("--singles", type=int, nargs="+", default=[4, 8, 16, 32])
+    mx.set_defaults(fn=mixed_attention)
+    rc = sub.add_parser("recurrences")
+    rc.add_argument("--lengths", type=int, nargs="+", default=[1024, 1024])
+    rc.add_argument("--heads", type=int, default=12)
+    rc.set_defaults(fn=recurrences)
     a = ap.parse_args(argv)
     return a.fn(a)
 
