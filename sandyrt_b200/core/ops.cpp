@@ -168,6 +168,15 @@ void layernorm(const Launch& l, const Tensor& x, const Tensor& gamma, const Tens
           "layernorm(width=" + std::to_string(width) + ")");
 }
 
+// Float32 products that the tensor cores take (gemm_f32_tc.cu; the operands in three pieces, sums off by less than those of the
+// fma kernels): above the rows up to which weights are streamed, except where the fma kernel's tiles of 64 x 64 in eight parts of k
+// are one round of short blocks.  us, fma / tensor cores: 33 rows 768 x 768 6.1 / 6.9, 2,304 x 768 11.5 / 9.0, 768 x 3,072 15.8 /
+// 10.6, 256 x 256 4.8 / 4.8, 1,000 x 512 6.8 / 6.2; 64 rows 768 x 768 6.4 / 7.0; 100 rows 9.4 / 7.3.
+static bool f32_on_tensor_cores(int64_t M, int64_t N, int64_t K) {
+    if (M <= 24) return false;
+    return M > 64 || N > 896 || K < 512 || K > 1024;
+}
+
 void gemm_simt(const Launch& l, const Tensor& a, const Tensor& w, const Tensor* bias, Tensor& out, bool w_out_in, Act act,
                const Tensor* residual) {
     const int64_t M = a.rows, K = a.cols, N = out.cols;
@@ -178,11 +187,19 @@ void gemm_simt(const Launch& l, const Tensor& a, const Tensor& w, const Tensor* 
     if (residual && (residual->dtype != DType::F32 || residual->rows != M || residual->cols != N))
         throw KernelError("gemm: residual must be float32 [M, N]");
     if (bias && (bias->dtype != w.dtype || bias->numel() != N)) throw KernelError("gemm: bias must have the weight's dtype and N elements");
-    OpTimer timer(l, "product, FFMA (float32)", tensor_bytes(&a) + tensor_bytes(&w) + tensor_bytes(&out) + 2 * tensor_bytes(residual),
+    OpTimer timer(l, "product, float32", tensor_bytes(&a) + tensor_bytes(&w) + tensor_bytes(&out) + 2 * tensor_bytes(residual),
                   2.0 * M * N * K);
     // weights whose rows run along k from 16-byte boundaries: the kernels that load four k at a time
     if (w_out_in && a.dtype == DType::F32 && w.dtype == DType::F32 && out.dtype == DType::F32 && K % 4 == 0 && a.ld % 4 == 0 &&
         w.ld % 4 == 0 && !((uintptr_t)a.data & 15) && !((uintptr_t)w.data & 15)) {
+        if (f32_on_tensor_cores(M, N, K)) {
+            static auto split = SANDY_KERNEL(gemm_f32_tc, sandy_gemm_f32_tc);
+            check(split((const float*)a.data, (const float*)w.data, bias ? (const float*)bias->data : nullptr,
+                        residual ? (const float*)residual->data : nullptr, (float*)out.data, (int)M, (int)N, (int)K, (int)a.ld, (int)w.ld,
+                        residual ? (int)residual->ld : 0, (int)out.ld, (int)act, 0, 0, l.kernel_status, l.stream),
+                  "gemm_f32_tc(M=" + std::to_string(M) + ",N=" + std::to_string(N) + ",K=" + std::to_string(K) + ")");
+            return;
+        }
         static auto fast = SANDY_KERNEL(gemm_f32, sandy_gemm_f32);
         check(fast((const float*)a.data, (const float*)w.data, bias ? (const float*)bias->data : nullptr,
                    residual ? (const float*)residual->data : nullptr, (float*)out.data, (int)M, (int)N, (int)K, (int)a.ld, (int)w.ld,

@@ -157,25 +157,34 @@ def gemm_simt(a, w, bias, out, *, w_out_in: bool, act=None, residual=None) -> No
     _check(code, f"gemm_simt(M={M},N={N},K={K},{a.dtype}->{out.dtype})")
 
 
-def gemm_f32(a, w, bias, out, *, act=None, residual=None, form: int = 0, splits: int = 1) -> None:
-    """out = act(a @ w.T + bias) + residual, all float32, w [N, K]: K and the row pitches of a and w multiples of 4, both on
-    16-byte boundaries.  form 0 lets the kernel choose; 1 streams the weights past a few rows; 2, 3 and 4 are tiles of
-    128 x 128, 64 x 128 and 64 x 64 whose k is split over `splits` (1, 2, 4, 8) blocks."""
+def _f32_product(name, a, w, bias, out, residual, act, *last) -> None:
     _cuda(a, w, bias, out, residual)
     M, K = a.shape
     N = out.shape[1]
     if tuple(w.shape) != (N, K) or out.shape[0] != M:
-        raise KernelError(f"gemm_f32: shapes disagree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+        raise KernelError(f"{name}: shapes disagree: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
     if any(t is not None and (t.dtype != torch.float32 or t.stride(-1) != 1) for t in (a, w, bias, out, residual)):
-        raise KernelError("gemm_f32: float32 tensors with an innermost stride of 1 expected")
+        raise KernelError(name + ": float32 tensors with an innermost stride of 1 expected")
     if (residual is not None and tuple(residual.shape) != (M, N)) or (bias is not None and bias.numel() != N):
-        raise KernelError("gemm_f32: residual must be [M, N], bias [N]")
-    lib = load_library("gemm_f32")
-    code = lib.sandy_gemm_f32(_p(a), _p(w), _p(bias), _p(residual), _p(out), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
-                              ctypes.c_int(a.stride(0)), ctypes.c_int(w.stride(0)),
-                              ctypes.c_int(0 if residual is None else residual.stride(0)), ctypes.c_int(out.stride(0)),
-                              ctypes.c_int(ACT_CODES[act]), ctypes.c_int(form), ctypes.c_int(splits), _stream())
-    _check(code, f"gemm_f32(M={M},N={N},K={K},form={form},splits={splits})")
+        raise KernelError(name + ": residual must be [M, N], bias [N]")
+    entry = getattr(load_library(name), "sandy_" + name)
+    code = entry(_p(a), _p(w), _p(bias), _p(residual), _p(out), ctypes.c_int(M), ctypes.c_int(N), ctypes.c_int(K),
+                 ctypes.c_int(a.stride(0)), ctypes.c_int(w.stride(0)), ctypes.c_int(0 if residual is None else residual.stride(0)),
+                 ctypes.c_int(out.stride(0)), ctypes.c_int(ACT_CODES[act]), *last, _stream())
+    _check(code, f"{name}(M={M},N={N},K={K})")
+
+
+def gemm_f32(a, w, bias, out, *, act=None, residual=None, form: int = 0, splits: int = 1) -> None:
+    """out = act(a @ w.T + bias) + residual, all float32, w [N, K]: K and the row pitches of a and w multiples of 4, both on
+    16-byte boundaries.  form 0 lets the kernel choose; 1 streams the weights past a few rows; 2, 3 and 4 are tiles of
+    128 x 128, 64 x 128 and 64 x 64 whose k is split over `splits` (1, 2, 4, 8) blocks."""
+    _f32_product("gemm_f32", a, w, bias, out, residual, act, ctypes.c_int(form), ctypes.c_int(splits))
+
+
+def gemm_f32_tc(a, w, bias, out, *, act=None, residual=None, tile: int = 0, parts: int = 0) -> None:
+    """The same product on the tensor cores, the operands in three bfloat16 pieces each.  tile: 64, 96 or 128 columns; parts: 1,
+    2, 4 or 8 blocks that share its k; 0, 0 lets the kernel choose."""
+    _f32_product("gemm_f32_tc", a, w, bias, out, residual, act, ctypes.c_int(tile), ctypes.c_int(parts), _p(kernel_status(a.device)))
 
 
 def _cache_args(k_cache, v_cache):

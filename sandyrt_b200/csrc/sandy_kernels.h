@@ -38,6 +38,10 @@ int sandy_gemm_simt(const void* a, const void* w, const void* bias, const float*
 int sandy_gemm_f32(const float* a, const float* w, const float* bias, const float* residual, float* out, int M, int N, int K,
                    int lda, int ldw, int ldr, int ldc, int act, int form, int splits, cudaStream_t stream);
 
+/* gemm_f32_tc.cu */
+int sandy_gemm_f32_tc(const float* a, const float* w, const float* bias, const float* residual, float* out, int M, int N, int K,
+                      int lda, int ldw, int ldr, int ldc, int act, int tile, int parts, int* status, cudaStream_t stream);
+
 /* gemm_tc.cu, gemm_tc2.cu */
 int sandy_gemm_tc(const void* a, const void* w, const void* bias, const float* residual, void* out, int M, int N, int K,
                   int lda, int ldw, int ldr, int ldc, int act, int out_dtype, int tile_n, void* k_cache, void* v_cache,

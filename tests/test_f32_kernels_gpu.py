@@ -65,6 +65,39 @@ def test_gemm_f32_refuses_what_it_cannot_load():
         ops.gemm_f32(torch.zeros(25, device=DEV)[1:].view(3, 8)[:, :4], w[:, :4].contiguous(), None, out)   # not on 16 bytes
 
 
+@pytest.mark.parametrize("tile,parts", [(0, 0), (64, 1), (64, 8), (96, 1), (96, 4), (128, 1), (128, 2), (128, 8)])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (33, 50, 12), (127, 97, 516), (129, 130, 576), (260, 257, 1028)])
+@pytest.mark.parametrize("size", [1.0, 2.0 ** -110, 2.0 ** 100])
+def test_gemm_f32_on_tensor_cores(M, N, K, tile, parts, size):
+    """Tiles, parts and chunks of k with remainders; pitches wider than the rows; the residual is the output itself; activations
+    whose pieces would leave the range of a bfloat16, and ones too large to be split; an infinite activation."""
+    from sandyrt_b200.csrc import ops
+
+    if parts > (K + 63) // 64:
+        pytest.skip("fewer chunks of k than parts")
+    g = torch.Generator().manual_seed(M * 1000 + N + K)
+    a = (torch.randn(M, K + 4, generator=g) * size).to(DEV)[:, :K]
+    w = (torch.randn(N, K + 8, generator=g) / size).to(DEV)[:, :K]
+    bias, x0 = torch.randn(N, generator=g).to(DEV), torch.randn(M, N + 3, generator=g).to(DEV)
+    want = a.double() @ w.double().t() + bias.double()
+    # of a product 2^-26 is left out with the three smallest products of pieces; sixteen products at a time are added with at
+    # most 2^-22 of their sizes lost to rounding towards zero: less than K * 2^-24 from K = 4 on; 4 for the write-back
+    bound = (K + 4) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t() + bias.double().abs() + x0[:, :N].double().abs())
+    wide = x0.clone()
+    x = wide[:, :N]
+    ops.gemm_f32_tc(a, w, bias, x, residual=x, tile=tile, parts=parts)
+    assert bool(((x.double() - want - x0[:, :N].double()).abs() <= bound).all())
+    assert torch.equal(wide[:, N:], x0[:, N:])
+    finite, out = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    ops.gemm_f32_tc(a, w, None, finite, tile=tile, parts=parts)
+    b = a.clone()
+    b[M - 1, K - 1] = float("inf")
+    ops.gemm_f32_tc(b, w, None, out, tile=tile, parts=parts)
+    assert torch.equal(out[M - 1], torch.sign(w[:, K - 1]) * float("inf"))
+    assert torch.equal(out[:M - 1], finite[:M - 1])
+    assert int(ops.kernel_status(a.device).item()) == 0
+
+
 # ---- attention of prompt portions ---------------------------------------------------------------------------------
 def _both(case, H, kw):
     """The prompt kernel's output and the general kernel's, which reads one (token, head) pair at a time."""
