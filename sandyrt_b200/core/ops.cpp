@@ -919,7 +919,14 @@ void expert_product(const Launch& l, const Routing& r, const Tensor& a, bool gat
     // bytes: every expert's matrix at most once, and no more matrices than slots
     const double matrices = std::min<double>(r.n_experts, (double)slots);
     static const int tc_mode = env_int("SANDYRT_EXPERT_TC", -1);      // 0 / 1 force one kernel, for comparisons
-    if (tc_mode != 0 && a.dtype == DType::BF16 && K % 8 == 0 && w.ld % 8 == 0 && !((uintptr_t)w.data & 15) && (!gather || sorted)) {
+    // float32 (gemm_f32_tc.cu): where an expert has more rows on average than the weights are streamed past, and a matrix is large
+    // enough for a block's start not to count.  16 experts, two a token, us, fma tiles / tensor cores with the gathering of the rows:
+    // 1,024 x 768, 40 tokens 59 / 24, 1,024 tokens 105 / 50 (24 tokens, streamed: 18 / 24); 256 x 192, 40 tokens 9.4 / 11.3, 1,024
+    // tokens 15 / 19; 64 experts, four a token, 512 x 512, 100 tokens 59 / 41.
+    const bool f32_tc = a.dtype == DType::F32 && out.dtype == DType::F32 && K % 4 == 0 && w.ld % 4 == 0 &&
+                        (slots + r.n_experts) / r.n_experts > 4 && N * K >= 512 * 512;
+    const bool bf16_tc = a.dtype == DType::BF16 && K % 8 == 0 && w.ld % 8 == 0;
+    if (tc_mode != 0 && (bf16_tc || f32_tc) && !((uintptr_t)w.data & 15) && (!gather || sorted)) {
         const Tensor* rows = &a;
         if (gather) {
             if (sorted->dtype != a.dtype || sorted->rows != slots || sorted->cols != K) throw KernelError("expert_product: the scratch for sorted rows must be [slots, K] of a's type");
@@ -930,13 +937,21 @@ void expert_product(const Launch& l, const Routing& r, const Tensor& a, bool gat
                   "moe_gather");
             rows = sorted;
         }
-        if (rows->ld % 8 == 0 && !((uintptr_t)rows->data & 15)) {
-            static auto tc = SANDY_KERNEL(grouped_gemm_tc, sandy_expert_product_tc);
+        if ((size_t)rows->ld * rows->elem_size() % 16 == 0 && !((uintptr_t)rows->data & 15)) {
             OpTimer timer(l, "product per expert (tcgen05)", matrices * N * K * w.elem_size() + (double)slots * (K * a.elem_size() + N * out.elem_size()),
                           2.0 * slots * N * K);
+            const std::string what = "(E=" + std::to_string(r.n_experts) + ",N=" + std::to_string(N) + ",K=" + std::to_string(K) + ")";
+            if (f32_tc) {
+                static auto split = SANDY_KERNEL(gemm_f32_tc, sandy_expert_product_f32_tc);
+                check(split((const float*)rows->data, (int)rows->ld, (const float*)w.data, (int)w.ld, (float*)out.data, (int)out.ld, (int)slots,
+                            r.n_experts, (int)N, (int)K, r.group_start, (int)act, l.kernel_status, l.stream),
+                      "expert_product_f32_tc" + what);
+                return;
+            }
+            static auto tc = SANDY_KERNEL(grouped_gemm_tc, sandy_expert_product_tc);
             check(tc(rows->data, (int)rows->ld, w.data, (int)w.ld, out.data, (int)out.ld, (int)slots, r.n_experts, (int)N, (int)K, r.group_start,
                      (int)act, code_of(out.dtype), l.kernel_status, l.stream),
-                  "expert_product_tc(E=" + std::to_string(r.n_experts) + ",N=" + std::to_string(N) + ",K=" + std::to_string(K) + ")");
+                  "expert_product_tc" + what);
             return;
         }
     }

@@ -3,6 +3,9 @@
 //
 //   out[m, n] = act( sum_k a[m, k] * w[n, k] + bias[n] ) + residual[m, n]
 //
+// The same with one matrix per expert: rows of a and out in the routing's sorted order (as in grouped_gemm_tc.cu), 16 experts, 1,024 x
+// 768, us, the fma tiles of grouped_gemm.cu -> this kernel: 80 slots 59 -> 23, 2,048 slots 105 -> 46.
+//
 // A block computes a tile of 128 x BN outputs, or a part of its k; the blocks of a tile's parts are a cluster.
 //   warp 17       brings the float operands by TMA, a chunk of 64 k a stage of two
 //   warps 0..15   split them: a's pieces go to tensor memory (a thread one row), w's to shared memory (128-byte swizzle); then add
@@ -37,7 +40,14 @@ struct Product {
     float* out;
     int M, N, K, lda, ldw, ldr, ldc, act;
     int wide;               // rows of out and residual start on 16-byte boundaries
+    const int* group_start; // a matrix per expert: where each expert's rows start, on the device
+    int groups;
 };
+
+// PLAIN: one matrix.  EXPERTS: expert g has the rows g * N .. of w and the rows group_start[g] .. group_start[g + 1] - 1 of a and out;
+// the grid covers the worst case of tiles, and blocks behind the step's last tile leave at once.  (A matrix per head, k 64 to 128, as a
+// third kind was no faster than the fma tiles: a block's start is most of so short a sum.)
+enum Kind { PLAIN, EXPERTS };
 
 constexpr int WORKERS = 16, THREADS = (WORKERS + 2) * 32, MAX_PARTS = 8;
 
@@ -54,7 +64,7 @@ struct Layout {
     static_assert(SUMS <= BODY && A_COL + 2 * A_COLS <= 512, "the sums reuse the stages; 512 columns there are");
 };
 
-template <int BN>
+template <int BN, Kind KIND>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const Product p,
                    int* __restrict__ status) {
@@ -69,8 +79,24 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 2);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
+    const int n0 = blockIdx.x * BN;
     const int parts = gridDim.z, part = blockIdx.z;
+    int group = 0, m0 = blockIdx.y * BM, m_end = p.M;
+    if (KIND == EXPERTS) {
+        pdl_wait();             // the groups' borders come from a kernel before
+        int tile = blockIdx.y;
+        m0 = p.group_start[0];
+        for (; group < p.groups; group++) {
+            m_end = p.group_start[group + 1];
+            const int tiles = (m_end - m0 + BM - 1) / BM;
+            if (tile < tiles) break;
+            tile -= tiles;
+            m0 = m_end;
+        }
+        if (group == p.groups) return;          // every thread of a cluster's blocks alike
+        m0 += tile * BM;
+    }
+    const int w_row0 = group * p.N + n0;
     const int chunks_all = (p.K + CHUNK - 1) / CHUNK;
     const int first = (int)((long long)chunks_all * part / parts), chunks = (int)((long long)chunks_all * (part + 1) / parts) - first;
 
@@ -94,9 +120,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     pdl_launch_dependents();
 
     if (warp < WORKERS) {
-        const int quarter = warp & 3, group = warp >> 2;
+        const int quarter = warp & 3, quad = warp >> 2;
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-        // a: a thread takes sixteen k (those of its warp's group) of its row
+        // a: a thread takes sixteen k (those of its warp's quad) of its row
         // w: an item is eight rows and the 32 k of a half, a thread eight k; lanes 0..3 and 4..7 take the rows r and r ^ 5, so that
         // eight lanes meet no bank twice, neither where they read floats (even or odd pieces of 16 bytes) nor where they write pieces
         constexpr int ITEMS = BN / 4, ROUNDS = (ITEMS + WORKERS - 1) / WORKERS;
@@ -111,7 +137,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         uint32_t a_at[4];
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            a_at[j] = (group >> 1) * L::A_HALF + (quarter * 32 + lane) * 128 + ((((group & 1) * 4 + j) ^ (lane & 7)) << 4);
+            a_at[j] = (quad >> 1) * L::A_HALF + (quarter * 32 + lane) * 128 + ((((quad & 1) * 4 + j) ^ (lane & 7)) << 4);
         constexpr int COLS = BN / 4;
         float sum[COLS];
 #pragma unroll
@@ -143,7 +169,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             split_eight(x[2], x[3], high);
 #pragma unroll
             for (int j = 0; j < N_PIECES; j++)
-                tmem_st_32x8(tmem + lanes + L::A_COL + s * L::A_COLS + j * (CHUNK / 2) + group * 8, low[j], high[j]);
+                tmem_st_32x8(tmem + lanes + L::A_COL + s * L::A_COLS + j * (CHUNK / 2) + quad * 8, low[j], high[j]);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");        // my pieces, before the tensor core reads them
             tmem_wait_st();
             tc_fence_before();
@@ -159,7 +185,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             tc_fence_after();
             uint32_t r[COLS];
 #pragma unroll
-            for (int j = 0; j < COLS; j += 8) tmem_ld_32x8(tmem + lanes + s * BN + group * COLS + j, *reinterpret_cast<uint32_t (*)[8]>(r + j));
+            for (int j = 0; j < COLS; j += 8) tmem_ld_32x8(tmem + lanes + s * BN + quad * COLS + j, *reinterpret_cast<uint32_t (*)[8]>(r + j));
             tmem_wait_ld();
 #pragma unroll
             for (int j = 0; j < COLS; j++) sum[j] += __uint_as_float(r[j]);
@@ -176,7 +202,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         }
         if (ok) add(chunks - 1, (chunks - 1) & 1);
         // the last products are done, so nothing reads the stages any more (no copy is under way either: every chunk was waited for)
-        float* mine = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * L::PITCH + group * COLS;
+        float* mine = reinterpret_cast<float*>(smem) + (quarter * 32 + lane) * L::PITCH + quad * COLS;
         if (ok) {
 #pragma unroll
             for (int j = 0; j < COLS; j += 4)
@@ -202,7 +228,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             uint8_t* raw = smem + (c & 1) * L::RAW + 2 * L::A_HALF;
             mbar_expect_tx(&raw_full[c & 1], L::RAW);
             for (int half = 0; half < 2; half++)
-                tma_load_2d(raw + half * L::W_HALF, &map_w, (first + c) * CHUNK + 32 * half, n0, &raw_full[c & 1]);
+                tma_load_2d(raw + half * L::W_HALF, &map_w, (first + c) * CHUNK + 32 * half, w_row0, &raw_full[c & 1]);
         };
         auto load_a = [&](int c) {
             uint8_t* raw = smem + (c & 1) * L::RAW;
@@ -239,7 +265,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             const int at = base + tid;
             const int row = at / PER_ROW * parts + part, col = at % PER_ROW * 4;
             const int m = m0 + row, n = n0 + col;
-            const bool live = at < total && m < p.M && n < p.N;
+            const bool live = at < total && m < m_end && n < p.N;
             float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             if (live) {
                 float* src = sums + row * L::PITCH + col;
@@ -266,7 +292,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     const int who = __ffs(again) - 1;
                     again &= again - 1;
                     const int mm = __shfl_sync(0xffffffffu, m, who), nn = __shfl_sync(0xffffffffu, n, who) + e;
-                    const float plain = plain_sum(p.a + (size_t)mm * p.lda, p.w + (size_t)nn * p.ldw, p.K);
+                    const float plain = plain_sum(p.a + (size_t)mm * p.lda, p.w + (size_t)(w_row0 - n0 + nn) * p.ldw, p.K);
                     if (lane == who) v[e] = plain;
                 }
             }
@@ -292,15 +318,16 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (parts > 1) cg::this_cluster().sync();         // nobody leaves while a peer may still read its shared memory
 }
 
-template <int BN>
-int launch(const Product& p, int parts, int* status, cudaStream_t stream) {
+// row_tiles: the grid's tiles of 128 rows; w_rows: the rows of w.
+template <int BN, Kind KIND>
+int launch(const Product& p, int row_tiles, int parts, long long w_rows, int* status, cudaStream_t stream) {
     using L = Layout<BN>;
-    const cudaError_t set = cudaFuncSetAttribute(gemm_f32_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
+    const cudaError_t set = cudaFuncSetAttribute(gemm_f32_tc_kernel<BN, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
     if (set != cudaSuccess) return (int)set;
     CUtensorMap map_a, map_w;
-    if (!get_map(p.a, p.M, p.K, p.lda, BM, &map_a, 4) || !get_map(p.w, p.N, p.K, p.ldw, BN, &map_w, 4)) return SANDY_ERR_ARGUMENT;
+    if (!get_map(p.a, p.M, p.K, p.lda, BM, &map_a, 4) || !get_map(p.w, w_rows, p.K, p.ldw, BN, &map_w, 4)) return SANDY_ERR_ARGUMENT;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((p.N + BN - 1) / BN, (p.M + BM - 1) / BM, parts);
+    cfg.gridDim = dim3((p.N + BN - 1) / BN, row_tiles, parts);
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = L::SMEM;
     cfg.stream = stream;
@@ -320,8 +347,17 @@ int launch(const Product& p, int parts, int* status, cudaStream_t stream) {
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel<BN>, map_a, map_w, p, status);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f32_tc_kernel<BN, KIND>, map_a, map_w, p, status);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+template <Kind KIND>
+int launch_tile(int tile, const Product& p, int row_tiles, int parts, long long w_rows, int* status, cudaStream_t stream) {
+    if (row_tiles > 65535) return SANDY_ERR_UNSUPPORTED;
+    if (tile == 64) return launch<64, KIND>(p, row_tiles, parts, w_rows, status, stream);
+    if (tile == 96) return launch<96, KIND>(p, row_tiles, parts, w_rows, status, stream);
+    if (tile == 128) return launch<128, KIND>(p, row_tiles, parts, w_rows, status, stream);
+    return SANDY_ERR_ARGUMENT;
 }
 
 // SMs that clusters of `parts` blocks, one block an SM, can cover (groups of SMs that share a crossbar are not all multiples).
@@ -333,13 +369,13 @@ int coverable(int parts) {
 // Which tile, in how many parts of k.  A block takes the SM to itself.  Its time is a start and a write-back, and a time for each
 // chunk that grows with the tile's columns by less than they do (the splitting of a's 128 rows is the rest): fitted to 1,500
 // measured (shape, tile, parts) of 26 to 2,048 rows, of which the choice meets the best within 0.4 % on average.
-void choose(int M, int N, int K, int& tile, int& parts) {
+void choose(long long row_tiles, int N, int K, int& tile, int& parts) {
     struct Shape { int columns; float chunk_us, block_us; };
     const Shape shapes[3] = {{64, 0.92f, 4.8f}, {96, 1.05f, 6.0f}, {128, 1.21f, 6.9f}};
     const int chunks = (K + CHUNK - 1) / CHUNK;
     float best = 0.0f;
     for (const Shape& h : shapes) {
-        const long long tiles = (long long)((N + h.columns - 1) / h.columns) * ((M + BM - 1) / BM);
+        const long long tiles = (long long)((N + h.columns - 1) / h.columns) * row_tiles;
         for (int p = 1; p <= MAX_PARTS && p <= chunks; p *= 2) {
             const long long rounds = (tiles * p + coverable(p) - 1) / coverable(p);
             const float cost = (float)rounds * ((float)((chunks + p - 1) / p) * h.chunk_us + h.block_us);
@@ -365,13 +401,26 @@ SANDY_API int sandy_gemm_f32_tc(const float* a, const float* w, const float* bia
     if (M == 0 || N == 0) return SANDY_OK;
     if (!a || !w || !out || K <= 0 || M < 0 || N < 0) return SANDY_ERR_ARGUMENT;
     if (K % 4 || lda % 4 || ldw % 4 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15)) return SANDY_ERR_UNSUPPORTED;
-    if (tile == 0 && parts == 0) choose(M, N, K, tile, parts);
+    if (tile == 0 && parts == 0) choose((M + BM - 1) / BM, N, K, tile, parts);
     if (parts < 1 || parts > MAX_PARTS || (parts & (parts - 1)) || parts > (K + CHUNK - 1) / CHUNK) return SANDY_ERR_ARGUMENT;
-    if ((M + BM - 1) / BM > 65535) return SANDY_ERR_UNSUPPORTED;
     const bool wide = !((uintptr_t)out & 15) && ldc % 4 == 0 && (!residual || (!((uintptr_t)residual & 15) && ldr % 4 == 0));
-    const Product p = {a, w, bias, residual, out, M, N, K, lda, ldw, ldr, ldc, act, wide ? 1 : 0};
-    if (tile == 64) return launch<64>(p, parts, status, stream);
-    if (tile == 96) return launch<96>(p, parts, status, stream);
-    if (tile == 128) return launch<128>(p, parts, status, stream);
-    return SANDY_ERR_ARGUMENT;
+    const Product p = {a, w, bias, residual, out, M, N, K, lda, ldw, ldr, ldc, act, wide ? 1 : 0, nullptr, 1};
+    return launch_tile<PLAIN>(tile, p, (M + BM - 1) / BM, parts, N, status, stream);
+}
+
+// Per expert: a [n_slots, K] with the rows of an expert one after another, w [G * N, K], group_start int32 [G + 1] on the device; act: 0
+// none, 1 the square of relu.
+SANDY_API int sandy_expert_product_f32_tc(const float* a, int lda, const float* w, int ldw, float* out, int ldo, int n_slots, int n_groups,
+                                          int N, int K, const int* group_start, int act, int* status, cudaStream_t stream) {
+    if (n_slots == 0 || n_groups == 0 || N == 0) return SANDY_OK;
+    if (!a || !w || !out || !group_start || K <= 0 || n_slots < 0 || n_groups < 0 || N < 0) return SANDY_ERR_ARGUMENT;
+    if (K % 4 || lda % 4 || ldw % 4 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15)) return SANDY_ERR_UNSUPPORTED;
+    const bool wide = !((uintptr_t)out & 15) && ldo % 4 == 0;
+    const Product p = {a, w, nullptr, nullptr, out, n_slots, N, K, lda, ldw, 0, ldo, act == 1 ? SANDY_ACT_RELU_SQUARED : SANDY_ACT_NONE, wide ? 1 : 0,
+                       group_start, n_groups};
+    // as many tiles as evenly spread rows would have
+    const long long spread = (long long)n_groups * (((n_slots + n_groups - 1) / n_groups + BM - 1) / BM);
+    int tile, parts;
+    choose(std::min<long long>(spread, n_slots), N, K, tile, parts);
+    return launch_tile<EXPERTS>(tile, p, (n_slots + BM - 1) / BM + n_groups, parts, (long long)n_groups * N, status, stream);
 }

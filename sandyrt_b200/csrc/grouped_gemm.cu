@@ -17,7 +17,7 @@
 // stages and read with ldmatrix; rows a tile does not have are zero-filled, so a decode step's one or two rows per
 // expert cost a tile's weight traffic and nothing else).  float32 operands in rows of whole 16 bytes: tiles of 64 x 64 with packed fma behind a
 // cp.async ring, as in gemm_f32.cu, or, where a group has few rows, its weights streamed past them, a warp four rows of w.
-// What is left (odd sizes) takes plain FFMA tiles.  Which kernel runs is a matter of the sizes and of the most rows a step
+// Experts with more rows and large matrices go to gemm_f32_tc.cu (core/ops.cpp).  What is left (odd sizes) takes plain FFMA tiles.  Which kernel runs is a matter of the sizes and of the most rows a step
 // may bring, never of how they fall on the groups.
 #include "common.cuh"
 

@@ -723,6 +723,21 @@ def expert_product_tc(r: Routing, a_sorted, w, out, *, act: str = "none") -> Non
     _check(code, f"expert_product_tc(E={r.n_experts},N={N},K={K})")
 
 
+def expert_product_f32_tc(r: Routing, a_sorted, w, out, *, act: str = "none") -> None:
+    """The per-expert product of float32 operands on the tensor cores, in three bfloat16 pieces each; a_sorted as in
+    expert_product_tc."""
+    _cuda(a_sorted, w, out)
+    N, K = w.shape[0] // r.n_experts, w.shape[1]
+    _f32(a_sorted, "a_sorted"); _f32(w, "w"); _f32(out, "out")
+    if not w.is_contiguous() or a_sorted.stride(1) != 1 or out.stride(1) != 1:
+        raise KernelError("expert_product_f32_tc: w [E * N, K] contiguous expected")
+    code = load_library("gemm_f32_tc").sandy_expert_product_f32_tc(
+        _p(a_sorted), ctypes.c_int(a_sorted.stride(0)), _p(w), ctypes.c_int(K), _p(out), ctypes.c_int(out.stride(0)),
+        ctypes.c_int(r.n_tokens * r.top), ctypes.c_int(r.n_experts), ctypes.c_int(N), ctypes.c_int(K), _p(r.group_start),
+        ctypes.c_int({"none": 0, "relu_squared": 1}[act]), _p(kernel_status(out.device)), _stream())
+    _check(code, f"expert_product_f32_tc(E={r.n_experts},N={N},K={K})")
+
+
 def moe_combine(r: Routing, rows, y, *, add: bool) -> None:
     """y[t] (+)= sum_j weight[t, j] * rows[slot of (t, j)]; float32."""
     _cuda(rows, y)

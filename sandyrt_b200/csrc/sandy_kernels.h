@@ -41,6 +41,8 @@ int sandy_gemm_f32(const float* a, const float* w, const float* bias, const floa
 /* gemm_f32_tc.cu */
 int sandy_gemm_f32_tc(const float* a, const float* w, const float* bias, const float* residual, float* out, int M, int N, int K,
                       int lda, int ldw, int ldr, int ldc, int act, int tile, int parts, int* status, cudaStream_t stream);
+int sandy_expert_product_f32_tc(const float* a, int lda, const float* w, int ldw, float* out, int ldo, int n_slots, int n_groups, int N,
+                                int K, const int* group_start, int act, int* status, cudaStream_t stream);
 
 /* gemm_tc.cu, gemm_tc2.cu */
 int sandy_gemm_tc(const void* a, const void* w, const void* bias, const float* residual, void* out, int M, int N, int K,

@@ -284,6 +284,35 @@ def test_expert_product_f32_infinity_at_the_end_of_a_row(sizes, K):
     assert torch.isfinite(out[:n - 1]).all()
 
 
+@pytest.mark.parametrize("sizes,N,K", [([1, 0, 2, 1], 33, 132), ([128, 129, 0, 127, 1], 130, 576), ([300], 64, 64), ([5, 9], 1000, 768)])
+def test_expert_product_f32_on_tensor_cores(sizes, N, K):
+    """Tiles that begin and end inside a's rows, empty groups, columns behind N that are the next expert's; an infinite activation stays
+    its own row's; rows behind the last group are not written."""
+    from sandyrt_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(N + K)
+    n, G = sum(sizes), len(sizes)
+    a, w = torch.randn(n + 3, K, generator=g), torch.randn(G, N, K, generator=g)
+    a[n:] = float("nan")
+    start = torch.tensor([0] + list(np.cumsum(sizes)), dtype=torch.int32)
+    r = types.SimpleNamespace(n_experts=G, n_tokens=n + 3, top=1, group_start=start.to(DEV))
+    out = torch.full((n + 3, N), 7.0, device=DEV)
+    ops.expert_product_f32_tc(r, a.to(DEV), w.view(G * N, K).to(DEV), out, act="relu_squared")
+    which = torch.repeat_interleave(torch.arange(G), torch.tensor(sizes))
+    z = torch.einsum("sk,snk->sn", a[:n].double(), w[which].double())
+    off = (K + 2) * 2.0 ** -24 * torch.einsum("sk,snk->sn", a[:n].double().abs(), w[which].double().abs())
+    want = torch.relu(z) ** 2
+    assert bool(((out[:n].double().cpu() - want).abs() <= 2 * torch.relu(z) * off + off ** 2 + 2.0 ** -23 * want).all())
+    assert bool((out[n:] == 7.0).all())
+    finite, again = torch.empty(n + 3, N, device=DEV), torch.empty(n + 3, N, device=DEV)
+    ops.expert_product_f32_tc(r, a.to(DEV), w.view(G * N, K).to(DEV), finite)
+    a[n - 1, K - 1] = float("inf")
+    ops.expert_product_f32_tc(r, a.to(DEV), w.view(G * N, K).to(DEV), again)
+    assert torch.equal(again[n - 1].cpu(), torch.sign(w[which[n - 1], :, K - 1]) * float("inf"))
+    assert torch.equal(again[:n - 1], finite[:n - 1])
+    assert int(ops.kernel_status(out.device).item()) == 0
+
+
 @pytest.mark.parametrize("T", [1, 4, 5, 64, 65, 150])
 def test_head_product_f32(T):
     from sandyrt_b200.csrc import ops
