@@ -254,9 +254,9 @@ Engine::Prepared Engine::prepare(const std::vector<StepEntry>& entries, const st
     c.host_slots = slots;
     c.max_q_len = max_q;
     c.max_kv_len = max_kv + extra;
-    // What the attention of a mixed step chooses its launches by (bfloat16 only).  Part of the graph's key, so rounded down: nothing
+    // What the attention of a mixed step chooses its launches by.  Part of the graph's key, so rounded down: nothing
     // below eight, then powers of two.
-    if (dtype_ == DType::BF16 && max_q > 1) {
+    if (max_q > 1) {
         const int singles = (int)std::count(q_lens.begin(), q_lens.end(), 1);
         for (int n = 8; n <= singles; n *= 2) c.n_single = n;
     }

@@ -604,6 +604,32 @@ void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const K
     }
     // float32 prompts (the general kernel also keeps heads above 128)
     if (s.max_q_len > 1 && q.dtype == DType::F32 && d <= 128 && !prompt_f32_general(d, s.max_q_len, s.max_blocks * c.page_size)) {
+        // Heads above 32 go to the tensor cores, whose blocks take 128 queries; single tokens beside the portions are best on the decode
+        // kernel, and where there are many that it has no form for (its head sizes, its rules) on the fma tiles of 64 queries.  Alone,
+        // us, fma tiles / tensor cores / tensor cores and decode kernel, single tokens behind some 100 to 700 keys beside a portion: 16
+        // heads of 64, 32 beside 480 109 / 113 / 73; 12 heads, 60 beside 16 134 / 179 / 97, 16 beside 300 52 / 41 / 30, 8 beside 300 48 /
+        // 22 / 26, 8 beside 30 33 / 21 / 15; 25 heads, 20 beside 200 63 / 55 / 30; 12 heads of 128, 32 beside 100 180 / 190 / 85.
+        const int seen = window > 0 ? std::min(window + keep, s.max_blocks * c.page_size) : s.max_blocks * c.page_size;
+        const bool decodable = (d == 64 || d == 128) && !ruled && !db && !gated && s.n_seqs <= 65535 && q.ld % 4 == 0 && !((uintptr_t)q.data & 15);
+        const bool apart = decodable && s.n_single * n_heads >= 150 && seen > 128;
+        if (d > 32 && (apart || s.n_single * n_heads < 384)) {
+            static auto fn = SANDY_KERNEL(attention_prefill_f32_tc, sandy_prefill_attention_f32_tc_rules);
+            OpTimer timer(l, "attention, prompt (float32, tcgen05)", attn_bytes, attn_flops);
+            const int code = fn((const float*)q.data, (int)q.ld, (const float*)c.k, (const float*)c.v, c.page_stride, s.block_table,
+                                s.max_blocks, s.q_start, s.kv_before, (float*)out.data, (int)out.ld, s.n_seqs, s.max_q_len, n_heads, hkv, d,
+                                c.page_size, scale, &rules, apart ? 2 : 0, c.num_pages, l.kernel_status, l.stream);
+            if (code != -1) {
+                check(code, "prefill_attention_f32_tc" + shape);
+                if (!apart) return;
+                static auto single = SANDY_KERNEL(attention_decode, sandy_decode_attention_single);
+                const int splits = std::min(kClusterMaxSplits, std::max(decode_splits(s.n_single, n_heads, seen), seen / 128));
+                check(single((const float*)q.data, (int)q.ld, (const float*)c.k, (const float*)c.v, c.page_stride, s.block_table, s.max_blocks,
+                             s.q_start, s.kv_before, (float*)out.data, (int)out.ld, s.n_seqs, n_heads, hkv, d, c.page_size, scale, window,
+                             splits, c.num_pages, sk, og, l.kernel_status, l.stream),
+                      "decode_attention_single" + shape);
+                return;
+            }
+        }
         static auto fn = SANDY_KERNEL(attention_prefill_f32, sandy_prefill_attention_f32_rules);
         OpTimer timer(l, "attention, prompt (float32)", attn_bytes, attn_flops);
         const int code = fn((const float*)q.data, (int)q.ld, (const float*)c.k, (const float*)c.v, c.page_stride, s.block_table,

@@ -76,7 +76,7 @@ struct StepContext {
     // host copies, for parts that plan their launches on the host
     std::vector<int> host_q_lens, host_kv_before, host_slots;
     int max_q_len = 0, max_kv_len = 0;
-    int n_single = 0;                    // of a bfloat16 step with portions: requests that bring one token, see Engine::prepare
+    int n_single = 0;                    // of a step with portions: requests that bring one token, see Engine::prepare
     ops::Launch launch;                  // stream and status words
 
     // `window` and `keep_first` of the layer that asks: the profile's figures count the keys it looks at

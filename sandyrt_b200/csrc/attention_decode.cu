@@ -92,10 +92,10 @@ __device__ __forceinline__ void copy16_async(uint8_t* dst, const void* src) {
 // The last step of a softmax row: a sink joins the denominator (exp(sink) relative to the row's maximum M,
 // nothing in the numerator), an output gate scales the head's result.
 __device__ __forceinline__ float finish_row(float O, float L, float M, const float* sink, const float* out_gate, int t,
-                                            int h, int n_heads) {
+                                            int h, int n_heads, bool keep_nan = false) {
     if (sink && M > -INFINITY) L += expf(sink[h] - M);
     const float g = out_gate ? out_gate[(size_t)t * n_heads + h] : 1.0f;
-    return L > 0.0f ? O / L * g : 0.0f;
+    return L > 0.0f || (keep_nan && L != L) ? O / L * g : 0.0f;
 }
 
 template <typename T, int D>
@@ -107,7 +107,7 @@ decode_attention_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__
                         T* __restrict__ out, int ld_out, float* __restrict__ partial_o,
                         float* __restrict__ partial_ml, int n_heads, int n_kv_heads, int page_size,
                         float scale, int window, int num_splits, int num_pages, const float* __restrict__ sink,
-                        const float* __restrict__ out_gate, int* __restrict__ status) {
+                        const float* __restrict__ out_gate, const int* __restrict__ single_of, int* __restrict__ status) {
     constexpr int VEC = 16 / sizeof(T);         // elements per 16-byte piece
     constexpr int LPK = D / VEC;                // lanes per key
     constexpr int KPW = 32 / LPK;               // keys per warp per round
@@ -126,16 +126,29 @@ decode_attention_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__
     __shared__ uint8_t st_ok[STAGE_KEYS];       // whether a staged key had a page behind it
 
     pdl_launch_dependents();
+    // With single_of (q_start of a step of mixed requests) blockIdx.z is a request, positions are the requests' first, and only
+    // requests that bring one token are taken; all blocks of a cluster leave together.  There a score that is NaN is one in the
+    // result too, as it is for the portions beside.
+    int t = blockIdx.z, s;
+    if (single_of) {
+        s = t;
+        t = single_of[s];
+        if (single_of[s + 1] - t != 1) {
+            pdl_wait();                                 // a kernel ends only after the one before it has
+            return;
+        }
+    } else {
+        s = token_seq[t];
+    }
     const bool in_cluster = num_splits > 1 && partial_o == nullptr;
     // A block may write into another block's shared memory only once that block is running: every
     // block says so here, and waits for the others only when it has its partial state to hand over.
     if (in_cluster) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    const int split = blockIdx.x, h = blockIdx.y, t = blockIdx.z;
+    const int split = blockIdx.x, h = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane / LPK, sub = lane % LPK;
     const int group = warp * KPW + g;
-    const int s = token_seq[t];
-    const int pos = positions[t];
+    const int pos = positions[blockIdx.z];
     const int kvh = h / (n_heads / n_kv_heads);
     const int lo = window > 0 ? max(0, pos + 1 - window) : 0;
     const int n_keys = pos - lo + 1;
@@ -230,15 +243,16 @@ decode_attention_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__
         float m_new = m;
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) m_new = fmaxf(m_new, sc[u]);
-        if (m_new > -INFINITY) {
-            const float corr = expf(m - m_new);              // exp(-inf) = 0 while nothing has been seen yet
+        if (m_new > -INFINITY || single_of) {
+            const float base = m_new > -INFINITY ? m_new : 0.0f;
+            const float corr = expf(m - base);               // exp(-inf) = 0 while nothing has been seen yet
             l *= corr;
 #pragma unroll
             for (int i = 0; i < VEC; i++) o[i] *= corr;
 #pragma unroll
             for (int u = 0; u < UNROLL; u++) {
                 if (ok[u]) {
-                    const float p = expf(sc[u] - m_new);
+                    const float p = expf(sc[u] - base);
                     l += p;
 #pragma unroll
                     for (int i = 0; i < VEC; i++) o[i] = fmaf(p, vf[u][i], o[i]);
@@ -267,16 +281,16 @@ decode_attention_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__
 #pragma unroll
         for (int i = 0; i < GROUPS; i++) M = fmaxf(M, sm_m[i]);
         float L = 0.0f, O = 0.0f;
-        if (M > -INFINITY) {
+        if (M > -INFINITY || single_of) {
 #pragma unroll
             for (int i = 0; i < GROUPS; i++) {
-                const float w = expf(sm_m[i] - M);     // exp(-inf) = 0 for groups that saw no key
+                const float w = expf(sm_m[i] - (M > -INFINITY ? M : 0.0f));     // exp(-inf) = 0 for groups that saw no key
                 L = fmaf(sm_l[i], w, L);
                 O = fmaf(sm_o[i][d], w, O);
             }
         }
         if (num_splits == 1) {
-            out[(size_t)t * ld_out + h * D + d] = from_f32<T>(finish_row(O, L, M, sink, out_gate, t, h, n_heads));
+            out[(size_t)t * ld_out + h * D + d] = from_f32<T>(finish_row(O, L, M, sink, out_gate, t, h, n_heads, single_of));
         } else if (partial_o == nullptr) {
             // cluster mode: the splits of this (token, head) are the blocks of one cluster, and each
             // hands its partial state to the first block's shared memory
@@ -304,14 +318,14 @@ decode_attention_kernel(const T* __restrict__ q, int ld_q, const T* __restrict__
             for (int r = 0; r < num_splits; r++) M = fmaxf(M, cl_all[r][D]);
             for (int d = threadIdx.x; d < D; d += WARPS * 32) {
                 float L = 0.0f, O = 0.0f;
-                if (M > -INFINITY) {
+                if (M > -INFINITY || single_of) {
                     for (int r = 0; r < num_splits; r++) {
-                        const float w = expf(cl_all[r][D] - M);
+                        const float w = expf(cl_all[r][D] - (M > -INFINITY ? M : 0.0f));
                         L = fmaf(cl_all[r][D + 1], w, L);
                         O = fmaf(cl_all[r][d], w, O);
                     }
                 }
-                out[(size_t)t * ld_out + h * D + d] = from_f32<T>(finish_row(O, L, M, sink, out_gate, t, h, n_heads));
+                out[(size_t)t * ld_out + h * D + d] = from_f32<T>(finish_row(O, L, M, sink, out_gate, t, h, n_heads, single_of));
             }
         }
     }
@@ -345,7 +359,7 @@ int launch(const void* q, int ld_q, const void* k_cache, const void* v_cache, lo
            const int* block_table, int max_blocks, const int* token_seq, const int* positions, void* out,
            int ld_out, float* scratch, int n_tokens, int n_heads, int n_kv_heads, int page_size, float scale,
            int window, int num_splits, int num_pages, const float* sink, const float* out_gate, int* status,
-           cudaStream_t stream) {
+           cudaStream_t stream, const int* single_of = nullptr) {
     float* partial_o = scratch;
     float* partial_ml = scratch ? scratch + (size_t)n_tokens * n_heads * num_splits * D : nullptr;
     dim3 grid(num_splits, n_heads, n_tokens);
@@ -353,7 +367,7 @@ int launch(const void* q, int ld_q, const void* k_cache, const void* v_cache, lo
                             (const T*)k_cache, (const T*)v_cache, page_stride, block_table, max_blocks, token_seq,
                             positions, (T*)out, ld_out, partial_o, partial_ml, n_heads, n_kv_heads, page_size, scale,
                             window, num_splits, num_pages, num_splits == 1 ? sink : nullptr,
-                            num_splits == 1 ? out_gate : nullptr, status);
+                            num_splits == 1 ? out_gate : nullptr, single_of, status);
     if (code != 0 || num_splits == 1) return code;
     return sandy_launch(merge_splits_kernel<T, D>, dim3(n_heads, n_tokens), dim3(D < 32 ? 32 : (D > 256 ? 256 : D)), 0,
                         stream, (const float*)partial_o, (const float*)partial_ml, (T*)out, ld_out, n_heads, num_splits,
@@ -366,7 +380,7 @@ int launch_cluster(const void* q, int ld_q, const void* k_cache, const void* v_c
                    const int* block_table, int max_blocks, const int* token_seq, const int* positions, void* out,
                    int ld_out, int n_tokens, int n_heads, int n_kv_heads, int page_size, float scale, int window,
                    int num_splits, int num_pages, const float* sink, const float* out_gate, int* status,
-                   cudaStream_t stream) {
+                   cudaStream_t stream, const int* single_of = nullptr) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(num_splits, n_heads, n_tokens);
     cfg.blockDim = dim3(WARPS * 32);
@@ -384,7 +398,7 @@ int launch_cluster(const void* q, int ld_q, const void* k_cache, const void* v_c
     const cudaError_t e = cudaLaunchKernelEx(
         &cfg, decode_attention_kernel<T, D>, (const T*)q, ld_q, (const T*)k_cache, (const T*)v_cache, page_stride,
         block_table, max_blocks, token_seq, positions, (T*)out, ld_out, (float*)nullptr, (float*)nullptr, n_heads,
-        n_kv_heads, page_size, scale, window, num_splits, num_pages, sink, out_gate, status);
+        n_kv_heads, page_size, scale, window, num_splits, num_pages, sink, out_gate, single_of, status);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
@@ -458,6 +472,28 @@ SANDY_API int sandy_decode_attention_ext(const void* q, int ld_q, const void* k_
 }
 
 // The two forms above without a sink or an output gate.
+// For a step of mixed requests in float32: takes the requests that bring one token (q_start [n_seqs + 1], kv_before [n_seqs]) and leaves
+// the others' rows alone; heads of 64 and 128.
+SANDY_API int sandy_decode_attention_single(const float* q, int ld_q, const float* k_cache, const float* v_cache, long long page_stride,
+                                            const int* block_table, int max_blocks, const int* q_start, const int* kv_before,
+                                            float* out, int ld_out, int n_seqs, int n_heads, int n_kv_heads, int head_dim,
+                                            int page_size, float scale, int window, int num_splits, int num_pages, const float* sink,
+                                            const float* out_gate, int* status, cudaStream_t stream) {
+    if (n_seqs == 0) return SANDY_OK;
+    if (!q || !k_cache || !v_cache || !block_table || !q_start || !kv_before || !out) return SANDY_ERR_ARGUMENT;
+    if (num_splits < 1 || num_splits > MAX_CLUSTER_SPLITS || (head_dim != 64 && head_dim != 128)) return SANDY_ERR_UNSUPPORTED;
+    if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0 || page_size <= 0 || window < 0) return SANDY_ERR_UNSUPPORTED;
+    if (n_heads > 65535 || n_seqs > 65535 || ld_q % 4 != 0 || page_stride % 4 != 0) return SANDY_ERR_UNSUPPORTED;
+    if (((uintptr_t)q & 15) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15)) return SANDY_ERR_UNSUPPORTED;
+    if (num_splits == 1)
+        return (head_dim == 64 ? launch<float, 64> : launch<float, 128>)(
+            q, ld_q, k_cache, v_cache, page_stride, block_table, max_blocks, nullptr, kv_before, out, ld_out, nullptr, n_seqs, n_heads,
+            n_kv_heads, page_size, scale, window, 1, num_pages, sink, out_gate, status, stream, q_start);
+    return (head_dim == 64 ? launch_cluster<float, 64> : launch_cluster<float, 128>)(
+        q, ld_q, k_cache, v_cache, page_stride, block_table, max_blocks, nullptr, kv_before, out, ld_out, n_seqs, n_heads, n_kv_heads,
+        page_size, scale, window, num_splits, num_pages, sink, out_gate, status, stream, q_start);
+}
+
 SANDY_API int sandy_decode_attention_cluster(const void* q, int ld_q, const void* k_cache, const void* v_cache,
                                              long long page_stride, const int* block_table, int max_blocks,
                                              const int* token_seq, const int* positions, void* out, int ld_out,

@@ -50,6 +50,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "attention_prefill": [],
     "attention_prefill_tc": [],
     "attention_prefill_f32": [],
+    "attention_prefill_f32_tc": [],
     "sampling": [],
     "rmsnorm": [],
     "elementwise": [],

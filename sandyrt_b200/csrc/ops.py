@@ -464,9 +464,11 @@ def mixed_attention(q, k_cache, v_cache, block_table, q_start, kv_before, out, *
 
 def prefill_attention_f32(q, k_cache, v_cache, block_table, q_start, kv_before, out, *, sink=None, out_gate=None, n_heads: int,
                           max_q_len: int, scale: float, window: int = 0, softcap: float = 0.0, chunk: int = 0, dist_bias=None,
-                          keep_first: int = 0, elem_gate=None) -> None:
+                          keep_first: int = 0, elem_gate=None, tc: bool = False,
+                          single_splits: int = 0) -> None:
     """Attention of prompt portions in float32, head sizes 16..128 in steps of 16; q_start and kv_before as in prefill_attention,
-    the rules as in paged_attention."""
+    the rules as in paged_attention.  tc: on the tensor cores, in three bfloat16 pieces (head sizes above 32).
+    single_splits > 0: those of one token go to the decode kernel, in so many splits (heads of 64 and 128, at least one portion)."""
     _cuda(q, k_cache, v_cache, block_table, q_start, kv_before, out, sink, out_gate)
     hkv, ps, d, page_stride, num_pages = _cache_args(k_cache, v_cache)
     if q.dtype != torch.float32 or d % 16 != 0 or d > 128:
@@ -478,13 +480,22 @@ def prefill_attention_f32(q, k_cache, v_cache, block_table, q_start, kv_before, 
     S = kv_before.numel()
     if q_start.numel() != S + 1 or block_table.shape[0] != S:
         raise KernelError("prefill_attention_f32: q_start, kv_before and block_table disagree on the requests")
-    code = load_library("attention_prefill_f32").sandy_prefill_attention_f32_rules(
-        _p(q), ctypes.c_int(q.stride(0)), _p(k_cache), _p(v_cache), ctypes.c_longlong(page_stride), _p(block_table),
-        ctypes.c_int(block_table.shape[1]), _p(q_start), _p(kv_before), _p(out), ctypes.c_int(out.stride(0)), ctypes.c_int(S),
-        ctypes.c_int(max_q_len), ctypes.c_int(n_heads), ctypes.c_int(hkv), ctypes.c_int(d), ctypes.c_int(ps), ctypes.c_float(scale),
-        _rules(q, n_heads, window, keep_first, softcap, chunk, sink, out_gate, dist_bias, elem_gate), ctypes.c_int(num_pages),
-        _p(kernel_status(q.device)), _stream())
-    _check(code, f"prefill_attention_f32(H={n_heads},Hkv={hkv},D={d})")
+    rules = _rules(q, n_heads, window, keep_first, softcap, chunk, sink, out_gate, dist_bias, elem_gate)
+    head = (_p(q), ctypes.c_int(q.stride(0)), _p(k_cache), _p(v_cache), ctypes.c_longlong(page_stride), _p(block_table),
+            ctypes.c_int(block_table.shape[1]), _p(q_start), _p(kv_before), _p(out), ctypes.c_int(out.stride(0)), ctypes.c_int(S))
+    sizes = (ctypes.c_int(n_heads), ctypes.c_int(hkv), ctypes.c_int(d), ctypes.c_int(ps), ctypes.c_float(scale))
+    last = (ctypes.c_int(num_pages), _p(kernel_status(q.device)))
+    name = f"prefill_attention_f32(H={n_heads},Hkv={hkv},D={d})"
+    if not tc:
+        _check(load_library("attention_prefill_f32").sandy_prefill_attention_f32_rules(*head, ctypes.c_int(max_q_len), *sizes, rules, *last, _stream()), name)
+        return
+    _check(load_library("attention_prefill_f32_tc").sandy_prefill_attention_f32_tc_rules(
+        *head, ctypes.c_int(max_q_len), *sizes, rules, ctypes.c_int(2 if single_splits else 0), *last, _stream()), name)
+    if single_splits:
+        code = load_library("attention_decode").sandy_decode_attention_single(
+            *head, *sizes, ctypes.c_int(window), ctypes.c_int(single_splits), ctypes.c_int(num_pages), _p(sink), _p(out_gate),
+            _p(kernel_status(q.device)), _stream())
+        _check(code, f"decode_attention_single(H={n_heads},Hkv={hkv},D={d},splits={single_splits})")
 
 
 def _f32(t, name: str) -> None:

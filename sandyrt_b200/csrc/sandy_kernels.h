@@ -121,6 +121,13 @@ int sandy_prefill_attention_f32_rules(const float* q, int ld_q, const float* k_c
                                       int page_size, float scale, const SandyAttentionRules* rules, int num_pages, int* status,
                                       cudaStream_t stream);
 
+/* attention_prefill_f32_tc.cu */
+int sandy_prefill_attention_f32_tc_rules(const float* q, int ld_q, const float* k_cache, const float* v_cache, long long page_stride,
+                                         const int* block_table, int max_blocks, const int* q_start, const int* kv_before,
+                                         float* out, int ld_out, int n_seqs, int max_q_len, int n_heads, int n_kv_heads,
+                                         int head_dim, int page_size, float scale, const SandyAttentionRules* rules, int portions,
+                                         int num_pages, int* status, cudaStream_t stream);
+
 int sandy_prefill_attention_tc(const void* q, int ld_q, const void* k_cache, const void* v_cache, long long page_stride,
                                const int* block_table, int max_blocks, const int* q_start, const int* kv_before, void* out,
                                int ld_out, int n_seqs, int max_q_len, int n_heads, int n_kv_heads, int head_dim,
@@ -170,6 +177,11 @@ int sandy_decode_attention_shared_cap(const void* q, int ld_q, const void* k_cac
                                       int page_size, float scale, int window, float softcap, int chunk, int splits,
                                       int num_pages, const float* sink, const float* out_gate, float* scratch, int* status,
                                       cudaStream_t stream);
+int sandy_decode_attention_single(const float* q, int ld_q, const float* k_cache, const float* v_cache, long long page_stride,
+                                  const int* block_table, int max_blocks, const int* q_start, const int* kv_before, float* out,
+                                  int ld_out, int n_seqs, int n_heads, int n_kv_heads, int head_dim, int page_size, float scale,
+                                  int window, int num_splits, int num_pages, const float* sink, const float* out_gate, int* status,
+                                  cudaStream_t stream);
 int sandy_decode_attention_cluster_ext(const void* q, int ld_q, const void* k_cache, const void* v_cache, long long page_stride,
                                        const int* block_table, int max_blocks, const int* token_seq, const int* positions,
                                        void* out, int ld_out, int n_tokens, int n_heads, int n_kv_heads, int head_dim,

@@ -9,7 +9,7 @@
 // then added into registers with ordinary float additions.
 //
 // A bfloat16 ends where a float does, so the pieces of small floats would lose their low bits: both operands are split at
-// SCALE times their size, which keeps every float's 24 bits, and the sums are scaled back (both exact).  What is large enough
+// SCALE times their size, which keeps every bit of the smallest float, and the sums are scaled back (both exact).  What is large enough
 // to overflow for that, infinities and NaN come out as infinity or NaN; write-backs form every sum that is not finite again,
 // with float arithmetic from the operands (plain_sum), so they end as they would there.
 #pragma once
@@ -25,7 +25,7 @@ constexpr int N_PRODUCTS = 6;
 __device__ constexpr int PIECE_OF_A[N_PRODUCTS] = {0, 1, 2, 0, 1, 0};
 __device__ constexpr int PIECE_OF_W[N_PRODUCTS] = {2, 1, 0, 1, 0, 0};
 
-constexpr float SCALE = 0x1p40f, UNSCALE = 0x1p-80f;        // of an operand, of a sum of products
+constexpr float SCALE = 0x1p20f, UNSCALE = 0x1p-40f;        // of an operand, of a sum of products
 
 // Two floats into their three pieces, each a pair of bfloat16 (x0 in the low half).
 __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t (&piece)[N_PIECES]) {

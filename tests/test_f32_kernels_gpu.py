@@ -1,4 +1,5 @@
 """The float32 kernels alone, at the edges of their tiles and splits, against torch in 64 bits."""
+import functools
 import types
 
 import numpy as np
@@ -208,6 +209,66 @@ def test_a_token_that_is_not_finite_reaches_every_query_that_sees_it(D, window, 
     assert (got.double().cpu() - want)[fine].abs().max().item() < 2e-5      # the bound of test_prompt_attention_f32
     if bad != "key":                                        # (the general kernel gives a NaN score no weight)
         assert torch.equal(torch.isnan(got), torch.isnan(general))
+
+
+@pytest.fixture
+def on_tensor_cores(monkeypatch):
+    from sandyrt_b200.csrc import ops
+
+    monkeypatch.setattr(ops, "prefill_attention_f32", functools.partial(ops.prefill_attention_f32, tc=True))
+
+
+@pytest.mark.parametrize("rules", RULES)
+@pytest.mark.parametrize("H,Hkv,D,page_size", [(3, 3, 64, 16), (4, 2, 48, 8), (2, 1, 128, 32), (3, 1, 80, 4), (2, 2, 64, 1)])
+def test_prompt_attention_f32_on_tensor_cores(on_tensor_cores, H, Hkv, D, page_size, rules):
+    test_prompt_attention_f32(H, Hkv, D, page_size, rules)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_tokens_that_are_not_finite_on_tensor_cores(on_tensor_cores, D):
+    """A tile that holds one is formed with float arithmetic: the same queries as before, and no others."""
+    for bad in (float("nan"), float("inf")):
+        test_a_value_that_is_not_finite_reaches_only_the_queries_that_see_it(D, bad)
+    for bad in ("key", "key and value", "query", "score of minus infinity", "score of minus infinity and value"):
+        for window, with_sink in ((0, False), (90, True)):
+            test_a_token_that_is_not_finite_reaches_every_query_that_sees_it(D, window, with_sink, bad)
+
+
+@pytest.mark.parametrize("D,splits", [(64, 1), (64, 3), (128, 1), (128, 8)])
+@pytest.mark.parametrize("window,bad", [(0, None), (50, None), (0, "key"), (0, "query")])
+def test_single_tokens_beside_portions_on_the_decode_kernel(D, splits, window, bad):
+    """Requests of one token (the first of a context among them) beside portions; a NaN key or query is one in every row that sees it."""
+    from sandyrt_b200.csrc import ops
+
+    seqs = [(0, 1), (40, 1), (0, 70), (199, 1), (330, 1), (64, 65), (17, 1)]
+    case = _paged_case(torch.float32, 4, 2, D, 16, seqs, seed=D)
+    if bad == "key":
+        case["kc"][int(case["table"][4, 200 // 16]), :, 200 % 16] = float("nan")
+    if bad == "query":
+        case["q"][1 + 1 + 70] = float("nan")                # the token behind 199
+    sink = torch.tensor([0.5, -1.0, 0.0, 2.0], device=DEV)
+    q_start = torch.tensor([0] + list(np.cumsum([n for _, n in seqs])), dtype=torch.int32, device=DEV)
+    kv_before = torch.tensor([b for b, _ in seqs], dtype=torch.int32, device=DEV)
+    outs = [torch.full(case["q"].shape, 7.0, device=DEV) for _ in range(2)]
+    for out, kw in zip(outs, ({}, {"tc": True, "single_splits": splits})):
+        ops.prefill_attention_f32(case["q"], case["kc"], case["vc"], case["table"], q_start, kv_before, out, n_heads=4, max_q_len=70, scale=0.1,
+                                  window=window, sink=sink, **kw)
+    ops.check_kernel_status(DEV)
+    want, got = outs
+    assert torch.isnan(want).any() == (bad is not None) and torch.equal(torch.isnan(got), torch.isnan(want))
+    fine = ~torch.isnan(want)
+    assert (got - want)[fine].abs().max().item() < 2e-5         # the bound of test_prompt_attention_f32
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("size", [2.0 ** -100, 2.0 ** 45])
+def test_prompt_attention_f32_sizes_on_tensor_cores(on_tensor_cores, D, size):
+    """Keys whose last pieces would lie below a bfloat16's range, and keys and values too large to be split."""
+    case = _paged_case(torch.float32, 2, 2, D, 16, [(0, 130), (63, 65)], seed=D)
+    case["kc"] *= size
+    case["vc"] *= size
+    got, want = _both(case, 2, {"scale": 0.8 / D ** 0.5 / size})
+    assert (got - want).abs().max().item() < 2e-5 * size        # the bound of test_prompt_attention_f32
 
 
 @pytest.mark.parametrize("name", ["A", "C"])
