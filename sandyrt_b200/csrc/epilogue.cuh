@@ -22,17 +22,17 @@ __device__ __forceinline__ float gelu_erf(float u) {
     return 0.5f * u * (1.0f + erff(u * 0.70710678118654752440f));
 }
 
-// gelu_new with tanh(y) = 1 - 2 / (exp(2y) + 1) on the fast exponential and division: a third
-// of tanhf's instructions, absolute error below 1e-6 (exp(2y) overflows to inf for large y,
-// giving exactly 1; underflows to 0 for very negative y, giving exactly -1).  For write-backs
-// that round to bfloat16 or sit in a tensor-core kernel's critical path; the 32-bit path keeps
-// tanhf.
+// gelu_new as u / (1 + exp(-2 y)), y = 0.79788456 (u + 0.044715 u^3), which is the formula above with tanh written out: two
+// special-function instructions and five others (with 1 - 2 / (exp(2 y) + 1) for tanh, __expf and __fdividef, twice as many, a
+// product of 2,048 x 3,072 x 768 took 16.2 us, with this 14.2).  Its relative error stays below 1e-6 where the
+// exponential is finite and not below 2^-126, the absolute one everywhere.  For write-backs that round to bfloat16 or sit in a
+// tensor-core kernel's critical path; the 32-bit path keeps tanhf.
 __device__ __forceinline__ float gelu_tanh_fast(float u) {
-    const float x2 = u * u;
-    const float inner = u + 0.044715f * (x2 * u);
-    const float e = __expf(1.5957691216057308f * inner);        // exp(2 * 0.79788456 * inner)
-    const float t = 1.0f - __fdividef(2.0f, e + 1.0f);
-    return (0.5f * u) * (1.0f + t);
+    // exp(-2 y) = 2^(u (c1 + c3 u^2)), c1 = -2 * 0.79788456 * log2(e), c3 = 0.044715 c1
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(u * fmaf(-0.10294324f, u * u, -2.3022082f)));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return u * r;
 }
 
 // relu(u)^2
