@@ -85,19 +85,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (elect_one()) {
+            // The first stages' weights, which no kernel writes, come while the kernel before is still running (with the other forms of
+            // this product: a prompt step of 2,048 tokens, 12 layers, 1,100 -> 1,074 us).
+            const int ahead = min(STAGES, k_tiles);
+            for (int kt = 0; kt < ahead; kt++) {
+                mbar_expect_tx(&full_bar[kt], L::STAGE_BYTES);
+                tma_load_2d(stage_base + kt * L::STAGE_BYTES + L::A_BYTES, &map_w, kt * BK, n0, &full_bar[kt]);
+            }
             pdl_wait();          // a may be the output of the kernel before
             for (int kt = 0; kt < k_tiles; kt++) {
                 const int s = kt % STAGES;
-                const uint32_t round = kt / STAGES;
-                if (!mbar_wait(&empty_bar[s], (round & 1) ^ 1)) {
-                    if (status) atomicOr(status, 1);
-                    break;
-                }
                 uint8_t* sa = stage_base + s * L::STAGE_BYTES;
-                uint8_t* sb = sa + L::A_BYTES;
-                mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
+                if (kt >= ahead) {
+                    if (!mbar_wait(&empty_bar[s], ((kt / STAGES) & 1) ^ 1)) {
+                        if (status) atomicOr(status, 1);
+                        break;
+                    }
+                    mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
+                    tma_load_2d(sa + L::A_BYTES, &map_w, kt * BK, n0, &full_bar[s]);
+                }
                 tma_load_2d(sa, &map_a, kt * BK, m0, &full_bar[s]);
-                tma_load_2d(sb, &map_w, kt * BK, n0, &full_bar[s]);
             }
         }
     } else if (warp == 1) {
@@ -222,6 +229,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (elect_one()) {
+            // The first stages' weights, which no kernel writes, come while the kernel before is still running.
+            const uint32_t ahead = min(STAGES, k_tiles);
+            for (uint32_t kt = 0; kt < ahead; kt++) {
+                mbar_expect_tx(&full_bar[kt], L::STAGE_BYTES);
+                tma_load_2d(stage_base + kt * L::STAGE_BYTES + L::A_BYTES, &map_w, kt * BK, blockIdx.x / m_tiles * BN, &full_bar[kt]);
+            }
             pdl_wait();             // a may be the output of the kernel before
             uint32_t it = 0;        // k-steps issued so far, over all tiles
             bool ok = true;
@@ -229,15 +242,17 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
                 const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * BN;
                 for (int kt = 0; kt < k_tiles; kt++, it++) {
                     const int s = it % STAGES;
-                    if (!mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1)) {
-                        if (status) atomicOr(status, 1);
-                        ok = false;
-                        break;
-                    }
                     uint8_t* sa = stage_base + s * L::STAGE_BYTES;
-                    mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
+                    if (it >= ahead) {
+                        if (!mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1)) {
+                            if (status) atomicOr(status, 1);
+                            ok = false;
+                            break;
+                        }
+                        mbar_expect_tx(&full_bar[s], L::STAGE_BYTES);
+                        tma_load_2d(sa + L::A_BYTES, &map_w, kt * BK, n0, &full_bar[s]);
+                    }
                     tma_load_2d(sa, &map_a, kt * BK, m0, &full_bar[s]);
-                    tma_load_2d(sa + L::A_BYTES, &map_w, kt * BK, n0, &full_bar[s]);
                 }
             }
         }

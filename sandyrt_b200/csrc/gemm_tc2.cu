@@ -141,6 +141,13 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
         if (elect_one()) {
+            // The first stages' weights, which no kernel writes, come while the kernel before is still running.
+            const uint32_t ahead = min(STAGES, k_tiles);
+            for (uint32_t kt = 0; kt < ahead; kt++) {
+                if (leader) mbar_expect_tx(&full_bar[kt], 2 * L::STAGE_BYTES);
+                tma_load_2d_pair(stage_base + kt * L::STAGE_BYTES + L::A_BYTES, &map_w, kt * BK, pair / m_tiles * BN + (int)rank * (BN / 2),
+                                 in_cta(smem_u32(&full_bar[kt]), 0));
+            }
             pdl_wait();          // a may be the output of the kernel before
             uint32_t it = 0;
             bool ok = true;
@@ -149,16 +156,18 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 const int n0 = (tile / m_tiles) * BN + (int)rank * (BN / 2);
                 for (int kt = 0; kt < k_tiles; kt++, it++) {
                     const int s = it % STAGES;
-                    if (!mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1)) {
-                        if (status) atomicOr(status, 1);
-                        ok = false;
-                        break;
-                    }
                     uint8_t* sa = stage_base + s * L::STAGE_BYTES;
-                    if (leader) mbar_expect_tx(&full_bar[s], 2 * L::STAGE_BYTES);
                     const uint32_t leader_full = in_cta(smem_u32(&full_bar[s]), 0);
+                    if (it >= ahead) {
+                        if (!mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1)) {
+                            if (status) atomicOr(status, 1);
+                            ok = false;
+                            break;
+                        }
+                        if (leader) mbar_expect_tx(&full_bar[s], 2 * L::STAGE_BYTES);
+                        tma_load_2d_pair(sa + L::A_BYTES, &map_w, kt * BK, n0, leader_full);
+                    }
                     tma_load_2d_pair(sa, &map_a, kt * BK, m0, leader_full);
-                    tma_load_2d_pair(sa + L::A_BYTES, &map_w, kt * BK, n0, leader_full);
                 }
             }
         }
