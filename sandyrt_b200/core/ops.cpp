@@ -177,6 +177,14 @@ static bool f32_on_tensor_cores(int64_t M, int64_t N, int64_t K) {
     return M > 64 || N > 896 || K < 512 || K > 1024;
 }
 
+// Those among them with a short k and few tiles, which the tensor cores' kernel would spend starting and ending: the kernel of 16 x 16
+// tiles in gemm_f32.cu.  us, short / tensor cores: 57 rows 192 x 64 2.5 / 5.3, 64 x 256 3.5 / 5.1; 256 rows 256 x 256 (64 K tiles times k)
+// 4.9 / 5.9; 1,024 rows 256 x 64 (64 K) 4.6 / 6.7, 96 x 256 (96 K) 6.6 / 6.0; 128 rows 768 x 192 (72 K) 5.8 / 7.4; 2,048 rows 256 x 64
+// (128 K) 7.8 / 6.8.
+static bool f32_short(int64_t M, int64_t N, int64_t K) {
+    return M > 24 && K <= 256 && ((M + 15) / 16) * ((N + 15) / 16) * K <= 80 * 1024;
+}
+
 void gemm_simt(const Launch& l, const Tensor& a, const Tensor& w, const Tensor* bias, Tensor& out, bool w_out_in, Act act,
                const Tensor* residual) {
     const int64_t M = a.rows, K = a.cols, N = out.cols;
@@ -192,7 +200,8 @@ void gemm_simt(const Launch& l, const Tensor& a, const Tensor& w, const Tensor* 
     // weights whose rows run along k from 16-byte boundaries: the kernels that load four k at a time
     if (w_out_in && a.dtype == DType::F32 && w.dtype == DType::F32 && out.dtype == DType::F32 && K % 4 == 0 && a.ld % 4 == 0 &&
         w.ld % 4 == 0 && !((uintptr_t)a.data & 15) && !((uintptr_t)w.data & 15)) {
-        if (f32_on_tensor_cores(M, N, K)) {
+        const bool brief = f32_short(M, N, K);
+        if (!brief && f32_on_tensor_cores(M, N, K)) {
             static auto split = SANDY_KERNEL(gemm_f32_tc, sandy_gemm_f32_tc);
             check(split((const float*)a.data, (const float*)w.data, bias ? (const float*)bias->data : nullptr,
                         residual ? (const float*)residual->data : nullptr, (float*)out.data, (int)M, (int)N, (int)K, (int)a.ld, (int)w.ld,
@@ -203,7 +212,7 @@ void gemm_simt(const Launch& l, const Tensor& a, const Tensor& w, const Tensor* 
         static auto fast = SANDY_KERNEL(gemm_f32, sandy_gemm_f32);
         check(fast((const float*)a.data, (const float*)w.data, bias ? (const float*)bias->data : nullptr,
                    residual ? (const float*)residual->data : nullptr, (float*)out.data, (int)M, (int)N, (int)K, (int)a.ld, (int)w.ld,
-                   residual ? (int)residual->ld : 0, (int)out.ld, (int)act, 0, 1, l.stream),
+                   residual ? (int)residual->ld : 0, (int)out.ld, (int)act, brief ? 5 : 0, 1, l.stream),
               "gemm_f32(M=" + std::to_string(M) + ",N=" + std::to_string(N) + ",K=" + std::to_string(K) + ")");
         return;
     }

@@ -13,8 +13,11 @@
 // 246, 768 x 3,072 379 -> 240 (44 TFLOP/s of the 74 the fma units could do: with three 64-bit operands a packed fma takes
 // about three cycles of the register file, not two).
 //
-// Two kernels:
+// Three kernels:
 //
+// short    small products with a short k (a tiny model's), where a launch's start and end are all there is: tiles of 16 x 16 whose
+//          whole k is brought at once, the weights' part before the kernel in front has ended; four warps split k.  57 rows, us:
+//          192 x 64 2.5, 64 x 256 3.5 (tiles of 64 x 64 8.6 and 5.3, gemm_f32_tc.cu 5.3 and 5.1).
 // stream   few rows.  What bounds it is the weights' way from memory, so nothing is staged: a warp owns four rows of w and
 //          a part of k, its lanes run along k in float4 steps (512 contiguous bytes of each row), and the first of them
 //          are on their way before the kernel in front has ended (weights are written by no kernel).  Four rows of w
@@ -332,6 +335,68 @@ gemm_f32_tile_kernel(const Product p) {
     cluster.sync();         // nobody leaves while a peer may still read its shared memory
 }
 
+// ---- short k -------------------------------------------------------------------------------------------------
+constexpr int SHORT_TILE = 16, SHORT_WARPS = 4, SHORT_K = 256;
+
+// grid (tiles of N, tiles of M).  A warp takes every fourth piece of four k, a lane 2 x 4 outputs; the warps' sums are added in order.
+__global__ void __launch_bounds__(SHORT_WARPS * 32)
+gemm_f32_short_kernel(const Product p) {
+    extern __shared__ __align__(16) float operands[];
+    __shared__ float sums[SHORT_WARPS][SHORT_TILE][SHORT_TILE + 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n0 = blockIdx.x * SHORT_TILE, m0 = blockIdx.y * SHORT_TILE;
+    const int pieces = p.K / 4, pitch = p.K + 4;            // eight rows one after another start in eight groups of banks
+    float* as = operands;
+    float* ws = operands + SHORT_TILE * pitch;
+    pdl_launch_dependents();
+    auto bring = [&](float* to, const float* from, int ld, int rows) {
+        for (int i = tid; i < SHORT_TILE * pieces; i += SHORT_WARPS * 32) {
+            const int row = i / pieces, at = i % pieces * 4;
+            copy_16((uint32_t)__cvta_generic_to_shared(to + row * pitch + at), from + (size_t)(row < rows ? row : 0) * ld + at, row < rows);
+        }
+    };
+    bring(ws, p.w + (size_t)n0 * p.ldw, p.ldw, p.N - n0);       // weights are written by no kernel
+    pdl_wait();
+    bring(as, p.a + (size_t)m0 * p.lda, p.lda, p.M - m0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const int ty = lane >> 2, tx = lane & 3;
+    float2 acc[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = make_float2(0.0f, 0.0f);
+#pragma unroll 4
+    for (int c = warp; c < pieces; c += SHORT_WARPS) {
+        float4 av[2], wv[4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) av[i] = *reinterpret_cast<const float4*>(as + (ty + 8 * i) * pitch + 4 * c);
+#pragma unroll
+        for (int j = 0; j < 4; j++) wv[j] = *reinterpret_cast<const float4*>(ws + (tx + 4 * j) * pitch + 4 * c);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = __ffma2_rn(high(av[i]), high(wv[j]), __ffma2_rn(low(av[i]), low(wv[j]), acc[i][j]));
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) sums[warp][ty + 8 * i][tx + 4 * j] = acc[i][j].x + acc[i][j].y;
+    __syncthreads();
+    for (int i = tid; i < SHORT_TILE * SHORT_TILE; i += SHORT_WARPS * 32) {
+        const int row = i / SHORT_TILE, col = i % SHORT_TILE;
+        float v = 0.0f;
+#pragma unroll
+        for (int k = 0; k < SHORT_WARPS; k++) v += sums[k][row][col];
+        if (m0 + row < p.M && n0 + col < p.N) write_back(p, m0 + row, n0 + col, v);
+    }
+}
+
+int launch_short(const Product& p, cudaStream_t stream) {
+    const dim3 grid((p.N + SHORT_TILE - 1) / SHORT_TILE, (p.M + SHORT_TILE - 1) / SHORT_TILE);
+    return sandy_launch(gemm_f32_short_kernel, grid, dim3(SHORT_WARPS * 32), (size_t)2 * SHORT_TILE * (p.K + 4) * 4, stream, p);
+}
+
 template <int MB, int AHEAD, int BLOCKS>
 int launch_stream(const Product& p, cudaStream_t stream) {
     // Groups of four rows of w in a block: few enough that there are blocks for every SM; the warps left over share k.
@@ -421,7 +486,7 @@ int choose(int M, int N, int K, int& splits) {
 // a: [M, K] (row stride lda), w: [N, K] (row stride ldw), bias: [N] or null, residual: [M, N] (row stride ldr) or null,
 // out: [M, N] (row stride ldc), which may be the residual itself; all float32, strides in elements.  K, lda and ldw are
 // multiples of 4, a and w start on 16-byte boundaries.  form: 0 the rule's choice; 1 stream; 2, 3, 4 a tile of 128 x 128,
-// 64 x 128, 64 x 64 in `splits` parts of k (1, 2, 4 or 8).
+// 64 x 128, 64 x 64 in `splits` parts of k (1, 2, 4 or 8); 5 short (K up to 256).
 SANDY_API int sandy_gemm_f32(const float* a, const float* w, const float* bias, const float* residual, float* out, int M, int N,
                              int K, int lda, int ldw, int ldr, int ldc, int act, int form, int splits, cudaStream_t stream) {
     if (M == 0 || N == 0) return SANDY_OK;
@@ -431,8 +496,12 @@ SANDY_API int sandy_gemm_f32(const float* a, const float* w, const float* bias, 
     if (form == 0) {
         if (M <= STREAM_MAX_ROWS) form = 1;
         else form = 2 + choose(M, N, K, splits);
-    } else if (form > 1 && (splits < 1 || splits > MAX_SPLITS || (splits & (splits - 1)))) {
+    } else if (form > 1 && form < 5 && (splits < 1 || splits > MAX_SPLITS || (splits & (splits - 1)))) {
         return SANDY_ERR_ARGUMENT;
+    }
+    if (form == 5) {
+        if (K > SHORT_K || (M + SHORT_TILE - 1) / SHORT_TILE > 65535) return SANDY_ERR_UNSUPPORTED;
+        return launch_short(p, stream);
     }
     if (form == 1) {
         if (M == 1) return launch_stream<1, 4, 2>(p, stream);

@@ -177,7 +177,7 @@ def _f32_product(name, a, w, bias, out, residual, act, *last) -> None:
 def gemm_f32(a, w, bias, out, *, act=None, residual=None, form: int = 0, splits: int = 1) -> None:
     """out = act(a @ w.T + bias) + residual, all float32, w [N, K]: K and the row pitches of a and w multiples of 4, both on
     16-byte boundaries.  form 0 lets the kernel choose; 1 streams the weights past a few rows; 2, 3 and 4 are tiles of
-    128 x 128, 64 x 128 and 64 x 64 whose k is split over `splits` (1, 2, 4, 8) blocks."""
+    128 x 128, 64 x 128 and 64 x 64 whose k is split over `splits` (1, 2, 4, 8) blocks; 5 small tiles for a K of up to 256."""
     _f32_product("gemm_f32", a, w, bias, out, residual, act, ctypes.c_int(form), ctypes.c_int(splits))
 
 

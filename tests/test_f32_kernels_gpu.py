@@ -66,6 +66,17 @@ def test_gemm_f32_refuses_what_it_cannot_load():
         ops.gemm_f32(torch.zeros(25, device=DEV)[1:].view(3, 8)[:, :4], w[:, :4].contiguous(), None, out)   # not on 16 bytes
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (15, 17, 20), (16, 16, 64), (57, 192, 64), (33, 50, 252), (130, 65, 256)])
+def test_gemm_f32_short(M, N, K):
+    """Remainders of the 16 x 16 tiles, a k that is no multiple of the four warps' share, the longest one; and that a longer is refused."""
+    from sandyrt_b200.csrc import ops
+
+    test_gemm_f32(M, N, K, 5, 1)
+    test_gemm_f32_infinity_at_the_end_of_a_row(M, N, K, 5, 1)
+    with pytest.raises(ops.UnsupportedShape):
+        ops.gemm_f32(torch.zeros(2, 260, device=DEV), torch.zeros(3, 260, device=DEV), None, torch.zeros(2, 3, device=DEV), form=5)
+
+
 @pytest.mark.parametrize("tile,parts", [(0, 0), (64, 1), (64, 8), (96, 1), (96, 4), (128, 1), (128, 2), (128, 8)])
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (33, 50, 12), (127, 97, 516), (129, 130, 576), (260, 257, 1028)])
 @pytest.mark.parametrize("size", [1.0, 2.0 ** -110, 2.0 ** 100])
