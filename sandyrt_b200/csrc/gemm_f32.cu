@@ -338,7 +338,7 @@ gemm_f32_tile_kernel(const Product p) {
 // ---- short k -------------------------------------------------------------------------------------------------
 constexpr int SHORT_TILE = 16, SHORT_WARPS = 4, SHORT_K = 256;
 
-// grid (tiles of N, tiles of M).  A warp takes every fourth piece of four k, a lane 2 x 4 outputs; the warps' sums are added in order.
+// grid (tiles of N, tiles of M).  A warp takes every fourth piece of four k, a lane 2 x 4 outputs; the warps' sums are added in pairs.
 __global__ void __launch_bounds__(SHORT_WARPS * 32)
 gemm_f32_short_kernel(const Product p) {
     extern __shared__ __align__(16) float operands[];
@@ -385,9 +385,7 @@ gemm_f32_short_kernel(const Product p) {
     __syncthreads();
     for (int i = tid; i < SHORT_TILE * SHORT_TILE; i += SHORT_WARPS * 32) {
         const int row = i / SHORT_TILE, col = i % SHORT_TILE;
-        float v = 0.0f;
-#pragma unroll
-        for (int k = 0; k < SHORT_WARPS; k++) v += sums[k][row][col];
+        const float v = (sums[0][row][col] + sums[1][row][col]) + (sums[2][row][col] + sums[3][row][col]);
         if (m0 + row < p.M && n0 + col < p.N) write_back(p, m0 + row, n0 + col, v);
     }
 }
