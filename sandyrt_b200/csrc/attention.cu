@@ -40,32 +40,35 @@ constexpr int MAX_HEAD_DIM = 256;            // the common instantiation
 constexpr int WIDE_HEAD_DIM = 640;           // the other
 constexpr int WARPS_PER_BLOCK = 4;
 
-template <typename T>
+// WIDE: everything starts on 16 bytes and moves in pieces of 16 (2,048 tokens of 12 heads of 64 in float: 7.0 us element by element,
+// 6.1 so; 8 tokens 3.1 -> 2.6).
+template <typename T, bool WIDE>
 __global__ void kv_append_kernel(const T* __restrict__ k_src, const T* __restrict__ v_src, int ld_src,
                                  T* __restrict__ k_cache, T* __restrict__ v_cache, long long page_stride,
                                  const int* __restrict__ block_table, int max_blocks,
                                  const int* __restrict__ token_seq, const int* __restrict__ positions,
                                  int n_kv_heads, int head_dim, int page_size, int num_pages,
                                  int* __restrict__ status) {
+    pdl_launch_dependents();
     const int t = blockIdx.x;
     const int s = token_seq[t];
     const int pos = positions[t];
-    if (pos < 0 || pos / page_size >= max_blocks) {   // a position the block table does not cover
-        if (threadIdx.x == 0 && status) atomicOr(status, 8);
-        return;
-    }
-    const int page = block_table[(size_t)s * max_blocks + pos / page_size];
+    const bool covered = pos >= 0 && pos / page_size < max_blocks;         // by the block table
+    const int page = covered ? block_table[(size_t)s * max_blocks + pos / page_size] : -1;
+    pdl_wait();
     if (page < 0 || page >= num_pages) {              // no page behind this position: nothing may be written
         if (threadIdx.x == 0 && status) atomicOr(status, 8);
         return;
     }
     const int slot = pos % page_size;
-    const int n = n_kv_heads * head_dim;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int h = i / head_dim, d = i % head_dim;
-        const size_t dst = (size_t)page * page_stride + ((size_t)h * page_size + slot) * head_dim + d;
-        k_cache[dst] = k_src[(size_t)t * ld_src + i];
-        v_cache[dst] = v_src[(size_t)t * ld_src + i];
+    constexpr int VEC = WIDE ? 16 / (int)sizeof(T) : 1;
+    const int n = n_kv_heads * head_dim / VEC, per_head = head_dim / VEC;
+    for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) {
+        const int at = i < n ? i : i - n, h = at / per_head, d = at % per_head * VEC;
+        T* dst = (i < n ? k_cache : v_cache) + (size_t)page * page_stride + ((size_t)h * page_size + slot) * head_dim + d;
+        const T* src = (i < n ? k_src : v_src) + (size_t)t * ld_src + (size_t)at * VEC;
+        if (WIDE) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+        else *dst = *src;
     }
 }
 
@@ -116,11 +119,13 @@ paged_attention_kernel(const T* __restrict__ q, int ld_q,
     __shared__ float q_smem[WARPS_PER_BLOCK][MAX_D];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long pair = (long long)blockIdx.x * WARPS_PER_BLOCK + warp;
+    pdl_launch_dependents();
     if (pair >= (long long)n_tokens * n_heads) return;
     const int t = (int)(pair / n_heads), h = (int)(pair % n_heads);
     const int s = token_seq[t];
     const int pos = positions[t];
     const int kvh = h / (n_heads / n_kv_heads);
+    pdl_wait();
     const VisibleKeys seen = visible_keys(pos, window, keep_first, chunk);
     const int* table = block_table + (size_t)s * max_blocks;
     const long long rows_per_page = page_stride / head_dim;  // page stride in rows of D
@@ -197,17 +202,19 @@ SANDY_API int sandy_kv_append(const void* k_src, const void* v_src, int ld_src,
         return SANDY_ERR_ARGUMENT;
     const int n = n_kv_heads * head_dim;
     const int threads = n >= 512 ? 256 : 128;
-    if (dtype == SANDY_F32)
-        kv_append_kernel<float><<<n_tokens, threads, 0, stream>>>(
-            (const float*)k_src, (const float*)v_src, ld_src, (float*)k_cache, (float*)v_cache, page_stride,
-            block_table, max_blocks, token_seq, positions, n_kv_heads, head_dim, page_size, num_pages, status);
-    else if (dtype == SANDY_BF16)
-        kv_append_kernel<bf16><<<n_tokens, threads, 0, stream>>>(
-            (const bf16*)k_src, (const bf16*)v_src, ld_src, (bf16*)k_cache, (bf16*)v_cache, page_stride,
-            block_table, max_blocks, token_seq, positions, n_kv_heads, head_dim, page_size, num_pages, status);
-    else
-        return SANDY_ERR_UNSUPPORTED;
-    return sandy_launch_status();
+#define APPEND(T)                                                                                                               \
+    do {                                                                                                                        \
+        const size_t any = (uintptr_t)k_src | (uintptr_t)v_src | (uintptr_t)k_cache | (uintptr_t)v_cache |                      \
+                           ((size_t)ld_src * sizeof(T)) | ((size_t)page_stride * sizeof(T)) | ((size_t)head_dim * sizeof(T));   \
+        return sandy_launch(any % 16 == 0 ? kv_append_kernel<T, true> : kv_append_kernel<T, false>, dim3(n_tokens),             \
+                            dim3(threads), 0, stream, (const T*)k_src, (const T*)v_src, ld_src, (T*)k_cache, (T*)v_cache,       \
+                            page_stride, block_table, max_blocks, token_seq, positions, n_kv_heads, head_dim, page_size,        \
+                            num_pages, status);                                                                                 \
+    } while (0)
+    if (dtype == SANDY_F32) APPEND(float);
+    if (dtype == SANDY_BF16) APPEND(bf16);
+#undef APPEND
+    return SANDY_ERR_UNSUPPORTED;
 }
 
 // q: [n_tokens, H*D] with row stride ld_q; out: [n_tokens, H*D] with row stride ld_out.
@@ -238,17 +245,17 @@ SANDY_API int sandy_paged_attention_rules(const void* q, int ld_q, const void* k
     if (page_stride % head_dim != 0 || softcap < 0.0f || chunk < 0) return SANDY_ERR_UNSUPPORTED;
     const long long pairs = (long long)n_tokens * n_heads;
     const unsigned blocks = (unsigned)((pairs + WARPS_PER_BLOCK - 1) / WARPS_PER_BLOCK);
-#define LAUNCH(T)                                                                                     \
-    (head_dim <= MAX_HEAD_DIM ? paged_attention_kernel<T, MAX_HEAD_DIM> : paged_attention_kernel<T, WIDE_HEAD_DIM>)<<<blocks, WARPS_PER_BLOCK * 32, 0, stream>>>( \
-        (const T*)q, ld_q, (const T*)k_cache, (const T*)v_cache, page_stride, block_table, max_blocks, \
-        token_seq, positions, (T*)out, ld_out, n_tokens, n_heads, n_kv_heads, head_dim, page_size,    \
-        scale, window, softcap, chunk, num_pages, sink, out_gate, dist_bias, n_dist, rules->keep_first,   \
-        (const T*)rules->elem_gate, rules->ld_elem_gate, rules->gate_dim, status)
+#define LAUNCH(T)                                                                                                               \
+    return sandy_launch(head_dim <= MAX_HEAD_DIM ? paged_attention_kernel<T, MAX_HEAD_DIM> : paged_attention_kernel<T, WIDE_HEAD_DIM>, \
+                        dim3(blocks), dim3(WARPS_PER_BLOCK * 32), 0, stream, (const T*)q, ld_q, (const T*)k_cache,              \
+                        (const T*)v_cache, page_stride, block_table, max_blocks, token_seq, positions, (T*)out, ld_out,         \
+                        n_tokens, n_heads, n_kv_heads, head_dim, page_size, scale, window, softcap, chunk, num_pages, sink,     \
+                        out_gate, dist_bias, n_dist, rules->keep_first, (const T*)rules->elem_gate, rules->ld_elem_gate,        \
+                        rules->gate_dim, status)
     if (dtype == SANDY_F32) LAUNCH(float);
-    else if (dtype == SANDY_BF16) LAUNCH(bf16);
-    else return SANDY_ERR_UNSUPPORTED;
+    if (dtype == SANDY_BF16) LAUNCH(bf16);
 #undef LAUNCH
-    return sandy_launch_status();
+    return SANDY_ERR_UNSUPPORTED;
 }
 
 // The same without kept first keys or a gate by element.

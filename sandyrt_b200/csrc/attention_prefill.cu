@@ -106,7 +106,9 @@ prefill_attention_kernel(const bf16* __restrict__ q, int ld_q, const bf16* __res
     const int qs = q_start[s];
     const int q_len = q_start[s + 1] - qs;
     const int n_tiles = (q_len + BM - 1) / BM;
+    pdl_launch_dependents();
     if ((int)blockIdx.x >= n_tiles) return;
+    pdl_wait();
     const int tile = n_tiles - 1 - blockIdx.x;         // the tiles with the most keys start first
     const int t0 = tile * BM;
     const int rows_valid = min(BM, q_len - t0);
@@ -403,11 +405,10 @@ int launch(const void* q, int ld_q, const void* k_cache, const void* v_cache, lo
         configured = true;
     }
     dim3 grid((max_q_len + BM - 1) / BM, n_heads, n_seqs);
-    prefill_attention_kernel<D><<<grid, THREADS, smem, stream>>>(
-        (const bf16*)q, ld_q, (const bf16*)k_cache, (const bf16*)v_cache, page_stride, block_table, max_blocks, q_start,
+    return sandy_launch(
+        prefill_attention_kernel<D>, grid, dim3(THREADS), (size_t)smem, stream, (const bf16*)q, ld_q, (const bf16*)k_cache, (const bf16*)v_cache, page_stride, block_table, max_blocks, q_start,
         kv_before, (bf16*)out, ld_out, n_heads, n_kv_heads, page_size, scale, r.window, r.softcap, r.chunk, num_pages, r.sink,
         r.out_gate, r.dist_bias, r.n_dist, r.keep_first, (const bf16*)r.elem_gate, r.ld_elem_gate, r.gate_dim, status);
-    return sandy_launch_status();
 }
 
 }  // namespace

@@ -28,6 +28,67 @@ __device__ __forceinline__ float act_of(float z, int act) {
     return z;
 }
 
+// Where rows and their pitches are whole pieces of 16 bytes, a block takes a run of pieces of one row (blockIdx.x the row): one load an
+// operand, no division (element by element with two 64-bit divisions each, 2,048 x 2,048 in bfloat16 took 17.6 us, 6.5 so).
+template <typename T>
+struct Piece {
+    static constexpr int N = 16 / (int)sizeof(T);
+    float v[N];
+    __device__ __forceinline__ void load(const T* p) {
+        uint4 raw = *reinterpret_cast<const uint4*>(p);
+        const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+        for (int i = 0; i < N; i++) v[i] = to_f32(e[i]);
+    }
+    __device__ __forceinline__ void store(T* p) const {
+        uint4 raw;
+        T* e = reinterpret_cast<T*>(&raw);
+#pragma unroll
+        for (int i = 0; i < N; i++) e[i] = from_f32<T>(v[i]);
+        *reinterpret_cast<uint4*>(p) = raw;
+    }
+};
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+glu_pieces_kernel(const T* __restrict__ a, const T* __restrict__ b, int ld_in, T* __restrict__ out, int ld_out, int cols, int act) {
+    const int j = (blockIdx.y * blockDim.x + threadIdx.x) * Piece<T>::N;
+    pdl_launch_dependents();
+    pdl_wait();
+    if (j >= cols) return;
+    const size_t in = (size_t)blockIdx.x * ld_in + j;
+    Piece<T> g, u;
+    g.load(a + in);
+    u.load(b + in);
+#pragma unroll
+    for (int i = 0; i < Piece<T>::N; i++) g.v[i] = act_of(g.v[i], act) * u.v[i];
+    g.store(out + (size_t)blockIdx.x * ld_out + j);
+}
+
+__global__ void __launch_bounds__(256)
+scale_add_pieces_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ gain, const float* __restrict__ y2, int ldy2,
+                        const float* __restrict__ gain2, float* __restrict__ x, int ldx, int cols) {
+    const int j = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    pdl_launch_dependents();
+    Piece<float> g, g2, v, w, to;
+    if (j < cols) {                             // weights are written by no kernel
+        g.load(gain + j);
+        if (y2) g2.load(gain2 + j);
+    }
+    pdl_wait();
+    if (j >= cols) return;
+    v.load(y + (size_t)blockIdx.x * ldy + j);
+    if (y2) w.load(y2 + (size_t)blockIdx.x * ldy2 + j);
+    to.load(x + (size_t)blockIdx.x * ldx + j);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float branch = g.v[i] * v.v[i];
+        if (y2) branch += g2.v[i] * w.v[i];
+        to.v[i] += branch;
+    }
+    to.store(x + (size_t)blockIdx.x * ldx + j);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 glu_kernel(const T* __restrict__ a, const T* __restrict__ b, int ld_in, T* __restrict__ out, int ld_out, int rows, int cols,
@@ -111,6 +172,11 @@ __global__ void __launch_bounds__(256) scale_f32_kernel(float* __restrict__ x, l
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) x[i] *= s;
 }
 
+// A block's threads and the grid for rows of `pieces` pieces of 16 bytes; up to 65,535 blocks along a row.
+inline int row_threads(int pieces) { return pieces >= 256 ? 256 : (pieces + 31) / 32 * 32; }
+inline dim3 row_grid(int rows, int pieces) { return dim3(rows, (pieces + row_threads(pieces) - 1) / row_threads(pieces)); }
+inline bool in_pieces(size_t bytes_or_addresses) { return bytes_or_addresses % 16 == 0; }
+
 inline unsigned blocks_for(long long n) {
     const long long want = (n + 255) / 256;
     const long long cap = (long long)sandy_sm_count() * 16;
@@ -139,6 +205,19 @@ SANDY_API int sandy_glu(const void* a, const void* b, int ld_in, void* out, int 
                         cudaStream_t stream) {
     if (rows == 0 || cols == 0) return SANDY_OK;
     if (!a || !b || !out) return SANDY_ERR_ARGUMENT;
+    const size_t size = dtype == SANDY_F32 ? 4 : 2;
+    if ((dtype == SANDY_F32 || dtype == SANDY_BF16) &&
+        in_pieces((uintptr_t)a | (uintptr_t)b | (uintptr_t)out | (size_t)ld_in * size | (size_t)ld_out * size | (size_t)cols * size)) {
+        const int pieces = (int)(cols * size / 16), threads = row_threads(pieces);
+        const dim3 wide = row_grid(rows, pieces);
+        if (wide.y <= 65535) {
+            if (dtype == SANDY_F32)
+                return sandy_launch(glu_pieces_kernel<float>, wide, dim3(threads), 0, stream, (const float*)a, (const float*)b, ld_in,
+                                    (float*)out, ld_out, cols, act);
+            return sandy_launch(glu_pieces_kernel<bf16>, wide, dim3(threads), 0, stream, (const bf16*)a, (const bf16*)b, ld_in, (bf16*)out,
+                                ld_out, cols, act);
+        }
+    }
     const unsigned grid = blocks_for((long long)rows * cols);
     if (dtype == SANDY_F32)
         return sandy_launch(glu_kernel<float>, dim3(grid), dim3(256), 0, stream, (const float*)a, (const float*)b, ld_in,
@@ -169,6 +248,10 @@ SANDY_API int sandy_scale_add(const float* y, int ldy, const float* gain, const 
                               int ldx, int rows, int cols, cudaStream_t stream) {
     if (rows == 0 || cols == 0) return SANDY_OK;
     if (!y || !gain || !x || (y2 && !gain2)) return SANDY_ERR_ARGUMENT;
+    if (in_pieces((uintptr_t)y | (uintptr_t)gain | (uintptr_t)y2 | (uintptr_t)gain2 | (uintptr_t)x | (size_t)ldy * 4 | (size_t)(y2 ? ldy2 : 0) * 4 |
+                  (size_t)ldx * 4 | (size_t)cols * 4) && row_grid(rows, cols / 4).y <= 65535)
+        return sandy_launch(scale_add_pieces_kernel, row_grid(rows, cols / 4), dim3(row_threads(cols / 4)), 0, stream, y, ldy, gain, y2, ldy2,
+                            gain2, x, ldx, cols);
     return sandy_launch(scale_add_kernel, dim3(blocks_for((long long)rows * cols)), dim3(256), 0, stream, y, ldy, gain, y2, ldy2,
                         gain2, x, ldx, rows, cols);
 }

@@ -37,42 +37,77 @@ __device__ __forceinline__ float act_gate(float z, int act) {
     return act == 1 ? z * s : s;       // 1: silu, otherwise sigmoid
 }
 
-// mode 0: out = norm(x[rows]) (TO);  mode 1: xio += mult * norm(x) (float)
-template <typename TO, int NV, int MODE>
+// Four consecutive elements with one access.
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+    const uint2 t = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&t.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&t.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void store4(float* p, const float4& v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(bf16* p, const float4& v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
+// mode 0: out = norm(x[rows]) (TO);  mode 1: xio += mult * norm(x) (float).  VEC: elements a lane takes at a time, 4 where the width and
+// every pitch are multiples of 4 and the rows aligned (2,048 rows of 768, added to the stream: 4.7 us -> 3.0).  NV: rounds of 32 * VEC.
+template <typename TO, int NV, int MODE, int VEC>
 __global__ void __launch_bounds__(ROWS_PER_BLOCK * 32)
 rmsnorm_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ gain, TO* __restrict__ out, int ldo,
                const int* __restrict__ rows, int n_rows, int width, float eps, float mult) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = blockIdx.x * ROWS_PER_BLOCK + warp;
     // the gain is a weight, which no kernel writes: asked for before the wait for the kernel that produces x
-    float g[NV];
+    float g[NV][VEC];
 #pragma unroll
     for (int i = 0; i < NV; i++) {
-        const int e = i * 32 + lane;
-        g[i] = (gain && e < width) ? gain[e] : 1.0f;
+        const int e = (i * 32 + lane) * VEC;
+        if constexpr (VEC == 4) {
+            const float4 t = gain && e < width ? load4(gain + e) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+            g[i][0] = t.x; g[i][1] = t.y; g[i][2] = t.z; g[i][3] = t.w;
+        } else {
+            g[i][0] = (gain && e < width) ? gain[e] : 1.0f;
+        }
     }
     pdl_wait();
     pdl_launch_dependents();
     if (r >= n_rows) return;
     const float* row = x + (size_t)(rows ? rows[r] : r) * ldx;
-    float v[NV];
+    TO* orow = out + (size_t)r * ldo;
+    float v[NV][VEC], old[MODE == 1 ? NV : 1][VEC];
     float ss = 0.0f;
 #pragma unroll
     for (int i = 0; i < NV; i++) {
-        const int e = i * 32 + lane;
-        v[i] = e < width ? row[e] : 0.0f;
-        ss = fmaf(v[i], v[i], ss);
+        const int e = (i * 32 + lane) * VEC;
+        if constexpr (VEC == 4) {
+            const float4 t = e < width ? load4(row + e) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            v[i][0] = t.x; v[i][1] = t.y; v[i][2] = t.z; v[i][3] = t.w;
+            if (MODE == 1 && e < width) {
+                const float4 u = load4(orow + e);
+                old[i][0] = u.x; old[i][1] = u.y; old[i][2] = u.z; old[i][3] = u.w;
+            }
+        } else {
+            v[i][0] = e < width ? row[e] : 0.0f;
+            if (MODE == 1 && e < width) old[i][0] = to_f32(orow[e]);
+        }
+#pragma unroll
+        for (int j = 0; j < VEC; j++) ss = fmaf(v[i][j], v[i][j], ss);
     }
     ss = warp_sum(ss);
     const float inv = 1.0f / sqrtf(ss / (float)width + eps);
-    TO* orow = out + (size_t)r * ldo;
 #pragma unroll
     for (int i = 0; i < NV; i++) {
-        const int e = i * 32 + lane;
+        const int e = (i * 32 + lane) * VEC;
         if (e < width) {
-            const float y = v[i] * inv * g[i];
-            if (MODE == 0) orow[e] = from_f32<TO>(y);
-            else orow[e] = from_f32<TO>(to_f32(orow[e]) + mult * y);
+            float y[VEC];
+#pragma unroll
+            for (int j = 0; j < VEC; j++) {
+                y[j] = v[i][j] * inv * g[i][j];
+                if (MODE == 1) y[j] = old[i][j] + mult * y[j];
+            }
+            if constexpr (VEC == 4) store4(orow + e, make_float4(y[0], y[1], y[2], y[3]));
+            else orow[e] = from_f32<TO>(y[0]);
         }
     }
 }
@@ -103,9 +138,18 @@ template <typename TO, int MODE>
 int launch(const float* x, int ldx, const float* gain, TO* out, int ldo, const int* rows, int n_rows, int width, float eps,
            float mult, cudaStream_t stream) {
     const dim3 grid((n_rows + ROWS_PER_BLOCK - 1) / ROWS_PER_BLOCK), block(ROWS_PER_BLOCK * 32);
+    const size_t any = (uintptr_t)x | (uintptr_t)gain | (uintptr_t)out * (16 / (4 * sizeof(TO)));
+    if (any % 16 == 0 && width % 4 == 0 && ldx % 4 == 0 && ldo % 4 == 0) {
+#define CASE(NV)                                                                                                        \
+    if (width <= 128 * NV)                                                                                              \
+        return sandy_launch(rmsnorm_kernel<TO, NV, MODE, 4>, grid, block, 0, stream, x, ldx, gain, out, ldo, rows, n_rows, \
+                            width, eps, mult)
+        CASE(1); CASE(2); CASE(4); CASE(6); CASE(8);
+#undef CASE
+    }
 #define CASE(NV)                                                                                                        \
     if (width <= 32 * NV)                                                                                               \
-        return sandy_launch(rmsnorm_kernel<TO, NV, MODE>, grid, block, 0, stream, x, ldx, gain, out, ldo, rows, n_rows, \
+        return sandy_launch(rmsnorm_kernel<TO, NV, MODE, 1>, grid, block, 0, stream, x, ldx, gain, out, ldo, rows, n_rows, \
                             width, eps, mult)
     CASE(2); CASE(4); CASE(8); CASE(12); CASE(16); CASE(24); CASE(MAX_ROUNDS);
 #undef CASE

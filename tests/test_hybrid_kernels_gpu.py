@@ -107,6 +107,32 @@ def test_prompt_kernels_with_sink_and_gate(H, Hkv, D, page_size, tc):
     assert (out.double().cpu() - _want(case, H, Hkv, scale, sink, gate)).abs().max().item() < ATT_TOL[torch.bfloat16] * 1.5
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("cols", [8, 248, 2056])
+def test_passes_in_pieces_and_element_by_element(dtype, cols):
+    """Rows that are whole pieces of 16 bytes, and the same one element further on: the same formula element by element."""
+    from sandyrt_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(cols)
+    rows, wide = 5, 2 * cols + 8
+    a = torch.randn(rows, wide, generator=g).to(dtype).to(DEV)
+    odd = torch.zeros(rows, wide + 1, dtype=dtype, device=DEV)
+    odd[:, 1:] = a
+    outs = [torch.empty(rows, cols, dtype=dtype, device=DEV) for _ in range(2)]
+    for x, out in zip((a, odd[:, 1:]), outs):
+        ops.glu(x[:, :cols], x[:, cols:2 * cols], out)
+    want = torch.nn.functional.silu(a[:, :cols].double()) * a[:, cols:2 * cols].double()
+    assert torch.equal(outs[0], outs[1])
+    assert (outs[0].double() - want).abs().max().item() <= (2e-6 if dtype == torch.float32 else 2.0 ** -8) * want.abs().max().item()
+    if dtype == torch.float32:
+        x, y, y2 = (torch.randn(rows, cols + 1, generator=g).to(DEV) for _ in range(3))
+        gain, gain2 = torch.randn(cols + 1, generator=g).to(DEV), torch.randn(cols + 1, generator=g).to(DEV)
+        even = [t[..., 1:].contiguous() for t in (x, y, y2, gain, gain2)]
+        ops.scale_add(even[1], even[3], even[0], even[2], even[4])
+        want = x[:, 1:] + (gain[1:] * y[:, 1:] + gain2[1:] * y2[:, 1:])
+        assert torch.allclose(even[0], want, rtol=1e-5, atol=1e-5)
+
+
 @pytest.mark.parametrize("width", [48, 100, 256, 777, 1600, 5000])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 def test_rmsnorm_and_its_residual_form(width, out_dtype):
