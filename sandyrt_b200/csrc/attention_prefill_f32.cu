@@ -1,7 +1,7 @@
-// Causal attention of prompt portions in float32, heads of up to 128, on the 32-bit pipes: heads up to 32, and steps of very many single
-// tokens that the decode kernel has no form for (attention_prefill_f32_tc.cu takes the others).  A tile of queries of one head against tiles of keys, every
-// product and sum on the 32-bit pipes.  The formula, the cache layout and the rules are those of the general kernel
-// (attention.cu), which gives a warp one (token, head) pair and so reads every key once per query: 2 TFLOP/s.
+// Causal attention of prompt portions in float32, heads of up to 128, on the 32-bit pipes: heads up to 32, and steps of very many
+// single tokens that the decode kernel has no form for (attention_prefill_f32_tc.cu takes the others).  A tile of queries of one head
+// against tiles of keys, every product and sum on the 32-bit pipes.  The formula, the cache layout and the rules are those of the
+// general kernel (attention.cu), which gives a warp one (token, head) pair and so reads every key once per query: 2 TFLOP/s.
 //
 // What bounds it is the fma rate.  A block of four warps takes 64 queries of one head and walks the keys they see 64 at a time,
 // with an online softmax.  A warp owns 16 queries (its rows of the scores and of the output never leave it), a thread 8

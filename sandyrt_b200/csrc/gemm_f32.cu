@@ -23,8 +23,9 @@
 //          are on their way before the kernel in front has ended (weights are written by no kernel).  Four rows of w
 //          share each load of a.  The sums cross the lanes in a halving exchange (31 shuffles for 32 sums), then the
 //          warps that share a row in shared memory.
-// tile     more rows, where the tensor cores (gemm_f32_tc.cu) do not pay.  Tiles of 32*WM x 8*TN*WN outputs behind a ring of cp.async stages of 32 k; 8 x TN outputs a thread.
-//          Where the tiles are too few for the SMs, the blocks of a cluster split k and add up through shared memory.
+// tile     up to 64 rows of narrow products, where the tensor cores (gemm_f32_tc.cu) do not pay.  Tiles of 32*WM x 8*TN*WN outputs
+//          behind a ring of cp.async stages of 32 k; 8 x TN outputs a thread.  Where the tiles are too few for the SMs, the blocks
+//          of a cluster split k and add up through shared memory.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -225,7 +225,7 @@ def grouped(a) -> int:
 
 
 def gemm_f32(a) -> int:
-    """The float32 product beside the general kernel, on distinct weights that together exceed L2."""
+    """The float32 product on the fma units and on the tensor cores beside the general kernel, on distinct weights that together exceed L2."""
     dev = torch.device("cuda:0")
     for M in a.rows:
         for shape in a.shape:
@@ -233,9 +233,10 @@ def gemm_f32(a) -> int:
             x, out = torch.randn(M, K, device=dev), torch.empty(M, N, device=dev)
             ws = [torch.randn(N, K, device=dev) for _ in range(max(1, min(24, 300_000_000 // (4 * N * K))))]
             us = [_time_graph(lambda l: ops.gemm_f32(x, ws[l], None, out), len(ws)),
-                  _time_graph(lambda l: ops.gemm_simt(x, ws[l], None, out, w_out_in=True), len(ws))]
+                  _time_graph(lambda l: ops.gemm_simt(x, ws[l], None, out, w_out_in=True), len(ws)),
+                  _time_graph(lambda l: ops.gemm_f32_tc(x, ws[l], None, out), len(ws))]
             print(f"{M:5d} rows {N:6d} x {K:5d}: {us[0]:8.1f} us  {4e-3 * N * K / us[0]:6.0f} GB/s  {2e-6 * M * N * K / us[0]:5.1f} TFLOP/s"
-                  f"   general kernel {us[1]:8.1f} us", flush=True)
+                  f"   general kernel {us[1]:8.1f} us   tensor cores {us[2]:8.1f} us", flush=True)
     return 0
 
 
@@ -259,7 +260,7 @@ def _cache(dev, H, D, ps, seqs, dtype):
 
 
 def attention_f32(a) -> int:
-    """Prompt portions in float32: the general kernel and the prompt kernel."""
+    """Prompt portions in float32: the general kernel and the prompt kernels on the fma units and on the tensor cores."""
     for shape in a.shape:
         reqs, rest = shape.split("x")
         new, cached = (int(v) for v in rest.split("+"))
@@ -267,7 +268,11 @@ def attention_f32(a) -> int:
         out, kw = torch.empty_like(q), dict(n_heads=a.heads, scale=a.head_dim ** -0.5)
         general = _time_graph(lambda l: ops.paged_attention(q, kc, vc, table, seq, pos, out, **kw), 10)
         tiles = _time_graph(lambda l: ops.prefill_attention_f32(q, kc, vc, table, start, before, out, max_q_len=new, **kw), 10)
-        print(f"{a.heads} heads of {a.head_dim}, {shape:>10}: general {general:8.1f} us  prompt kernel {tiles:8.1f} us", flush=True)
+        line = f"{a.heads} heads of {a.head_dim}, {shape:>10}: general {general:8.1f} us  prompt kernel {tiles:8.1f} us"
+        if a.head_dim > 32:
+            tc = _time_graph(lambda l: ops.prefill_attention_f32(q, kc, vc, table, start, before, out, max_q_len=new, tc=True, **kw), 10)
+            line += f"  tensor cores {tc:8.1f} us"
+        print(line, flush=True)
     return 0
 
 
