@@ -541,10 +541,6 @@ constexpr int kClusterMaxSplits = 8;
 // but a whole decode step of 8 x 12 pairs (its cache fits in L2) took 414 against 400 us and one of
 // 1 x 12 pairs 356 against 333 us, the register kernel starting sooner.
 constexpr int kBulkMinPairs = 256;
-// Up to here the bulk kernel keeps the bfloat16 launches of heads of 64 with one split.  Decode steps of 4 layers, us, bulk / mma.sync:
-// 64 x 12 pairs of 384 keys 324 / 334, of 700 375 / 391 (of 64 to 448 keys 327 / 312), 32 x 25 of 384 369 / 379; 64 x 16 of 384 397 /
-// 373, 64 x 25 503 / 491, 40 x 25 of 600 to 700 477 / 442.
-constexpr int kBulkMaxPairs = 900;
 
 bool decode_head_dim(DType dt, int d) {
     if (d == 16 || d == 32 || d == 64 || d == 128) return true;
@@ -689,7 +685,7 @@ void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const K
         // 8 tokens of 1,000 keys 12.9 / 12.5 / 7.8.  So it takes every launch but those with so many pairs that
         // a pair is one block (one split), where the bulk kernel's deeper ring of pages keeps its small lead.
         static const int mma_mode = env_int("SANDYRT_DECODE_MMA", 1);          // 0 keeps the two kernels below, for comparisons
-        if (q.dtype == DType::BF16 && d == 64 && (gated || (mma_mode != 0 && !(bulk && splits == 1 && T * n_heads <= kBulkMaxPairs)))) {
+        if (q.dtype == DType::BF16 && d == 64 && (gated || (mma_mode != 0 && !(bulk && splits == 1)))) {
             static auto max_keys_fn = SANDY_KERNEL(attention_decode_mma, sandy_decode_attention_mma_max_keys);
             if (max_kv <= max_keys_fn(splits, c.page_size)) {
                 static auto fn = SANDY_KERNEL(attention_decode_mma, sandy_decode_attention_mma_rules);

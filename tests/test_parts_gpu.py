@@ -417,6 +417,28 @@ def _rotary_plain_logits(w, ids, E, H, base, rnd):
     return rnd(ln(x, "nf")) @ rnd(w["emb"]).T
 
 
+def test_decode_attention_of_very_many_pairs_keeps_its_weights_in_32_bits():
+    """1,024 and 512 (token, head) pairs of up to 256 keys are a pair a block on the bulk kernel, whose softmax weights are float; the
+    mma.sync kernel rounds them to 16 bits."""
+    from sandyrt_b200 import core
+
+    spec = _spec("causal_attention", {"width": 64, "n_heads": 16, "n_kv_heads": 16, "head_dim": 64, "scale": 0.125, "window": None,
+                                      "weight_layout": "out_in"}, ["qkv.weight", "qkv.bias", "out.weight", "out.bias"])
+    for n in (64, 32):
+        part = _harness("mixer", spec, torch.bfloat16, seed=4, page_size=16, max_tokens=64 * 48, max_requests=64)
+        h = torch.randn(30 * n, 64, device=DEV).bfloat16()
+        x = torch.zeros(30 * n, 64, device=DEV)
+        part.set_step([(0, 30)] * n)
+        part.run_mixer(h, x)
+        core.call("global", None, "profile_kernels", enable=True)
+        try:
+            part.set_step([(30, 1)] * n)
+            part.run_mixer(h[:n].contiguous(), x)
+        finally:
+            classes = {row["class"] for row in core.call("global", None, "profile_kernels", enable=False)}
+        assert [c for c in classes if c.startswith("attention")] == ["attention, decode (bulk copies)"], classes
+
+
 @pytest.mark.parametrize("dtype,atol,rtol", [("float32", 3e-5, 1e-4), ("bfloat16", 6e-3, 2e-2)])
 def test_position_encoding_that_rotates_queries_and_keys(tmp_path, dtype, atol, rtol):
     from sandyrt_b200.engine.step import Engine, StepEntry
