@@ -275,7 +275,8 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
         __syncwarp();
         asm volatile("bar.sync %0, 128;" ::"r"(1 + (warp & 3)) : "memory");        // the four warps of these rows
     };
-    // m: the row's maximum times log2(e), rounded once, so that a row's exponentials and corrections all refer to the same number
+    // m: the row's maximum.  It is taken from a score before the product with log2(e): of scores of 2^31 and more that product alone is
+    // off by more than an exponential's range.
     float m = -INFINITY, l = 0.0f, corr = 0.0f;     // l: of this thread's keys alone, until the end
     float o[F::COLS];
 #pragma unroll
@@ -382,15 +383,15 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
         part_of[t & 1][part][row] = top;
         meet();
         const float(&tops)[SHARE][BM] = part_of[t & 1];
-        top = fmaxf(fmaxf(tops[0][row], tops[1][row]), fmaxf(tops[2][row], tops[3][row])) * LOG2E;
+        top = fmaxf(fmaxf(tops[0][row], tops[1][row]), fmaxf(tops[2][row], tops[3][row]));
         if (t > 0) add_sum(t - 1);
         const float m_new = fmaxf(m, top), base = m_new == -INFINITY ? 0.0f : m_new;
-        corr = exp2_of(m - base);
+        corr = exp2_of((m - base) * LOG2E);
         m = m_new;
         float sum = 0.0f;
 #pragma unroll
         for (int j = 0; j < MINE; j++) {
-            s[j] = exp2_of(fmaf(s[j], LOG2E, -base));       // (a score that is NaN stays one)
+            s[j] = exp2_of((s[j] - base) * LOG2E);          // (a score that is NaN stays one)
             sum += s[j];
         }
         l = l * corr + sum;
@@ -420,7 +421,7 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
     const float(&ls)[SHARE][BM] = part_of[tiles & 1];
     l = (ls[0][row] + ls[1][row]) + (ls[2][row] + ls[3][row]);
     const int token = t0 + row;
-    const float den = r.sink ? l + exp2f(fmaf(r.sink[head], LOG2E, -m)) : l;
+    const float den = r.sink ? l + expf(r.sink[head] - m) : l;
     const float gate = r.out_gate ? r.out_gate[(size_t)token * p.n_heads + head] : 1.0f;
     float* out = p.out + (size_t)token * p.ld_out + head * d + part * F::COLS;
 #pragma unroll

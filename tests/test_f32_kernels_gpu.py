@@ -282,6 +282,48 @@ def test_prompt_attention_f32_sizes_on_tensor_cores(on_tensor_cores, D, size):
     assert (got - want).abs().max().item() < 2e-5 * size        # the bound of test_prompt_attention_f32
 
 
+def _keys_of(case):
+    """(request, its context's pages and slots) of a _paged_case."""
+    for s, (before, n) in enumerate(case["seqs"]):
+        at = torch.arange(before + n, device=DEV)
+        yield s, case["table"][s, at // 16].long(), at % 16
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("top", [1e8, 3e9, -3e9, 1e10, -1e30])
+def test_large_scores_on_tensor_cores(on_tensor_cores, D, top):
+    """Scores so far apart that a row is the value of its largest one: its weight is exactly 1, and 24 bits of the value are kept."""
+    case = _paged_case(torch.float32, 2, 2, D, 16, [(0, 150), (90, 70)], seed=D)
+    g = torch.Generator().manual_seed(D)
+    case["q"].fill_(1.0)
+    best = []
+    for s, pages, slots in _keys_of(case):
+        before, n = case["seqs"][s]
+        size = 1.0 + torch.randperm(before + n, generator=g).to(DEV) / (before + n)         # at least a 300th apart
+        case["kc"][pages, :, slots] = size[:, None, None]
+        best += [case["vc"][pages, :, slots][(size * np.sign(top))[:before + i + 1].argmax()].reshape(-1) for i in range(n)]
+    got, general = _both(case, 2, {"scale": top / D})
+    want = torch.stack(best)
+    assert (got - want).abs().max().item() <= 2.0 ** -22 * want.abs().max().item()
+    assert (general - want).abs().max().item() <= 2.0 ** -22 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("low", [-1e9, -1e30, -3.4028234663852886e38])
+def test_a_bias_that_hides_far_keys_on_tensor_cores(on_tensor_cores, D, low):
+    """A bias of very low values is a window; whole tiles have it in front of the keys that count."""
+    from sandyrt_b200.csrc import ops
+
+    case = _paged_case(torch.float32, 2, 2, D, 16, [(0, 200), (90, 70)], seed=D)
+    bias = torch.zeros(2, 300, device=DEV)
+    bias[:, 40:] = low
+    got, _ = _both(case, 2, {"scale": 0.8 / D ** 0.5, "dist_bias": bias})
+    want = torch.empty_like(got)
+    ops.paged_attention(case["q"], case["kc"], case["vc"], case["table"], case["tok_seq"], case["tok_pos"], want, n_heads=2,
+                        scale=0.8 / D ** 0.5, window=40)
+    assert (got - want).abs().max().item() < 2e-5               # the bound of test_prompt_attention_f32
+
+
 @pytest.mark.parametrize("name", ["A", "C"])
 def test_float32_portions_on_both_sides_of_the_rule(model_dirs, plain_models, name):
     """Heads of 16 and 48: prompts of 32 to 100 tokens (48 is the last that the general kernel keeps) and portions behind a context,
