@@ -90,12 +90,13 @@ __device__ __forceinline__ void copy16_async(uint8_t* dst, const void* src) {
 }
 
 // The last step of a softmax row: a sink joins the denominator (exp(sink) relative to the row's maximum M,
-// nothing in the numerator), an output gate scales the head's result.
+// nothing in the numerator), an output gate scales the head's result.  as_portion: the row ends as the prompt kernels end theirs,
+// a NaN stays one and scores that are all minus infinity leave 0 / 0 (0 where a sink joins them).
 __device__ __forceinline__ float finish_row(float O, float L, float M, const float* sink, const float* out_gate, int t,
-                                            int h, int n_heads, bool keep_nan = false) {
-    if (sink && M > -INFINITY) L += expf(sink[h] - M);
+                                            int h, int n_heads, bool as_portion = false) {
+    if (sink && (M > -INFINITY || as_portion)) L += expf(sink[h] - M);
     const float g = out_gate ? out_gate[(size_t)t * n_heads + h] : 1.0f;
-    return L > 0.0f || (keep_nan && L != L) ? O / L * g : 0.0f;
+    return L > 0.0f || as_portion ? O / L * g : 0.0f;
 }
 
 template <typename T, int D>
@@ -471,7 +472,6 @@ SANDY_API int sandy_decode_attention_ext(const void* q, int ld_q, const void* k_
     return SANDY_ERR_UNSUPPORTED;
 }
 
-// The two forms above without a sink or an output gate.
 // For a step of mixed requests in float32: takes the requests that bring one token (q_start [n_seqs + 1], kv_before [n_seqs]) and leaves
 // the others' rows alone; heads of 64 and 128.
 SANDY_API int sandy_decode_attention_single(const float* q, int ld_q, const float* k_cache, const float* v_cache, long long page_stride,
@@ -494,6 +494,7 @@ SANDY_API int sandy_decode_attention_single(const float* q, int ld_q, const floa
         page_size, scale, window, num_splits, num_pages, sink, out_gate, status, stream, q_start);
 }
 
+// The two forms above without a sink or an output gate.
 SANDY_API int sandy_decode_attention_cluster(const void* q, int ld_q, const void* k_cache, const void* v_cache,
                                              long long page_stride, const int* block_table, int max_blocks,
                                              const int* token_seq, const int* positions, void* out, int ld_out,

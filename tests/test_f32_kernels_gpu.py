@@ -271,6 +271,33 @@ def test_single_tokens_beside_portions_on_the_decode_kernel(D, splits, window, b
     assert (got - want)[fine].abs().max().item() < 2e-5         # the bound of test_prompt_attention_f32
 
 
+@pytest.mark.parametrize("D,splits", [(64, 1), (64, 3), (128, 8)])
+@pytest.mark.parametrize("with_sink", [False, True])
+def test_single_tokens_whose_scores_are_all_minus_infinity(D, splits, with_sink):
+    """A row ends the same beside many single tokens as beside few: 0 / 0 of the formula without a sink, 0 with one."""
+    from sandyrt_b200.csrc import ops
+
+    seqs = [(40, 1), (0, 70), (330, 1), (0, 1)]
+    case = _paged_case(torch.float32, 4, 2, D, 16, seqs, seed=D)
+    for row, request in ((0, 0), (72, 3)):                  # queries above zero, every key of their requests -inf
+        case["q"][row] = case["q"][row].abs()
+        pages = case["table"][request]
+        case["kc"][pages[pages >= 0].long()] = -float("inf")
+    sink = torch.tensor([0.5, -1.0, 0.0, 2.0], device=DEV) if with_sink else None
+    q_start = torch.tensor([0] + list(np.cumsum([n for _, n in seqs])), dtype=torch.int32, device=DEV)
+    kv_before = torch.tensor([b for b, _ in seqs], dtype=torch.int32, device=DEV)
+    outs = []
+    for kw in ({}, {"tc": True}, {"tc": True, "single_splits": splits}):
+        outs.append(torch.full(case["q"].shape, 7.0, device=DEV))
+        ops.prefill_attention_f32(case["q"], case["kc"], case["vc"], case["table"], q_start, kv_before, outs[-1], n_heads=4, max_q_len=70,
+                                  scale=0.1, sink=sink, **kw)
+    ops.check_kernel_status(DEV)
+    for got in outs:
+        for row in (0, 72):
+            assert torch.isnan(got[row]).all() if sink is None else (got[row] == 0.0).all()
+        assert torch.isfinite(got[1:72]).all()
+
+
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("size", [2.0 ** -100, 2.0 ** 45])
 def test_prompt_attention_f32_sizes_on_tensor_cores(on_tensor_cores, D, size):
