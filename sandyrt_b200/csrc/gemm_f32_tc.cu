@@ -261,6 +261,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         constexpr int PER_ROW = BN / 4, WRITERS = WORKERS * 32;
         float* sums = reinterpret_cast<float*>(smem);
         const int total = BM / parts * PER_ROW;
+        int nan_row = -1;           // the row of a in which this warp last found a NaN: all its sums are one
         for (int base = 0; base < total; base += WRITERS) {
             const int at = base + tid;
             const int row = at / PER_ROW * parts + part, col = at % PER_ROW * 4;
@@ -285,16 +286,17 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 }
                 v[0] = s.x; v[1] = s.y; v[2] = s.z; v[3] = s.w;
             }
+            bool odd = false;
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                unsigned again = __ballot_sync(0xffffffffu, live && n + e < p.N && !is_finite(v[e]));
-                while (again) {
-                    const int who = __ffs(again) - 1;
-                    again &= again - 1;
-                    const int mm = __shfl_sync(0xffffffffu, m, who), nn = __shfl_sync(0xffffffffu, n, who) + e;
-                    const float plain = plain_sum(p.a + (size_t)mm * p.lda, p.w + (size_t)(w_row0 - n0 + nn) * p.ldw, p.K);
-                    if (lane == who) v[e] = plain;
-                }
+            for (int e = 0; e < 4; e++) odd |= live && n + e < p.N && !is_finite(v[e]);
+            for (unsigned again = __ballot_sync(0xffffffffu, odd); again; again &= again - 1) {
+                const int who = __ffs(again) - 1, mm = __shfl_sync(0xffffffffu, m, who), nn = __shfl_sync(0xffffffffu, n, who);
+                float plain[4] = {NAN, NAN, NAN, NAN};
+                if (mm != nan_row && plain_sums(p.a + (size_t)mm * p.lda, p.w + (size_t)(w_row0 - n0 + nn) * p.ldw, p.ldw, min(4, p.N - nn), p.K, plain))
+                    nan_row = mm;
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    if (lane == who && !is_finite(v[e])) v[e] = plain[e];
             }
             if (!live) continue;
             float* out = p.out + (size_t)m * p.ldc + n;

@@ -11,7 +11,7 @@
 // A bfloat16 ends where a float does, so the pieces of small floats would lose their low bits: both operands are split at
 // SCALE times their size, which keeps every bit of the smallest float, and the sums are scaled back (both exact).  What is large enough
 // to overflow for that, infinities and NaN come out as infinity or NaN; write-backs form every sum that is not finite again,
-// with float arithmetic from the operands (plain_sum), so they end as they would there.
+// with float arithmetic from the operands (plain_sums), so they end as they would there.
 #pragma once
 
 #include "tcgen05.cuh"
@@ -52,17 +52,27 @@ __device__ __forceinline__ void split_eight(const float4& x, const float4& y, ui
 
 __device__ __forceinline__ bool is_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
 
-// One element's sum in float arithmetic, by a whole warp; K is a multiple of 4 and both rows start on 16 bytes.
-__device__ __noinline__ float plain_sum(const float* a, const float* w, int K) {
-    float s = 0.0f;
+// The sums of a row of a with up to four rows of w in float arithmetic, by a whole warp; K is a multiple of 4 and all rows start on 16
+// bytes.  Returns whether the row of a holds a NaN: then its sum with any row is one.
+__device__ __forceinline__ bool plain_sums(const float* a, const float* w, int ldw, int rows, int K, float (&sum)[4]) {
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    bool nan = false;
+#pragma unroll 1
     for (int k = (threadIdx.x & 31) * 4; k < K; k += 128) {
-        const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
-        s = fmaf(x.x, y.x, s);
-        s = fmaf(x.y, y.y, s);
-        s = fmaf(x.z, y.z, s);
-        s = fmaf(x.w, y.w, s);
+        const float4 x = *reinterpret_cast<const float4*>(a + k);
+        nan |= x.x != x.x || x.y != x.y || x.z != x.z || x.w != x.w;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float4 y = *reinterpret_cast<const float4*>(w + (size_t)min(i, rows - 1) * ldw + k);
+            s[i] = fmaf(x.x, y.x, s[i]);
+            s[i] = fmaf(x.y, y.y, s[i]);
+            s[i] = fmaf(x.z, y.z, s[i]);
+            s[i] = fmaf(x.w, y.w, s[i]);
+        }
     }
-    return warp_sum(s);
+#pragma unroll
+    for (int i = 0; i < 4; i++) sum[i] = warp_sum(s[i]);
+    return __any_sync(0xffffffffu, nan);
 }
 
 // tensor-core product with the A operand in tensor memory

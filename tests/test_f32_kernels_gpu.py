@@ -110,6 +110,39 @@ def test_gemm_f32_on_tensor_cores(M, N, K, tile, parts, size):
     assert int(ops.kernel_status(a.device).item()) == 0
 
 
+def _milliseconds(call):
+    """The fastest of five calls."""
+    times = []
+    for _ in range(5):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        call()
+        end.record()
+        end.synchronize()
+        times.append(begin.elapsed_time(end))
+    return min(times)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_gemm_f32_on_tensor_cores_is_not_slow_on_what_is_not_finite(bad):
+    """A NaN in a row of a is found once (2.7 times as long as finite rows; 35 with every sum formed again by itself); infinities have
+    every sum formed again, which is not timed."""
+    from sandyrt_b200.csrc import ops
+
+    a, w, out = torch.randn(2048, 768, device=DEV), torch.randn(2304, 768, device=DEV), torch.empty(2048, 2304, device=DEV)
+    finite = _milliseconds(lambda: ops.gemm_f32_tc(a, w, None, out))
+    a[:, 5] = bad
+    time = _milliseconds(lambda: ops.gemm_f32_tc(a, w, None, out))
+    assert bad == bad or time < 10 * finite
+    assert torch.isnan(out).all() if bad != bad else torch.equal(out, (torch.sign(w[:, 5]) * bad).expand_as(out))
+    a, w, out = a[:130, :516].contiguous(), w[:99, :516].contiguous(), torch.empty(130, 99, device=DEV)
+    a[::3, 5] = float("nan")                                # rows of NaN between rows of infinities (or of NaN), columns no multiple of 4
+    ops.gemm_f32_tc(a, w, None, out)
+    assert torch.isnan(out[::3]).all()
+    if bad == bad:
+        assert torch.equal(out[1::3], (torch.sign(w[:, 5]) * bad).expand_as(out[1::3]))
+
+
 # ---- attention of prompt portions ---------------------------------------------------------------------------------
 def _both(case, H, kw):
     """The prompt kernel's output and the general kernel's, which reads one (token, head) pair at a time."""
