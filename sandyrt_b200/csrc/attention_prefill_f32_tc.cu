@@ -11,9 +11,9 @@
 // so no accumulator takes more than one chunk of k (two for heads above 64).  S of the next tile runs beside a tile's softmax, O beside the
 // next tile's; keys and values are fetched into registers a tile ahead.
 //
-// What is not finite, or so large that its product could leave the pieces' range (2^39 and more), takes its tile out of the tensor
-// cores: such a tile's scores, or its weighted sum, are formed with float arithmetic from the cache, so that a NaN or an infinity
-// reaches the queries that see it and no others.
+// What is not finite, or so large that its product could leave the pieces' range (2^39 and more), the tensor cores can't take: the scores
+// of such a query or key are formed with float arithmetic from the cache, such a value is left out of its tile's sum and added in float
+// arithmetic, so that a NaN or an infinity reaches the queries that see it and no others.
 //
 // What bounds it: the issue slots of the sixteen warps (splitting keys, values and probabilities, softmax: 3,500 a tile and scheduler of
 // the 5,000 clocks a tile takes) and the chain from a tile's scores to the next; the products are a quarter of that.  Alone, us, the fma
@@ -63,10 +63,28 @@ struct Form {
     static constexpr int COLS = D / SHARE;                      // output columns a thread
 };
 
+__device__ __forceinline__ bool is_large(float x) { return (__float_as_uint(x) & 0x7fffffffu) >= TOO_LARGE; }
 __device__ __forceinline__ bool too_large(const float4& v) {
     const uint32_t a = __float_as_uint(v.x) & 0x7fffffffu, b = __float_as_uint(v.y) & 0x7fffffffu, c = __float_as_uint(v.z) & 0x7fffffffu,
                    d = __float_as_uint(v.w) & 0x7fffffffu;
     return max(max(a, b), max(c, d)) >= TOO_LARGE;
+}
+
+__device__ __forceinline__ bool has_nan(const float4& v) { return v.x != v.x || v.y != v.y || v.z != v.z || v.w != v.w; }
+__device__ __forceinline__ void keep_small(float4& v) {
+    v = make_float4(is_large(v.x) ? 0.0f : v.x, is_large(v.y) ? 0.0f : v.y, is_large(v.z) ? 0.0f : v.z, is_large(v.w) ? 0.0f : v.w);
+}
+
+// A query times a key in float arithmetic; the key's row starts on 16 bytes, the query's if `pieces`.
+__device__ __forceinline__ float plain_score(const float* q, int pieces, const float* k, int d) {
+    float x = 0.0f;
+#pragma unroll 1
+    for (int c = 0; c < d; c += 4) {
+        const float4 a = pieces ? *reinterpret_cast<const float4*>(q + c) : make_float4(q[c], q[c + 1], q[c + 2], q[c + 3]);
+        const float4 b = *reinterpret_cast<const float4*>(k + c);
+        x = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, x))));
+    }
+    return x;
 }
 
 __device__ __forceinline__ float exp2_of(float x) {
@@ -84,8 +102,10 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
     __shared__ long long key_row[ROW_SLOTS][KEYS];  // row of the cache (in rows of a head) of each key of a tile; -1: none
     __shared__ float part_of[2][SHARE][BM];         // what the threads of a row exchange
     __shared__ uint64_t bars[4];                    // scores are there; a weighted sum is; keys' pieces are; probabilities and values are
-    __shared__ int odd_k[2], odd_v[2];              // the last tile (of even, of odd number) whose keys, values the tensor cores can't take
-    __shared__ int odd_q;
+    // What the tensor cores can't take: the queries (ODD, and NAN_TOO where one of its entries is a NaN), and the keys and values by the
+    // last tile of even, of odd number in which there was one, and in which this one was one.
+    enum { ODD = 1, NAN_TOO = 2 };
+    __shared__ int odd_q[BM], odd_k[2], odd_v[2], odd_key[2][KEYS], nan_key[2][KEYS], odd_value[2][KEYS];
     __shared__ uint32_t tmem_slot;
     enum { SCORES, SUM, KEYS_IN, PROBS_IN };
     const int seq = blockIdx.y, head = blockIdx.x;
@@ -142,21 +162,37 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
             to[i][1] = there ? src[1] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
-    // Rows of 128 bytes (64 entries), 128-byte swizzle.  Whether one of the floats is too large for the tensor cores.
+    // Rows of 128 bytes (64 entries), 128-byte swizzle.
     auto leave = [&](const float4 (&x)[2], uint8_t* to, int at_row, int at_entry, int block_bytes, int piece_bytes) {
         uint4 piece[N_PIECES];
         split_eight(x[0], x[1], piece);
         uint8_t* dst = to + (at_entry >> 6) * block_bytes + at_row * 128 + ((((at_entry & 63) >> 3) ^ (at_row & 7)) << 4);
 #pragma unroll
         for (int j = 0; j < N_PIECES; j++) *reinterpret_cast<uint4*>(dst + j * piece_bytes) = piece[j];
-        return too_large(x[0]) || too_large(x[1]);
     };
-    auto leave_tile = [&](const float4 (&x)[F::ITEMS][2], uint8_t* to) {
-        bool odd = false;
+    auto leave_keys = [&](int t) {
 #pragma unroll
-        for (int i = 0; i < F::ITEMS; i++) odd |= leave(x[i], to, at_key + i * APART, at_d, KEYS * 128, F::KV_PIECE);
+        for (int i = 0; i < F::ITEMS; i++) {
+            leave(kv[i], smem + F::OFF_K, at_key + i * APART, at_d, KEYS * 128, F::KV_PIECE);
+            if (too_large(kv[i][0]) || too_large(kv[i][1])) {
+                odd_k[t & 1] = odd_key[t & 1][at_key + i * APART] = t;
+                if (has_nan(kv[i][0]) || has_nan(kv[i][1])) nan_key[t & 1][at_key + i * APART] = t;
+            }
+        }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // my pieces, before the tensor core reads them
-        return odd;
+    };
+    // (what the tensor cores can't take of the values is added afterwards, see add_sum)
+    auto leave_values = [&](int t) {
+#pragma unroll
+        for (int i = 0; i < F::ITEMS; i++) {
+            if (too_large(vv[i][0]) || too_large(vv[i][1])) {
+                odd_v[t & 1] = odd_value[t & 1][at_key + i * APART] = t;
+                keep_small(vv[i][0]);
+                keep_small(vv[i][1]);
+            }
+            leave(vv[i], smem + F::OFF_V, at_key + i * APART, at_d, KEYS * 128, F::KV_PIECE);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     };
     bool expired = false;
     auto wait = [&](int bar, int phase) {
@@ -174,8 +210,9 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
         mbar_init(&bars[PROBS_IN], WORKERS / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         odd_k[0] = odd_k[1] = odd_v[0] = odd_v[1] = -1;
-        odd_q = 0;
     }
+    if (tid < BM) odd_q[tid] = 0;
+    if (tid < 2 * KEYS) odd_key[tid & 1][tid >> 1] = nan_key[tid & 1][tid >> 1] = odd_value[tid & 1][tid >> 1] = -1;
     if (warp == WORKERS / 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -228,8 +265,7 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
                 if (t < 0) continue;
                 wait(PROBS_IN, t);
                 if (expired) break;
-                if (odd_v[t & 1] == t) mbar_arrive(&bars[SUM]);
-                else issue_o();
+                issue_o();
             }
         }
         __syncwarp();
@@ -247,7 +283,6 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
 
     pdl_wait();
     fetch(0, p.k, kv);
-    bool odd = false;
     for (int i = tid; i < BM * D / 8; i += WORKERS) {
         const int at_row = i / (D / 8), at = i % (D / 8) * 8;
         float4 x[2] = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
@@ -261,10 +296,10 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
                 x[1] = make_float4(src[4], src[5], src[6], src[7]);
             }
         }
-        odd |= leave(x, smem, at_row, at, BM * 128, F::Q_PIECE);
+        leave(x, smem, at_row, at, BM * 128, F::Q_PIECE);
+        if (too_large(x[0]) || too_large(x[1])) atomicOr(&odd_q[at_row], has_nan(x[0]) || has_nan(x[1]) ? ODD | NAN_TOO : ODD);
     }
-    if (odd) odd_q = 1;
-    if (leave_tile(kv, smem + F::OFF_K)) odd_k[0] = 0;
+    leave_keys(0);
     arrive(KEYS_IN);
     if (tiles > 1) fetch(1, p.k, kv);
     fetch(0, p.v, vv);
@@ -284,39 +319,6 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
     // Tile t's weighted sum into o.
     auto add_sum = [&](int t) {
         wait(SUM, t);
-        if (odd_v[t & 1] == t) {
-            // in float arithmetic, the probabilities put together again from their pieces (which is exact): a value that a query does
-            // not see must not reach it (0 times it is not 0)
-#pragma unroll
-            for (int c = 0; c < F::COLS; c++) o[c] *= corr;
-#pragma unroll 1
-            for (int j = 0; j < KEYS; j += 16) {
-                uint32_t raw[N_PIECES][8];
-#pragma unroll
-                for (int i = 0; i < N_PIECES; i++) tmem_ld_32x8(tmem + lanes + F::P_COL + i * (KEYS / 2) + j / 2, raw[i]);
-                tmem_wait_ld();
-#pragma unroll
-                for (int e = 0; e < 16; e++) {
-                    float of[N_PIECES];
-#pragma unroll
-                    for (int i = 0; i < N_PIECES; i++) of[i] = __uint_as_float(e % 2 ? raw[i][e / 2] & 0xffff0000u : raw[i][e / 2] << 16);
-                    const float pr = (of[0] + (of[1] + of[2])) * (1.0f / SCALE);
-                    const long long at = key_row[t % ROW_SLOTS][j + e];
-                    if (at >= 0 && __float_as_uint(of[0]) != __float_as_uint(NOT_SEEN)) {
-                        const float* v = p.v + at * d + part * F::COLS;
-#pragma unroll 1
-                        for (int c0 = 0; c0 < F::COLS && part * F::COLS + c0 < d; c0++) {
-                            const float add = v[c0];
-#pragma unroll
-                            for (int c = 0; c < F::COLS; c++) o[c] = c == c0 ? fmaf(pr, add, o[c]) : o[c];
-                        }
-                    }
-                    __syncwarp();
-                }
-            }
-            meet();                                 // the other threads of these rows have read the probabilities
-            return;
-        }
 #pragma unroll
         for (int c = 0; c < F::COLS; c += 16) {
             uint32_t raw[16];
@@ -325,6 +327,34 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
 #pragma unroll
             for (int i = 0; i < 16; i++) o[c + i] = fmaf(o[c + i], corr, __uint_as_float(raw[i]) * UNSCALE);
         }
+        if (odd_v[t & 1] != t) return;
+        // What was left out of the tile's values, times the probabilities put together again from their pieces (which is exact); a value
+        // that a query does not see must not reach it (0 times it is not 0).
+#pragma unroll 1
+        for (int j = 0; j < KEYS; j++) {
+            if (odd_value[t & 1][j] != t) continue;
+            __syncwarp();
+            uint32_t raw[N_PIECES];
+#pragma unroll
+            for (int i = 0; i < N_PIECES; i++) raw[i] = tmem_ld_32x1(tmem + lanes + F::P_COL + i * (KEYS / 2) + j / 2);
+            tmem_wait_ld();
+            float of[N_PIECES];
+#pragma unroll
+            for (int i = 0; i < N_PIECES; i++) of[i] = __uint_as_float(j % 2 ? raw[i] & 0xffff0000u : raw[i] << 16);
+            const float pr = (of[0] + (of[1] + of[2])) * (1.0f / SCALE);
+            const bool seen = __float_as_uint(of[0]) != __float_as_uint(NOT_SEEN);
+            const float* v = p.v + key_row[t % ROW_SLOTS][j] * d + part * F::COLS;
+#pragma unroll
+            for (int c = 0; c < F::COLS; c += 4) {
+                if (part * F::COLS + c >= d) break;
+                const float4 x = *reinterpret_cast<const float4*>(v + c);
+                if (seen && is_large(x.x)) o[c] = fmaf(pr, x.x, o[c]);
+                if (seen && is_large(x.y)) o[c + 1] = fmaf(pr, x.y, o[c + 1]);
+                if (seen && is_large(x.z)) o[c + 2] = fmaf(pr, x.z, o[c + 2]);
+                if (seen && is_large(x.w)) o[c + 3] = fmaf(pr, x.w, o[c + 3]);
+            }
+        }
+        meet();                                     // the other threads of these rows have read the probabilities
     };
 
     const float unscale = UNSCALE * p.scale;
@@ -341,25 +371,31 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
 #pragma unroll
             for (int j = 0; j < MINE; j++) s[j] = __uint_as_float(raw[j]) * unscale;
         }
-        const bool odd_s = odd_q || odd_k[t & 1] == t;
+        unsigned again = 0;                         // bit j: the score of key j is to be formed again; bit 16 + j: as a NaN
+        if (odd_q[row] | (odd_k[t & 1] == t)) {
+#pragma unroll 1
+            for (int j = 0; j < MINE; j++) {
+                const int key = part * MINE + j;
+                if (odd_q[row] || odd_key[t & 1][key] == t) again |= 1u << j;
+                if ((odd_q[row] & NAN_TOO) || nan_key[t & 1][key] == t) again |= 65537u << j;
+            }
+        }
         if (t + 1 < tiles) {
-            if (leave_tile(kv, smem + F::OFF_K)) odd_k[(t + 1) & 1] = t + 1;
+            leave_keys(t + 1);
             arrive(KEYS_IN);
             if (t + 2 < tiles) fetch(t + 2, p.k, kv);
         }
         const int start = tile_start(t), end = tile_end(t);
         const long long* key_rows = &key_row[t % ROW_SLOTS][part * MINE];
-        if (odd_s) {                                // the same scores, in float arithmetic
-#pragma unroll 1
-            for (int j = 0; j < MINE; j++) {
-                const long long at = key_rows[j];
-                float x = 0.0f;
-                if (at >= 0 && row < rows)
-                    for (int c = 0; c < d; c++) x = fmaf(p.q[(size_t)(t0 + row) * p.ld_q + head * d + c], p.k[at * d + c], x);
+        for (; again & 0xffffu; again &= again - 1) {
+            const int j = __ffs(again) - 1;
+            float x = again >> 16 >> j & 1 ? NAN : 0.0f;
+            if (x == 0.0f && key_rows[j] >= 0 && row < rows)
+                x = plain_score(p.q + (size_t)(t0 + row) * p.ld_q + head * d, p.q_pieces, p.k + key_rows[j] * d, d) * p.scale;
 #pragma unroll
-                for (int i = 0; i < MINE; i++) s[i] = i == j ? x * p.scale : s[i];
-            }
+            for (int i = 0; i < MINE; i++) s[i] = i == j ? x : s[i];
         }
+        __syncwarp();
         const bool found = key_rows[lane % MINE] >= 0;
         unsigned hidden = 0;                        // bit j: this query does not see key j, whatever its score is
         if (!__all_sync(0xffffffffu, !ruled && found && start + KEYS - 1 <= pos0)) {
@@ -407,7 +443,7 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
 #pragma unroll
             for (int i = 0; i < N_PIECES; i++) tmem_st_32x8(tmem + lanes + F::P_COL + i * (KEYS / 2) + part * (MINE / 2), low[i], high[i]);
         }
-        if (leave_tile(vv, smem + F::OFF_V)) odd_v[t & 1] = t;
+        leave_values(t);
         tmem_wait_st();
         arrive(PROBS_IN);
         if (t + 1 < tiles) fetch(t + 1, p.v, vv);
