@@ -81,8 +81,9 @@ def test_gemm_f32_short(M, N, K):
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (33, 50, 12), (127, 97, 516), (129, 130, 576), (260, 257, 1028)])
 @pytest.mark.parametrize("size", [1.0, 2.0 ** -110, 2.0 ** 100])
 def test_gemm_f32_on_tensor_cores(M, N, K, tile, parts, size):
-    """Tiles, parts and chunks of k with remainders; pitches wider than the rows; the residual is the output itself; activations
-    whose pieces would leave the range of a bfloat16, and ones too large to be split; an infinite activation."""
+    """Tiles, parts and chunks of k with remainders; pitches wider than the rows; the residual is the output itself; an infinite
+    activation; very small activations with weights too large to be split (every sum is formed again in float arithmetic), and the reverse,
+    which can be split."""
     from sandyrt_b200.csrc import ops
 
     if parts > (K + 63) // 64:
@@ -92,7 +93,7 @@ def test_gemm_f32_on_tensor_cores(M, N, K, tile, parts, size):
     w = (torch.randn(N, K + 8, generator=g) / size).to(DEV)[:, :K]
     bias, x0 = torch.randn(N, generator=g).to(DEV), torch.randn(M, N + 3, generator=g).to(DEV)
     want = a.double() @ w.double().t() + bias.double()
-    # of a product 2^-26 is left out with the three smallest products of pieces; sixteen products at a time are added with at
+    # of a product 2^-24 is left out with the three smallest products of pieces; sixteen products at a time are added with at
     # most 2^-22 of their sizes lost to rounding towards zero: less than K * 2^-24 from K = 4 on; 4 for the write-back
     bound = (K + 4) * 2.0 ** -24 * (a.double().abs() @ w.double().abs().t() + bias.double().abs() + x0[:, :N].double().abs())
     wide = x0.clone()
@@ -108,6 +109,52 @@ def test_gemm_f32_on_tensor_cores(M, N, K, tile, parts, size):
     assert torch.equal(out[M - 1], torch.sign(w[:, K - 1]) * float("inf"))
     assert torch.equal(out[:M - 1], finite[:M - 1])
     assert int(ops.kernel_status(a.device).item()) == 0
+
+
+# What a product of two floats may be off by: the three products of pieces that are left out reach 2^-24 of it together, and the
+# tensor core's last addition takes up to 2^-23 towards zero (the ones before it are of 2^-8 of the size).
+ONE_PRODUCT = 2.0 ** -24 + 2.0 ** -23 + 2.0 ** -30
+
+TILES = [(0, 0), (64, 1), (64, 8), (96, 1), (96, 4), (128, 1), (128, 2), (128, 8)]
+
+
+@pytest.mark.parametrize("tile,parts", TILES)
+@pytest.mark.parametrize("M,N,K", [(130, 97, 516), (257, 130, 1028)])
+@pytest.mark.parametrize("size_a,size_w", [(0, 0), (-118, 40), (40, -118), (-100, 100)])
+def test_gemm_f32_on_tensor_cores_keeps_24_bits(M, N, K, tile, parts, size_a, size_w):
+    """Rows with one number each, at every place of every chunk: an output is one product, whose six products of pieces show: without
+    any of them it is off by 2^-20 to 2^-8 of its size in one place or another.  Sizes (powers of two) whose last pieces would lie below
+    a bfloat16's range were they not scaled; all of them can be split, so no sum is formed again in float arithmetic."""
+    from sandyrt_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(M + N + K)
+    number, w = (1.0 + torch.rand(M, generator=g)) * 2.0 ** size_a, (1.0 + torch.rand(N, K, generator=g)) * 2.0 ** size_w
+    at = torch.arange(M) * 37 % K
+    a = torch.zeros(M, K)
+    a[torch.arange(M), at] = number * torch.where(torch.arange(M) % 2 == 0, 1.0, -1.0)
+    want = a[torch.arange(M), at].double()[:, None] * w[:, at].t().double()
+    out = torch.empty(M, N, device=DEV)
+    ops.gemm_f32_tc(a.to(DEV), w.to(DEV), None, out, tile=tile, parts=parts)
+    assert bool(((out.double().cpu() - want).abs() <= ONE_PRODUCT * want.abs()).all())
+
+
+@pytest.mark.parametrize("tile,parts", TILES)
+@pytest.mark.parametrize("M,N,K", [(129, 130, 576), (260, 257, 1028), (64, 96, 3072)])
+@pytest.mark.parametrize("sign", ["both", "one operand", "none"])
+def test_gemm_f32_on_tensor_cores_error(M, N, K, tile, parts, sign):
+    """The whole error (2-norm) over many chunks.  Sums of one sign: four additions of a chunk's own size lose up to 2^-23 of a quarter,
+    a half, three quarters and all of it, which is 2.5 * 2^-23 at the most and half of that on average, and the chunks are added with
+    float roundings.  Centred ones shrink as their partial sums do: four times half of 2^-23 of a chunk, whose size is sqrt(64 / K) of the
+    sum's, once for every chunk.  Three products of pieces less cost 4e-6."""
+    from sandyrt_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(M + N + K)
+    a, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    a, w = a.abs() if sign != "both" else a, w.abs() if sign == "none" else w
+    want = a.double() @ w.double().t()
+    out = torch.empty(M, N, device=DEV)
+    ops.gemm_f32_tc(a, w, None, out, tile=tile, parts=parts)
+    assert float((out.double() - want).norm() / want.norm()) < 2.0 * 2.0 ** -23
 
 
 def _milliseconds(call):
@@ -351,12 +398,41 @@ def test_single_tokens_whose_scores_are_all_minus_infinity(D, splits, with_sink)
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("size", [2.0 ** -100, 2.0 ** 45])
 def test_prompt_attention_f32_sizes_on_tensor_cores(on_tensor_cores, D, size):
-    """Keys whose last pieces would lie below a bfloat16's range, and keys and values too large to be split."""
+    """Small keys and values, and ones too large to be split."""
     case = _paged_case(torch.float32, 2, 2, D, 16, [(0, 130), (63, 65)], seed=D)
     case["kc"] *= size
     case["vc"] *= size
     got, want = _both(case, 2, {"scale": 0.8 / D ** 0.5 / size})
     assert (got - want).abs().max().item() < 2e-5 * size        # the bound of test_prompt_attention_f32
+
+
+@pytest.mark.parametrize("D", [64, 80, 128])
+def test_prompt_attention_f32_on_tensor_cores_keeps_24_bits(on_tensor_cores, D):
+    """A query that sees one key has that key's value, every bit of it: its weight is 1, and a value is the sum of its pieces.  With all
+    keys: scores of up to 4 may be off by ONE_PRODUCT of the products they add up (sizes of about their own), an exponential by 2^-22, and
+    so may the weights' sum; the 2-norm stays below a quarter of what the worst of them add up to, 2^-19.  Scores without their last pieces
+    are off by 2^-17."""
+    case = _paged_case(torch.float32, 4, 2, D, 16, [(0, 130), (63, 65), (200, 70)], seed=D)
+    got, _ = _both(case, 4, {"scale": 1.0, "window": 1})
+    own = torch.cat([v[before:].repeat_interleave(2, 1).reshape(n, -1) for (before, n), v in zip(case["seqs"], case["dense_v"])])
+    assert torch.equal(got.cpu(), own)
+    case["dense_k"], case["dense_v"] = ([x.repeat_interleave(2, 1) for x in case[name]] for name in ("dense_k", "dense_v"))
+    got, _ = _both(case, 4, {"scale": D ** -0.5})
+    want = _formula(case, 4, D ** -0.5, 0, None)
+    assert float((got.double().cpu() - want).norm() / want.norm()) < 2.0 ** -21
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_prompt_attention_f32_of_very_small_keys_on_tensor_cores(on_tensor_cores, D):
+    """Keys and values of 2^-120, whose last pieces would lie below a bfloat16's range were they not scaled, under queries that make ordinary
+    scores of them."""
+    case = _paged_case(torch.float32, 2, 2, D, 16, [(0, 130), (63, 65)], seed=D)
+    case["kc"] *= 2.0 ** -120
+    case["vc"] *= 2.0 ** -120
+    case["q"] *= 2.0 ** 35
+    got, _ = _both(case, 2, {"scale": 2.0 ** 85 / D ** 0.5})
+    want = _formula(case, 2, D ** -0.5, 0, None)
+    assert float((got.double().cpu() * 2.0 ** 120 - want).norm() / want.norm()) < 2.0 ** -21
 
 
 def _keys_of(case):
@@ -502,6 +578,25 @@ def test_expert_product_f32_on_tensor_cores(sizes, N, K):
     assert torch.equal(again[n - 1].cpu(), torch.sign(w[which[n - 1], :, K - 1]) * float("inf"))
     assert torch.equal(again[:n - 1], finite[:n - 1])
     assert int(ops.kernel_status(out.device).item()) == 0
+
+
+@pytest.mark.parametrize("sizes,N,K", [([128, 129, 0, 127, 1], 130, 576), ([300], 64, 516), ([5, 9], 1000, 768)])
+def test_expert_product_f32_on_tensor_cores_keeps_24_bits(sizes, N, K):
+    """As test_gemm_f32_on_tensor_cores_keeps_24_bits, a matrix per expert."""
+    from sandyrt_b200.csrc import ops
+
+    g = torch.Generator().manual_seed(N + K)
+    n, G = sum(sizes), len(sizes)
+    at = torch.arange(n) * 37 % K
+    a, w = torch.zeros(n, K), 1.0 + torch.rand(G, N, K, generator=g)
+    a[torch.arange(n), at] = 1.0 + torch.rand(n, generator=g)
+    start = torch.tensor([0] + list(np.cumsum(sizes)), dtype=torch.int32)
+    r = types.SimpleNamespace(n_experts=G, n_tokens=n, top=1, group_start=start.to(DEV))
+    out = torch.empty(n, N, device=DEV)
+    ops.expert_product_f32_tc(r, a.to(DEV), w.view(G * N, K).to(DEV), out)
+    which = torch.repeat_interleave(torch.arange(G), torch.tensor(sizes))
+    want = a[torch.arange(n), at].double()[:, None] * w[which, :, at].double()
+    assert bool(((out.double().cpu() - want).abs() <= ONE_PRODUCT * want.abs()).all())
 
 
 @pytest.mark.parametrize("T", [1, 4, 5, 64, 65, 150])

@@ -48,12 +48,15 @@ def wide(tmp_path_factory):
 class _Running:
     """An engine and what its requests have been fed."""
 
-    def __init__(self, wide, contexts, seed):
+    def __init__(self, wide, contexts, seed, dtype=torch.bfloat16):
         from sandyrt_b200.engine.step import Engine
         from sandyrt_b200.models.model import load_model
 
         self.plain = wide[1]
-        self.eng = Engine(load_model(wide[0], device="cuda:0", dtype=torch.bfloat16), max_tokens=8192, max_requests=48)
+        self.eng = Engine(load_model(wide[0], device="cuda:0", dtype=dtype), max_tokens=8192, max_requests=48)
+        # two layers of bfloat16 roundings in another order: 5e-3 of the row; of float32 ones: 1e-6; a row that no launch wrote is off by
+        # its size
+        self.tol = 2e-2 if dtype == torch.bfloat16 else 1e-5
         self.eng.cache.device_caches.poison()
         self.rng = np.random.default_rng(seed)
         self.fed = {}
@@ -73,8 +76,7 @@ class _Running:
         if check:
             for (r, n), row in zip(portions, got):
                 want = self.plain.logits(self.fed[r], [len(self.fed[r]) - 1])[0].astype(np.float64)
-                # two layers of bfloat16 roundings in another order: 5e-3 of the row; a row that no launch wrote is off by its size
-                assert np.linalg.norm(row - want) < 2e-2 * np.linalg.norm(want), (r, n, portions)
+                assert np.linalg.norm(row - want) < self.tol * np.linalg.norm(want), (r, n, portions)
         return self.eng.last_launches
 
 
@@ -117,6 +119,70 @@ def test_engine_step_without_single_tokens_takes_no_second_launch(wide):
 def test_engine_recording_is_not_shared_by_steps_with_and_without_single_tokens(wide):
     """Equal tokens, requests and longest portion: sixteen single tokens beside two portions, then portions alone."""
     run = _Running(wide, [150] + [4] * 17, seed=6)
+    for _ in range(2):
+        run.step([(r, 1) for r in range(16)] + [(16, 40), (17, 24)])
+    for _ in range(2):
+        run.step([(0, 40)] + [(r, 2) for r in range(1, 7)] + [(r, 3) for r in range(7, 13)] + [(r, 2) for r in range(13, 18)])
+    for _ in range(2):
+        run.step([(r, 1) for r in range(2, 18)] + [(1, 24), (0, 40)])
+
+
+# ---- the same in float32 ------------------------------------------------------------------------------------------
+@pytest.fixture(scope="module")
+def models32(tmp_path_factory):
+    """16 heads of 64, which the decode kernel has a form for, and 16 of 48, which it has none for."""
+    from conftest import make_model_dir
+    from plain_gpt2 import PlainGPT2
+
+    out = {}
+    for size in (64, 48):
+        folder = make_model_dir(dict(architectures=["GPT2LMHeadModel"], model_type="gpt2", n_layer=LAYERS, n_embd=HEADS * size, n_head=HEADS,
+                                     n_inner=256, vocab_size=VOCAB, n_positions=1024, layer_norm_epsilon=1e-5, activation_function="gelu_new"),
+                                str(tmp_path_factory.mktemp("mixed32") / "model"), seed=8)
+        out[size] = (folder, PlainGPT2(folder, "f32"))
+    return out
+
+
+def _attention_classes(run, portions):
+    """The classes of attention launches in a step that is not a recorded one."""
+    from sandyrt_b200 import core
+
+    core.call("global", None, "profile_kernels", enable=True)
+    try:
+        run.step(portions)
+    finally:
+        rows = core.call("global", None, "profile_kernels", enable=False)
+    return {r["class"] for r in rows if r["class"].startswith("attention")}
+
+
+# heads of 64 leave the prompt kernel from 150 (token, head) pairs on, behind a table of more than 128 keys; heads of 48 stay on the tensor
+# cores up to 384 pairs (single tokens are counted in powers of two: 15 as 8, 33 as 32)
+@pytest.mark.parametrize("size,singles,longest,apart,kernel", [
+    (64, 15, 150, False, "tcgen05"), (64, 16, 150, True, "tcgen05"), (64, 20, 150, True, "tcgen05"), (64, 33, 150, True, "tcgen05"),
+    (64, 20, 60, False, "tcgen05"), (64, 16, 820, True, "tcgen05"),
+    (48, 20, 150, False, "tcgen05"), (48, 31, 150, False, "tcgen05"), (48, 32, 150, False, "fma")])
+def test_engine_steps_of_single_tokens_beside_a_portion_in_float32(models32, size, singles, longest, apart, kernel):
+    run = _Running(models32[size], _contexts(singles)[:-1] + [longest], seed=singles, dtype=torch.float32)
+    launches, replays = [], run.eng.graph_replays
+    for step, at in enumerate((singles, 0, singles // 2, 1)):
+        portions = [(r, 1) for r in range(singles)]
+        portions.insert(at, (f"new {step}", 37))
+        if step == 0:
+            want = "attention, prompt (float32, tcgen05)" if kernel == "tcgen05" else "attention, prompt (float32)"
+            assert _attention_classes(run, portions) == {want}
+        else:
+            run.step(portions)
+        launches.append(run.eng.last_launches)
+        run.eng.release(f"new {step}")
+    assert run.eng.graph_replays - replays >= 2 and len(set(launches)) == 1
+    alone = _Running(models32[size], [3], seed=1, dtype=torch.float32)
+    one = alone.step([(0, 1), ("new", 37)])
+    assert launches[0] - one == (LAYERS if apart else 0)
+
+
+def test_engine_recording_in_float32_is_not_shared_by_steps_with_and_without_single_tokens(models32):
+    """Equal tokens, requests and longest portion: sixteen single tokens beside two portions, then portions alone."""
+    run = _Running(models32[64], [150] + [4] * 17, seed=6, dtype=torch.float32)
     for _ in range(2):
         run.step([(r, 1) for r in range(16)] + [(16, 40), (17, 24)])
     for _ in range(2):
