@@ -631,6 +631,9 @@ void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const K
                 check(code, "prefill_attention_f32_tc" + shape);
                 if (!apart) return;
                 static auto single = SANDY_KERNEL(attention_decode, sandy_decode_attention_single);
+                // (6 and 7 splits too: beside a portion they are within 5 % of their neighbours.  4 / 5 / 6 / 7 / 8 splits, us: 16 heads
+                // of 64, 16 tokens behind up to 760 keys 31.5 / 32.5 / 32.3 / 34.0 / 34.3, 32 behind 800 76.5 / 77.5 / 77.1 / 79.1 / 79.4;
+                // 12 of 128, 16 behind 850 80.0 / 75.0 / 73.9 / 77.1 / 75.3.)
                 const int splits = std::min(kClusterMaxSplits, std::max(decode_splits(s.n_single, n_heads, seen), seen / 128));
                 check(single((const float*)q.data, (int)q.ld, (const float*)c.k, (const float*)c.v, c.page_stride, s.block_table, s.max_blocks,
                              s.q_start, s.kv_before, (float*)out.data, (int)out.ld, s.n_seqs, n_heads, hkv, d, c.page_size, scale, window,

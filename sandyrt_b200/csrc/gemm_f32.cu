@@ -25,7 +25,8 @@
 //          warps that share a row in shared memory.
 // tile     up to 64 rows of narrow products, where the tensor cores (gemm_f32_tc.cu) do not pay.  Tiles of 32*WM x 8*TN*WN outputs
 //          behind a ring of cp.async stages of 32 k; 8 x TN outputs a thread.  Where the tiles are too few for the SMs, the blocks
-//          of a cluster split k and add up through shared memory.
+//          of a cluster split k and add up through shared memory.  What is left to it takes tiles of 64 x 64 in as many parts as k
+//          allows; 128 x 128 and 64 x 128, and the rule that weighs them, serve comparisons (microbench.py) and tests.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -19,7 +19,11 @@
 // registers pass the same memory (1.4).  Alone, bias folded in, weights from HBM, us, the fma tiles of gemm_f32.cu -> this kernel:
 // 2,048 rows, 2,304 x 768 167 -> 48 (151 TFLOP/s), 768 x 768 70 -> 20, 3,072 x 768 250 -> 71, 768 x 3,072 241 -> 55 (176 TFLOP/s
 // of the 278 that a sixth of the measured bfloat16 rate is); 128 rows, 3,072 x 768 21 -> 11; 64 rows, 50,257 x 768 137 -> 76.
-// Error against 64 bits (2-norm, normal operands), k 768: 3.5e-7 -> 1.0e-7; k 3,072: 5.0e-7 -> 1.5e-7.
+// Error against 64 bits (2-norm), fma kernels -> this one.  Operands of both signs, or one of them: 1.1e-7 -> 0.8e-7 (k 64),
+// 1.4e-7 to 1.9e-7 -> 0.9e-7 (768), 2.6e-7 -> 1.1e-7 (3,072).  Operands all of one sign, which the additions towards zero shrink
+// (split_f32.cuh): 0.7e-7 -> 0.8e-7 to 0.9e-7 (64), 0.5e-7 to 0.7e-7 -> 0.9e-7 (768 and 3,072), 0.8e-7 -> 0.9e-7 to 1.0e-7 (6,400).
+// What is not finite, 2,048 x 2,304 x 768, us: finite 50; a NaN in one row of a 52, in every row 131, in one of w 62; infinities in every
+// row of a 960 (the fma tiles 169 throughout).
 // Every wait on an mbarrier is bounded: on expiry the kernel raises `*status`, stops issuing, frees its tensor memory and
 // returns.
 #include <cooperative_groups.h>

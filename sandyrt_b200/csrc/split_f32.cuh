@@ -3,10 +3,13 @@
 // A float is the sum of three bfloat16 (24 bits in three times 8, each piece the rounded rest of the ones before), and a
 // product of two bfloat16 is exact in the tensor core's float sums.  Of the nine products of pieces six are formed,
 //   a0 w0 + (a0 w1 + a1 w0) + (a0 w2 + a1 w1 + a2 w0);
-// the other three lie below 2^-25 of the product, where a float product is itself rounded.  The tensor core's own additions
+// the other three lie below 2^-24 of the product together, which is what a float product is itself rounded by.  (The method is that of
+// G. Henry, P. T. P. Tang and A. Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations",
+// 2019.)  The tensor core's own additions
 // round towards zero, which over a long k would shrink a sum by more than float additions in order miss it by, so an
 // accumulator takes CHUNK k only: first the small products, then the large ones (four roundings of the sum's own size), and is
-// then added into registers with ordinary float additions.
+// then added into registers with ordinary float additions.  What is left of it: sums whose products all have one sign are 0.6 * 2^-23 of
+// their size too small on average.
 //
 // A bfloat16 ends where a float does, so the pieces of small floats would lose their low bits: both operands are split at
 // SCALE times their size, which keeps every bit of the smallest float, and the sums are scaled back (both exact).  What is large enough

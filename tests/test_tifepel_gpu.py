@@ -156,7 +156,9 @@ def test_mixed_batches_with_pages_and_slots_used_again(models, name, dtype):
     cfg, w, path = models[name, dtype]
     eng = _engine(path, dtype, max_tokens=192, page_size=16, max_requests=4)
     lengths = [37, 50, 21, 64, 45, 30, 58, 17]
-    prompts = [_tokens(cfg, n, seed=20 + i) for i, n in enumerate(lengths)]
+    prompts = [_tokens(cfg, n, seed=28 + i) for i, n in enumerate(lengths)]
+    # no router decides by less than float32 sums in another order differ (the seeds from 20 on have one of 45 tokens that does, by 1.7e-7)
+    assert dtype == "bfloat16" or min(plain.router_margin(cfg, w, ids) for ids in prompts) > 1e-5
     rng = np.random.default_rng(1)
     fed = [0] * len(prompts)
     got = [[] for _ in prompts]
