@@ -613,15 +613,26 @@ void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const K
     }
     // float32 prompts (the general kernel also keeps heads above 128)
     if (s.max_q_len > 1 && q.dtype == DType::F32 && d <= 128 && !prompt_f32_general(d, s.max_q_len, s.max_blocks * c.page_size)) {
-        // Heads above 32 go to the tensor cores, whose blocks take 128 queries; single tokens beside the portions are best on the decode
-        // kernel, and where there are many that it has no form for (its head sizes, its rules) on the fma tiles of 64 queries.  Alone,
-        // us, fma tiles / tensor cores / tensor cores and decode kernel, single tokens behind some 100 to 700 keys beside a portion: 16
-        // heads of 64, 32 beside 480 109 / 113 / 73; 12 heads, 60 beside 16 134 / 179 / 97, 16 beside 300 52 / 41 / 30, 8 beside 300 48 /
-        // 22 / 26, 8 beside 30 33 / 21 / 15; 25 heads, 20 beside 200 63 / 55 / 30; 12 heads of 128, 32 beside 100 180 / 190 / 85.
+        // Heads above 32 go to the tensor cores, whose blocks take 128 queries and an SM each; single tokens beside the portions are best on
+        // the decode kernel, and where there are many that it has no form for (its head sizes, its rules, short tables) on the fma tiles of
+        // 64 queries, of which an SM holds three.  Alone, us, fma tiles / tensor cores / tensor cores and decode kernel, single tokens behind
+        // some 100 to 700 keys beside a portion: 16 heads of 64, 32 beside 480 109 / 113 / 73; 12 heads, 60 beside 16 134 / 179 / 97, 16
+        // beside 300 52 / 41 / 30, 8 beside 300 48 / 22 / 26, 8 beside 30 33 / 21 / 15; 25 heads, 20 beside 200 63 / 55 / 30; 12 heads of
+        // 128, 32 beside 100 180 / 190 / 85.
+        // Without the decode kernel the line is a round of their blocks on the SMs, more where a long portion or many keys weigh more than
+        // the blocks' starts.  A layer of an engine's step, us that the tensor cores save: behind 5 to 60 keys beside a portion of 16, 12
+        // heads of 64, 8 tokens 5, 12 -2, 15 -7, 31 -15; beside 100 17, 4, 4, 0, beside 400 33, 32, 36, 30.  Behind 100 to 700 beside 16 34,
+        // 32, 16, -12 (23 tokens 8); 25 heads of 48, 8 tokens 15, 12 -6; 12 heads of 128, 12 tokens 24, 15 -13, 31 -37, beside 400 27, -10.
         const int seen = window > 0 ? std::min(window + keep, s.max_blocks * c.page_size) : s.max_blocks * c.page_size;
+        // Single tokens there are at least, from the counts that a recorded step is kept by: the other requests share what the longest
+        // portion leaves, two tokens each or one.  With one portion this is their number, n_single rounds it down.
+        const int singles = std::max(s.n_single, 2 * (s.n_seqs - 1) - (T - s.max_q_len));
+        const bool long_portion = s.max_q_len >= 64 && (d <= 64 || seen < s.max_q_len + 256);
+        const int rounds = long_portion ? (s.max_q_len >= 256 ? 3 : 2) : d <= 64 && seen >= 256 ? 2 : 1;
+        const bool few = singles * n_heads <= rounds * sm_count();
         const bool decodable = (d == 64 || d == 128) && !ruled && !db && !gated && s.n_seqs <= 65535 && q.ld % 4 == 0 && !((uintptr_t)q.data & 15);
-        const bool apart = decodable && s.n_single * n_heads >= 150 && seen > 128;
-        if (d > 32 && (apart || s.n_single * n_heads < 384)) {
+        const bool apart = decodable && (!few || singles * n_heads >= 150) && seen > 128;
+        if (d > 32 && (apart || few)) {
             static auto fn = SANDY_KERNEL(attention_prefill_f32_tc, sandy_prefill_attention_f32_tc_rules);
             OpTimer timer(l, "attention, prompt (float32, tcgen05)", attn_bytes, attn_flops);
             const int code = fn((const float*)q.data, (int)q.ld, (const float*)c.k, (const float*)c.v, c.page_stride, s.block_table,
@@ -634,7 +645,7 @@ void attention(const Launch& l, const AttentionStep& s, const Tensor& q, const K
                 // (6 and 7 splits too: beside a portion they are within 5 % of their neighbours.  4 / 5 / 6 / 7 / 8 splits, us: 16 heads
                 // of 64, 16 tokens behind up to 760 keys 31.5 / 32.5 / 32.3 / 34.0 / 34.3, 32 behind 800 76.5 / 77.5 / 77.1 / 79.1 / 79.4;
                 // 12 of 128, 16 behind 850 80.0 / 75.0 / 73.9 / 77.1 / 75.3.)
-                const int splits = std::min(kClusterMaxSplits, std::max(decode_splits(s.n_single, n_heads, seen), seen / 128));
+                const int splits = std::min(kClusterMaxSplits, std::max(decode_splits(singles, n_heads, seen), seen / 128));
                 check(single((const float*)q.data, (int)q.ld, (const float*)c.k, (const float*)c.v, c.page_stride, s.block_table, s.max_blocks,
                              s.q_start, s.kv_before, (float*)out.data, (int)out.ld, s.n_seqs, n_heads, hkv, d, c.page_size, scale, window,
                              splits, c.num_pages, sk, og, l.kernel_status, l.stream),

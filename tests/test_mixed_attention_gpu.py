@@ -155,12 +155,13 @@ def _attention_classes(run, portions):
     return {r["class"] for r in rows if r["class"].startswith("attention")}
 
 
-# heads of 64 leave the prompt kernel from 150 (token, head) pairs on, behind a table of more than 128 keys; heads of 48 stay on the tensor
-# cores up to 384 pairs (single tokens are counted in powers of two: 15 as 8, 33 as 32)
+# Heads of 64 leave the prompt kernel behind a table of more than 128 keys from 150 (token, head) pairs on; what cannot leave it stays on the
+# tensor cores up to a round of blocks on 148 SMs, up to two behind 256 keys and more.
 @pytest.mark.parametrize("size,singles,longest,apart,kernel", [
-    (64, 15, 150, False, "tcgen05"), (64, 16, 150, True, "tcgen05"), (64, 20, 150, True, "tcgen05"), (64, 33, 150, True, "tcgen05"),
-    (64, 20, 60, False, "tcgen05"), (64, 16, 820, True, "tcgen05"),
-    (48, 20, 150, False, "tcgen05"), (48, 31, 150, False, "tcgen05"), (48, 32, 150, False, "fma")])
+    (64, 9, 150, False, "tcgen05"), (64, 10, 150, True, "tcgen05"), (64, 15, 150, True, "tcgen05"), (64, 16, 150, True, "tcgen05"),
+    (64, 33, 150, True, "tcgen05"), (64, 16, 820, True, "tcgen05"), (64, 9, 60, False, "tcgen05"), (64, 10, 60, False, "fma"),
+    (48, 9, 60, False, "tcgen05"), (48, 10, 60, False, "fma"), (48, 18, 150, False, "tcgen05"), (48, 19, 150, False, "fma"),
+    (48, 33, 820, False, "fma")])
 def test_engine_steps_of_single_tokens_beside_a_portion_in_float32(models32, size, singles, longest, apart, kernel):
     run = _Running(models32[size], _contexts(singles)[:-1] + [longest], seed=singles, dtype=torch.float32)
     launches, replays = [], run.eng.graph_replays
