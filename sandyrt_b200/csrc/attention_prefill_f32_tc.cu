@@ -13,15 +13,15 @@
 //
 // What is not finite, or so large that its product could leave the pieces' range (2^39 and more), the tensor cores can't take: the scores
 // of such a query or key are formed with float arithmetic from the cache, such a value is left out of its tile's sum and added in float
-// arithmetic, so that a NaN or an infinity reaches the queries that see it and no others.
+// arithmetic at the end, so that a NaN or an infinity reaches the queries that see it and no others.
 //
 // What bounds it: the issue slots of the sixteen warps (splitting keys, values and probabilities, softmax: 3,500 a tile and scheduler of
 // the 5,000 clocks a tile takes) and the chain from a tile's scores to the next; the products are a quarter of that.  Alone, us, the fma
 // tiles of attention_prefill_f32.cu -> this kernel: two prompts of 1,024 tokens, 12 heads of 64 132 -> 52; four of 100 to 412, 12 heads
-// of 64 54 -> 25, 12 heads of 128 on one key/value head 92 -> 49; one of 16 14 -> 9; four tokens behind 300 33 -> 19.  Error against 64
+// of 64 54 -> 25, 12 heads of 128 on one key/value head 92 -> 40; one of 16 14 -> 9; four tokens behind 300 33 -> 19.  Error against 64
 // bits (2-norm) of the first 2.8e-7 -> 1.5e-7, with values of one sign 2.4e-7 -> 1.0e-7, sharp scores 5.5e-7 -> 3.0e-7 (the exponentials are
-// the hardware's base-2 ones, good to 2^-22, on a difference rounded to a float, as expf's argument was).  One query of NaN in the first 86 us,
-// one key 55, one value 57, nothing but NaN keys 122, values 470 (fma tiles 132 to 254); one infinite query 416.  With eight warps, one of them issuing the products too, it took 100 us.
+// the hardware's base-2 ones, good to 2^-22, on a difference rounded to a float, as expf's argument was).  One query of NaN in the first 88 us,
+// one key or value 56, nothing but NaN keys 144, values 94 (fma tiles 132 to 254); one infinite query 445.  With eight warps, one of them issuing the products too, it took 100 us.
 //
 // Every wait on an mbarrier is bounded: on expiry the kernel raises `*status` (bit 8) and runs to its end (its output is then not valid).
 #include "attention_rules.h"
@@ -104,10 +104,11 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
     __shared__ long long key_row[ROW_SLOTS][KEYS];  // row of the cache (in rows of a head) of each key of a tile; -1: none
     __shared__ float part_of[2][SHARE][BM];         // what the threads of a row exchange
     __shared__ uint64_t bars[4];                    // scores are there; a weighted sum is; keys' pieces are; probabilities and values are
-    // What the tensor cores can't take: the queries (ODD, and NAN_TOO where one of its entries is a NaN), and the keys and values by the
-    // last tile of even, of odd number in which there was one, and in which this one was one.
+    // What the tensor cores can't take: the queries (ODD, and NAN_TOO where one of its entries is a NaN); the keys by the last tile (of
+    // those whose number ends in the same bits: other warps leave the keys of two tiles on) in which there was one, and in which this one
+    // was one; the first and the last tile with such a value.
     enum { ODD = 1, NAN_TOO = 2 };
-    __shared__ int odd_q[BM], odd_k[2], odd_v[2], odd_key[2][KEYS], nan_key[2][KEYS], odd_value[2][KEYS];
+    __shared__ int odd_q[BM], odd_k[4], odd_key[4][KEYS], nan_key[4][KEYS], odd_v[2];
     __shared__ uint32_t tmem_slot;
     enum { SCORES, SUM, KEYS_IN, PROBS_IN };
     const int seq = blockIdx.y, head = blockIdx.x;
@@ -177,18 +178,19 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
         for (int i = 0; i < F::ITEMS; i++) {
             leave(kv[i], smem + F::OFF_K, at_key + i * APART, at_d, KEYS * 128, F::KV_PIECE);
             if (too_large(kv[i][0]) || too_large(kv[i][1])) {
-                odd_k[t & 1] = odd_key[t & 1][at_key + i * APART] = t;
-                if (has_nan(kv[i][0]) || has_nan(kv[i][1])) nan_key[t & 1][at_key + i * APART] = t;
+                odd_k[t & 3] = odd_key[t & 3][at_key + i * APART] = t;
+                if (has_nan(kv[i][0]) || has_nan(kv[i][1])) nan_key[t & 3][at_key + i * APART] = t;
             }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // my pieces, before the tensor core reads them
     };
-    // (what the tensor cores can't take of the values is added afterwards, see add_sum)
+    // (what the tensor cores can't take of the values is added at the end)
     auto leave_values = [&](int t) {
 #pragma unroll
         for (int i = 0; i < F::ITEMS; i++) {
             if (too_large(vv[i][0]) || too_large(vv[i][1])) {
-                odd_v[t & 1] = odd_value[t & 1][at_key + i * APART] = t;
+                atomicMin(&odd_v[0], t);
+                atomicMax(&odd_v[1], t);
                 keep_small(vv[i][0]);
                 keep_small(vv[i][1]);
             }
@@ -211,10 +213,12 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
         mbar_init(&bars[KEYS_IN], WORKERS / 32);
         mbar_init(&bars[PROBS_IN], WORKERS / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        odd_k[0] = odd_k[1] = odd_v[0] = odd_v[1] = -1;
+        odd_v[0] = tiles;
+        odd_v[1] = -1;
     }
     if (tid < BM) odd_q[tid] = 0;
-    if (tid < 2 * KEYS) odd_key[tid & 1][tid >> 1] = nan_key[tid & 1][tid >> 1] = odd_value[tid & 1][tid >> 1] = -1;
+    if (tid < 4) odd_k[tid] = -1;
+    if (tid < 4 * KEYS) odd_key[tid & 3][tid >> 2] = nan_key[tid & 3][tid >> 2] = -1;
     if (warp == WORKERS / 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -329,34 +333,6 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
 #pragma unroll
             for (int i = 0; i < 16; i++) o[c + i] = fmaf(o[c + i], corr, __uint_as_float(raw[i]) * UNSCALE);
         }
-        if (odd_v[t & 1] != t) return;
-        // What was left out of the tile's values, times the probabilities put together again from their pieces (which is exact); a value
-        // that a query does not see must not reach it (0 times it is not 0).
-#pragma unroll 1
-        for (int j = 0; j < KEYS; j++) {
-            if (odd_value[t & 1][j] != t) continue;
-            __syncwarp();
-            uint32_t raw[N_PIECES];
-#pragma unroll
-            for (int i = 0; i < N_PIECES; i++) raw[i] = tmem_ld_32x1(tmem + lanes + F::P_COL + i * (KEYS / 2) + j / 2);
-            tmem_wait_ld();
-            float of[N_PIECES];
-#pragma unroll
-            for (int i = 0; i < N_PIECES; i++) of[i] = __uint_as_float(j % 2 ? raw[i] & 0xffff0000u : raw[i] << 16);
-            const float pr = (of[0] + (of[1] + of[2])) * (1.0f / SCALE);
-            const bool seen = __float_as_uint(of[0]) != __float_as_uint(NOT_SEEN);
-            const float* v = p.v + key_row[t % ROW_SLOTS][j] * d + part * F::COLS;
-#pragma unroll
-            for (int c = 0; c < F::COLS; c += 4) {
-                if (part * F::COLS + c >= d) break;
-                const float4 x = *reinterpret_cast<const float4*>(v + c);
-                if (seen && is_large(x.x)) o[c] = fmaf(pr, x.x, o[c]);
-                if (seen && is_large(x.y)) o[c + 1] = fmaf(pr, x.y, o[c + 1]);
-                if (seen && is_large(x.z)) o[c + 2] = fmaf(pr, x.z, o[c + 2]);
-                if (seen && is_large(x.w)) o[c + 3] = fmaf(pr, x.w, o[c + 3]);
-            }
-        }
-        meet();                                     // the other threads of these rows have read the probabilities
     };
 
     const float unscale = UNSCALE * p.scale;
@@ -373,15 +349,6 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
 #pragma unroll
             for (int j = 0; j < MINE; j++) s[j] = __uint_as_float(raw[j]) * unscale;
         }
-        unsigned again = 0;                         // bit j: the score of key j is to be formed again; bit 16 + j: as a NaN
-        if (odd_q[row] | (odd_k[t & 1] == t)) {
-#pragma unroll 1
-            for (int j = 0; j < MINE; j++) {
-                const int key = part * MINE + j;
-                if (odd_q[row] || odd_key[t & 1][key] == t) again |= 1u << j;
-                if ((odd_q[row] & NAN_TOO) || nan_key[t & 1][key] == t) again |= 65537u << j;
-            }
-        }
         if (t + 1 < tiles) {
             leave_keys(t + 1);
             arrive(KEYS_IN);
@@ -389,18 +356,25 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
         }
         const int start = tile_start(t), end = tile_end(t);
         const long long* key_rows = &key_row[t % ROW_SLOTS][part * MINE];
-        for (; again & 0xffffu; again &= again - 1) {
-            const int j = __ffs(again) - 1;
-            float x = again >> 16 >> j & 1 ? NAN : 0.0f;
-            if (x == 0.0f && key_rows[j] >= 0 && row < rows)
-                x = plain_score(p.q + (size_t)(t0 + row) * p.ld_q + head * d, p.q_pieces, p.k + key_rows[j] * d, d) * p.scale;
-#pragma unroll
-            for (int i = 0; i < MINE; i++) s[i] = i == j ? x : s[i];
-        }
-        __syncwarp();
         const bool found = key_rows[lane % MINE] >= 0;
         unsigned hidden = 0;                        // bit j: this query does not see key j, whatever its score is
-        if (!__all_sync(0xffffffffu, !ruled && found && start + KEYS - 1 <= pos0)) {
+        const bool odd = odd_q[row] | (odd_k[t & 3] == t);
+        if (!__all_sync(0xffffffffu, !odd && !ruled && found && start + KEYS - 1 <= pos0)) {
+            // (in a branch that is there anyway: one of its own, never taken, costs heads of 128 5 %)
+            if (odd) {
+#pragma unroll 1
+                for (int j = 0; j < MINE; j++) {
+                    const int key = part * MINE + j;
+                    if (!odd_q[row] && odd_key[t & 3][key] != t) continue;
+                    float x = 0.0f;
+                    if ((odd_q[row] & NAN_TOO) || nan_key[t & 3][key] == t) x = NAN;
+                    else if (key_rows[j] >= 0 && row < rows)
+                        x = plain_score(p.q + (size_t)(t0 + row) * p.ld_q + head * d, p.q_pieces, p.k + key_rows[j] * d, d) * p.scale;
+#pragma unroll
+                    for (int i = 0; i < MINE; i++) s[i] = i == j ? x : s[i];
+                }
+            }
+            __syncwarp();
             const unsigned there = __ballot_sync(0xffffffffu, found);        // (behind the tile's end no row was found)
             if (r.softcap > 0.0f) {
 #pragma unroll
@@ -455,6 +429,51 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
     pdl_launch_dependents();
     tc_fence_before();
     __syncthreads();
+    // What was left out of the values, with the weights that its keys' scores give; what a query does not see must not reach it (0 times
+    // it is not 0).  (In the loop over the tiles this code, never taken, took heads of 128 from 82 to 106 us for two prompts of 1,024.)
+    for (int t = odd_v[0]; t <= odd_v[1]; t++) {
+        bool all_nan = row < rows;
+#pragma unroll
+        for (int c = 0; c < F::COLS; c++) all_nan &= o[c] != o[c];
+        if (__all_sync(0xffffffffu, all_nan || row >= rows)) break;         // nothing changes that any more
+        const int end = min(tile_start(t) + KEYS, tile_end(t));
+        for (int k0 = tile_start(t); k0 < end; k0 += 32) {
+            // a lane a key: whether there is such a value among this warp's columns, and one that is no NaN (which is one under any weight)
+            const int block = (k0 + lane) / p.page_size, page = k0 + lane < end && block < p.max_blocks ? table[block] : -1;
+            long long at = 0;
+            bool large = false, weighed = false;
+            if (page >= 0 && page < p.num_pages) {
+                at = page * rows_per_page + (long long)kv_head * p.page_size + (k0 + lane) % p.page_size;
+                for (int c = part * F::COLS; c < min((part + 1) * F::COLS, d); c += 4) {
+                    const float4 y = *reinterpret_cast<const float4*>(p.v + at * d + c);
+                    large |= too_large(y);
+                    weighed |= (is_large(y.x) && y.x == y.x) || (is_large(y.y) && y.y == y.y) || (is_large(y.z) && y.z == y.z) || (is_large(y.w) && y.w == y.w);
+                }
+            }
+            const unsigned weigh = __ballot_sync(0xffffffffu, weighed);
+            for (unsigned keys = __ballot_sync(0xffffffffu, large); keys; keys &= keys - 1) {
+                const int j = __ffs(keys) - 1, key = k0 + j;
+                const long long of = __shfl_sync(0xffffffffu, at, j) * d;
+                if (row >= rows || key > pos || (key < my_lo && key >= r.keep_first)) continue;
+                float weight = NAN;
+                if (weigh >> j & 1) {
+                    float x = plain_score(p.q + (size_t)(t0 + row) * p.ld_q + head * d, p.q_pieces, p.k + of, d) * p.scale;
+                    if (r.softcap > 0.0f) x = r.softcap * tanhf(x / r.softcap);
+                    if (r.dist_bias) x += r.dist_bias[(size_t)head * r.n_dist + min(pos - key, r.n_dist - 1)];
+                    weight = exp2_of((x - (m == -INFINITY ? 0.0f : m)) * LOG2E);
+                }
+#pragma unroll
+                for (int c = 0; c < F::COLS; c += 4) {
+                    if (part * F::COLS + c >= d) break;
+                    const float4 y = *reinterpret_cast<const float4*>(p.v + of + part * F::COLS + c);
+                    o[c] = is_large(y.x) ? fmaf(weight, y.x, o[c]) : o[c];
+                    o[c + 1] = is_large(y.y) ? fmaf(weight, y.y, o[c + 1]) : o[c + 1];
+                    o[c + 2] = is_large(y.z) ? fmaf(weight, y.z, o[c + 2]) : o[c + 2];
+                    o[c + 3] = is_large(y.w) ? fmaf(weight, y.w, o[c + 3]) : o[c + 3];
+                }
+            }
+        }
+    }
     if (row >= rows) return;
     const float(&ls)[SHARE][BM] = part_of[tiles & 1];
     l = (ls[0][row] + ls[1][row]) + (ls[2][row] + ls[3][row]);

@@ -435,6 +435,28 @@ def test_prompt_attention_f32_of_very_small_keys_on_tensor_cores(on_tensor_cores
     assert float((got.double().cpu() * 2.0 ** 120 - want).norm() / want.norm()) < 2.0 ** -21
 
 
+@pytest.mark.parametrize("rules", RULES)
+@pytest.mark.parametrize("D", [64, 80, 128])
+def test_values_too_large_to_be_split_under_every_rule(on_tensor_cores, D, rules):
+    """Some entries of some values at 2^100: their part is added by itself, with the weights that the rules give their keys."""
+    case = _paged_case(torch.float32, 2, 2, D, 16, [(0, 130), (40, 1), (63, 65), (199, 70)], seed=D)
+    g = torch.Generator().manual_seed(D)
+    for s, pages, slots in _keys_of(case):
+        some = torch.rand(len(pages), 1, 1, generator=g) < 0.2
+        case["vc"][pages, :, slots] *= torch.where(some & (torch.rand(1, 2, D, generator=g) < 0.3), 2.0 ** 100, 1.0).to(DEV)
+    kw = {k: v for k, v in rules.items() if k in ("window", "keep_first", "softcap", "chunk")}
+    kw["scale"] = 0.8 / D ** 0.5
+    if rules.get("sink"):
+        kw["sink"] = torch.randn(2, generator=g).to(DEV)
+    if rules.get("bias"):
+        kw["dist_bias"] = torch.randn(2, rules["bias"], generator=g).to(DEV)
+    got, want = _both(case, 2, kw)
+    small = want.abs() < 2.0 ** 60
+    assert small.any() and not small.all()
+    assert (got - want)[~small].abs().max().item() < 2e-5 * 2.0 ** 100          # the bound of test_prompt_attention_f32
+    assert (got - want)[small].abs().max().item() < 2e-5
+
+
 def _keys_of(case):
     """(request, its context's pages and slots) of a _paged_case."""
     for s, (before, n) in enumerate(case["seqs"]):
