@@ -32,7 +32,6 @@ namespace {
 constexpr int KEYS = 64, WORKERS = 512, THREADS = WORKERS + 32, SHARE = 4;         // SHARE: threads a row
 constexpr int ROW_SLOTS = 8;            // tiles whose keys' rows are kept
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr float NOT_SEEN = -0.0f;       // the probability of a key that a query does not see (one it sees has at least +0)
 constexpr uint32_t TOO_LARGE = 0x53000000u;     // 2^39: products of two, 128 of them, at SCALE twice stay below 2^127
 
 struct PromptArgs {
@@ -357,7 +356,6 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
         const int start = tile_start(t), end = tile_end(t);
         const long long* key_rows = &key_row[t % ROW_SLOTS][part * MINE];
         const bool found = key_rows[lane % MINE] >= 0;
-        unsigned hidden = 0;                        // bit j: this query does not see key j, whatever its score is
         const bool odd = odd_q[row] | (odd_k[t & 3] == t);
         if (!__all_sync(0xffffffffu, !odd && !ruled && found && start + KEYS - 1 <= pos0)) {
             // (in a branch that is there anyway: one of its own, never taken, costs heads of 128 5 %)
@@ -386,7 +384,6 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
                 const bool seen = (there >> j & 1) && key <= pos && (key >= my_lo || key < r.keep_first);
                 if (r.dist_bias && seen) s[j] += r.dist_bias[(size_t)head * r.n_dist + min(pos - key, r.n_dist - 1)];
                 s[j] = seen ? s[j] : -INFINITY;
-                hidden |= seen ? 0u : 1u << j;
             }
         }
         float top = s[0];
@@ -407,11 +404,6 @@ prefill_attention_f32_tc_kernel(const PromptArgs p) {
             sum += s[j];
         }
         l = l * corr + sum;
-        if (hidden) {
-#pragma unroll
-            for (int j = 0; j < MINE; j++)
-                if (hidden >> j & 1) s[j] = NOT_SEEN;
-        }
         {
             uint4 low[N_PIECES], high[N_PIECES];
             split_eight(make_float4(s[0], s[1], s[2], s[3]), make_float4(s[4], s[5], s[6], s[7]), low);
